@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(G *(N / 16) + (PW ? 32 : 0), 1) blind_rotate_k
 #pragma unroll
                 for (int m = 0; m < kR / 2; m++) {
                     const cpair zp = make_cpair(z[2 * m], z[2 * m + 1]);
-                    const float2 nzi = mul2(zp.im, make_float2(-1.f, -1.f));
+                    const float2 nzi = neg2(zp.im);
 #pragma unroll
                     for (int v = 0; v < KP1; v++) {
                         const float4 *kp = reinterpret_cast<const float4 *>(
@@ -634,7 +634,7 @@ __global__ void __launch_bounds__((K + 1) * L * (N / 16) + 32, 1) blind_rotate_w
                     for (int m = 0; m < kR / 2; m++) {
                         const float4 f = sp[m * NT];
                         const cpair zp{{f.x, f.y}, {f.z, f.w}};
-                        const float2 nzi = mul2(zp.im, make_float2(-1.f, -1.f));
+                        const float2 nzi = neg2(zp.im);
                         cmac_pair(acc[m], zp, nzi, kp[((v * (kR / 2) + m) * 2 + limb) * NT + t]);
                     }
                     mbar_arrive(empty_bar(s));

@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(G *(N / 16) + (PW ? 32 : 0), 1) blind_rotate_p
                 auto mac_m = [&](int m, const uint32_t(&f)[16], float4 kh, float4 kl) {
                     const cpair zp{make_float2(__uint_as_float(f[4 * m]), __uint_as_float(f[4 * m + 1])),
                                    make_float2(__uint_as_float(f[4 * m + 2]), __uint_as_float(f[4 * m + 3]))};
-                    const float2 nzi = mul2(zp.im, make_float2(-1.f, -1.f));
+                    const float2 nzi = neg2(zp.im);
                     cmac_pair(ah[m], zp, nzi, kh);
                     cmac_pair(al[m], zp, nzi, kl);
                 };
@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(G *(N / 16) + (PW ? 32 : 0), 1) blind_rotate_p
                 for (int m = 0; m < kR / 2; m++) {
                     const cpair zp{make_float2(__uint_as_float(f[4 * m]), __uint_as_float(f[4 * m + 1])),
                                    make_float2(__uint_as_float(f[4 * m + 2]), __uint_as_float(f[4 * m + 3]))};
-                    const float2 nzi = mul2(zp.im, make_float2(-1.f, -1.f));
+                    const float2 nzi = neg2(zp.im);
                     cmac_pair(ah[m], zp, nzi, kp[(2 * m) * NT]);
                     cmac_pair(al[m], zp, nzi, kp[(2 * m + 1) * NT]);
                 }
