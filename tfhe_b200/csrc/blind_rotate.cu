@@ -732,18 +732,30 @@ int blind_rotate_supported(const tfheb_params &p) {
     return br_variants(p.N, p.l, p.k == 1 ? TFHEB_FP64 : -1, nullptr, nullptr, 0) > 0;
 }
 
-// Compiled launch variants: (ring degree, precision, bootstraps per CTA G, key-ring depth D, and
-// whether a producer warp streams the key; without it, thread 0 does).
-// Every variant's shared memory stays within 227 KB.  Tuned variants are the autotuner's candidates:
-// the first of a (N, l, precision) triple is the default, and tfheb_autotune times all of them on the
-// device and keeps the fastest per key.  Small variants (few bootstraps per CTA) serve batches that
-// fit one wave of CTAs with fewer bootstraps per SM than the tuned variant would pack (see
-// launch_blind_rotate).
+// The warp kernel's split form keeps a word's digits in a float's mantissa: parameter sets with wider
+// digits (l Bgbit > 23; the reference's sets have 21 and 20) run what was the default before it.
+static cudaError_t launch_warp_split3(const BrArgs &a, cudaStream_t s) {
+    return 3 * a.Bgbit <= 23 ? launch_warp<true, 3, 8, 6>(a, s) : launch_paired_il3<1024, 3, 7, 12, 1>(a, s);
+}
+template <int G>
+static cudaError_t launch_warp_split2(const BrArgs &a, cudaStream_t s) {
+    return 2 * a.Bgbit <= 23 ? launch_warp<true, 2, G, 8>(a, s) : launch_g<float, 1024, 2, true, 7, 4>(a, s);
+}
+
+// Compiled launch variants: (ring degree, gadget length, precision, bootstraps per CTA G, key-ring depth D).
+// Every variant's shared memory stays within 227 KB, and every variant gives the same bits.  Tuned variants are
+// the autotuner's candidates; small ones (few bootstraps per CTA) serve batches, and last waves of
+// batches, with fewer bootstraps per SM than the chosen variant packs.  `us` is the time of a full wave
+// (one CTA on each of 148 SMs at 1965 MHz) per step, by which launch_blind_rotate chooses without a tuned key: a
+// kernel's time hardly depends on how many of its G bootstraps are there, so a batch is as fast as
+// the waves it is cut into.
 struct BrVariant {
     int N, l, precision, G, D;
     bool tuned;
+    float us;  // measured time per step of a wave of SMs x G bootstraps, us (0: not measured)
     cudaError_t (*launch)(const BrArgs &, cudaStream_t);
     int plan = 0;  // 0: one transform per thread; 1: two per thread, spectra in TMEM (blind_rotate_paired.cu)
+    int most_bits = 32;  // the default rule takes the variant for l Bgbit up to this
 };
 static const BrVariant kBrVariants[] = {
     // the split default: two transforms per thread, spectra in TMEM, a 12-half-row key ring; the
@@ -755,66 +767,73 @@ static const BrVariant kBrVariants[] = {
     // without that prefetch: 31.27 ms; loading 3 or 4 slot pairs ahead: 31.49 / 31.68 ms; with less interleaving: 31.59 ms (inverse input in registers, 20 B of
     // spills), 31.85 ms (forward only), 32.2 ms (none, rotated words in registers); 36.24 ms for the
     // plan-0 G = 7, D = 6 below.
-    {1024, 3, TFHEB_SPLIT_FP32, 7, 12, true, launch_paired_il7<1024, 3, 7, 12, 1>, 1},
-    {1024, 3, TFHEB_SPLIT_FP32, 7, 12, true, launch_paired_il3<1024, 3, 7, 12, 1>, 1},
-    {1024, 3, TFHEB_SPLIT_FP32, 7, 12, true, launch_paired_il2<1024, 3, 7, 12, 1>, 1},
-    {1024, 3, TFHEB_SPLIT_FP32, 7, 12, true, launch_paired_il<1024, 3, 7, 12, 1>, 1},
-    {1024, 3, TFHEB_SPLIT_FP32, 7, 12, true, launch_paired<1024, 3, 7, 12, 1, true>, 1},
-    {1024, 3, TFHEB_SPLIT_FP32, 7, 6, true, launch_g<float, 1024, 3, true, 7, 6>},
-    {1024, 3, TFHEB_SPLIT_FP32, 7, 4, true, launch_g<float, 1024, 3, true, 7, 4>},
-    {1024, 3, TFHEB_SPLIT_FP32, 5, 4, true, launch_g<float, 1024, 3, true, 5, 4>},
-    {1024, 3, TFHEB_SPLIT_FP32, 4, 4, true, launch_g<float, 1024, 3, true, 4, 4>},
+    {1024, 3, TFHEB_SPLIT_FP32, 7, 12, true, 12.32, launch_paired_il7<1024, 3, 7, 12, 1>, 1},
+    {1024, 3, TFHEB_SPLIT_FP32, 7, 12, true, 12.24, launch_paired_il3<1024, 3, 7, 12, 1>, 1},
+    {1024, 3, TFHEB_SPLIT_FP32, 7, 12, true, 12.45, launch_paired_il2<1024, 3, 7, 12, 1>, 1},
+    {1024, 3, TFHEB_SPLIT_FP32, 7, 12, true, 12.42, launch_paired_il<1024, 3, 7, 12, 1>, 1},
+    {1024, 3, TFHEB_SPLIT_FP32, 7, 12, true, 12.71, launch_paired<1024, 3, 7, 12, 1, true>, 1},
+    {1024, 3, TFHEB_SPLIT_FP32, 7, 6, true, 14.32, launch_g<float, 1024, 3, true, 7, 6>},
+    {1024, 3, TFHEB_SPLIT_FP32, 7, 4, true, 14.40, launch_g<float, 1024, 3, true, 7, 4>},
+    {1024, 3, TFHEB_SPLIT_FP32, 5, 4, true, 10.63, launch_g<float, 1024, 3, true, 5, 4>},
+    {1024, 3, TFHEB_SPLIT_FP32, 4, 4, true, 8.94, launch_g<float, 1024, 3, true, 4, 4>},
     // plan 1: D counts half rows (8 KB) here; single or double exchange buffers per team
-    {1024, 3, TFHEB_SPLIT_FP32, 7, 8, true, launch_paired<1024, 3, 7, 8, 1, true>, 1},
-    {1024, 3, TFHEB_SPLIT_FP32, 7, 4, true, launch_paired<1024, 3, 7, 4, 2, true>, 1},
-    {1024, 3, TFHEB_SPLIT_FP32, 6, 6, true, launch_paired<1024, 3, 6, 6, 2, true>, 1},
-    {1024, 3, TFHEB_SPLIT_FP32, 3, 4, false, launch_g<float, 1024, 3, true, 3, 4>},
-    {1024, 3, TFHEB_SPLIT_FP32, 2, 4, false, launch_g<float, 1024, 3, true, 2, 4>},
-    {1024, 3, TFHEB_SPLIT_FP32, 1, 4, false, launch_g<float, 1024, 3, true, 1, 4>},
+    {1024, 3, TFHEB_SPLIT_FP32, 7, 8, true, 13.24, launch_paired<1024, 3, 7, 8, 1, true>, 1},
+    {1024, 3, TFHEB_SPLIT_FP32, 7, 4, true, 13.37, launch_paired<1024, 3, 7, 4, 2, true>, 1},
+    {1024, 3, TFHEB_SPLIT_FP32, 6, 6, true, 10.50, launch_paired<1024, 3, 6, 6, 2, true>, 1},
+    // one warp per bootstrap, exchanges in TMEM (blind_rotate_warp.cu; D counts 16 KB units): the split default
+    {1024, 3, TFHEB_SPLIT_FP32, 8, 6, true, 10.94, launch_warp_split3, 1, 23},
+    {1024, 3, TFHEB_SPLIT_FP32, 3, 4, false, 7.74, launch_g<float, 1024, 3, true, 3, 4>},
+    {1024, 3, TFHEB_SPLIT_FP32, 2, 4, false, 5.84, launch_g<float, 1024, 3, true, 2, 4>},
+    {1024, 3, TFHEB_SPLIT_FP32, 1, 4, false, 4.81, launch_g<float, 1024, 3, true, 1, 4>},
     // the default's kernel with 3-6 teams, for batches of one wave (later than plan 0's equals, so
     // the default small-batch rule takes them): one wave of 148 G bootstraps in 4.78 / 5.03 / 6.12 /
     // 6.59 ms at G = 3 / 4 / 5 / 6, against 5.64 (G = 4) and 6.85 ms (G = 5) for plan 0
-    {1024, 3, TFHEB_SPLIT_FP32, 6, 12, false, launch_paired_il3<1024, 3, 6, 12, 1>, 1},
-    {1024, 3, TFHEB_SPLIT_FP32, 5, 12, false, launch_paired_il3<1024, 3, 5, 12, 1>, 1},
-    {1024, 3, TFHEB_SPLIT_FP32, 4, 12, false, launch_paired_il3<1024, 3, 4, 12, 1>, 1},
-    {1024, 3, TFHEB_SPLIT_FP32, 3, 12, false, launch_paired_il3<1024, 3, 3, 12, 1>, 1},
-    {1024, 3, TFHEB_SPLIT_FP32, 1, 8, false, launch_wide<float, 1024, 3, true, 8, 2>},
-    {1024, 3, TFHEB_FP64, 4, 5, true, launch_g<double, 1024, 3, false, 4, 5, false>},
-    {1024, 3, TFHEB_FP64, 4, 4, true, launch_g<double, 1024, 3, false, 4, 4, false>},
-    {1024, 3, TFHEB_FP64, 4, 6, true, launch_g<double, 1024, 3, false, 4, 6>},
-    {1024, 3, TFHEB_FP64, 4, 4, true, launch_g<double, 1024, 3, false, 4, 4>},
-    {1024, 3, TFHEB_FP64, 3, 4, true, launch_g<double, 1024, 3, false, 3, 4>},
-    {1024, 3, TFHEB_FP64, 2, 4, true, launch_g<double, 1024, 3, false, 2, 4>},
-    {1024, 3, TFHEB_FP64, 1, 4, false, launch_g<double, 1024, 3, false, 1, 4>},
-    {1024, 3, TFHEB_FP64, 1, 6, false, launch_wide<double, 1024, 3, false, 6, 1>},
+    {1024, 3, TFHEB_SPLIT_FP32, 6, 12, false, 10.33, launch_paired_il3<1024, 3, 6, 12, 1>, 1},
+    {1024, 3, TFHEB_SPLIT_FP32, 5, 12, false, 9.57, launch_paired_il3<1024, 3, 5, 12, 1>, 1},
+    {1024, 3, TFHEB_SPLIT_FP32, 4, 12, false, 7.86, launch_paired_il3<1024, 3, 4, 12, 1>, 1},
+    {1024, 3, TFHEB_SPLIT_FP32, 3, 12, false, 7.51, launch_paired_il3<1024, 3, 3, 12, 1>, 1},
+    {1024, 3, TFHEB_SPLIT_FP32, 1, 8, false, 3.22, launch_wide<float, 1024, 3, true, 8, 2>},
+    {1024, 3, TFHEB_FP64, 4, 5, true, 9.85, launch_g<double, 1024, 3, false, 4, 5, false>},
+    {1024, 3, TFHEB_FP64, 4, 4, true, 10.18, launch_g<double, 1024, 3, false, 4, 4, false>},
+    {1024, 3, TFHEB_FP64, 4, 6, true, 11.18, launch_g<double, 1024, 3, false, 4, 6>},
+    {1024, 3, TFHEB_FP64, 4, 4, true, 11.04, launch_g<double, 1024, 3, false, 4, 4>},
+    {1024, 3, TFHEB_FP64, 3, 4, true, 8.58, launch_g<double, 1024, 3, false, 3, 4>},
+    {1024, 3, TFHEB_FP64, 2, 4, true, 5.86, launch_g<double, 1024, 3, false, 2, 4>},
+    {1024, 3, TFHEB_FP64, 8, 6, true, 16.08, launch_warp<false, 3, 8, 6>},
+    {1024, 3, TFHEB_FP64, 1, 4, false, 4.57, launch_g<double, 1024, 3, false, 1, 4>},
+    {1024, 3, TFHEB_FP64, 1, 6, false, 3.74, launch_wide<double, 1024, 3, false, 6, 1>},
     // the split default at N = 2048: the N = 1024 default's structure with three teams and a 6-deep
     // ring of 16 KB half rows (51.3 ms per 2048 bootstraps; 51.7 ms with output 0's inverse input in
     // registers, 51.9 ms forward interleave only, 53.1 ms no interleave, 54.1 ms rotated words in
     // registers too, 56.5 ms 4 deep, 62.6 ms for the plan-0 G = 2 below)
-    {2048, 3, TFHEB_SPLIT_FP32, 3, 6, true, launch_paired_il3<2048, 3, 3, 6, 1>, 1},
-    {2048, 3, TFHEB_SPLIT_FP32, 3, 6, true, launch_paired_il2<2048, 3, 3, 6, 1>, 1},
-    {2048, 3, TFHEB_SPLIT_FP32, 3, 6, true, launch_paired_il<2048, 3, 3, 6, 1>, 1},
-    {2048, 3, TFHEB_SPLIT_FP32, 3, 4, true, launch_paired<2048, 3, 3, 4, 1, true>, 1},
-    {2048, 3, TFHEB_SPLIT_FP32, 2, 4, true, launch_g<float, 2048, 3, true, 2, 4, false>},
-    {2048, 3, TFHEB_SPLIT_FP32, 2, 4, true, launch_g<float, 2048, 3, true, 2, 4>},
-    {2048, 3, TFHEB_SPLIT_FP32, 3, 3, true, launch_g<float, 2048, 3, true, 3, 3>},
-    {2048, 3, TFHEB_SPLIT_FP32, 2, 3, true, launch_g<float, 2048, 3, true, 2, 3>},
-    {2048, 3, TFHEB_SPLIT_FP32, 1, 3, false, launch_g<float, 2048, 3, true, 1, 3>},
-    {2048, 3, TFHEB_SPLIT_FP32, 2, 4, true, launch_paired<2048, 3, 2, 4, 2, false>, 1},
-    {2048, 3, TFHEB_SPLIT_FP32, 2, 4, true, launch_paired<2048, 3, 2, 4, 2, true>, 1},
-    {2048, 3, TFHEB_FP64, 2, 3, true, launch_g<double, 2048, 3, false, 2, 3, false>},
-    {2048, 3, TFHEB_FP64, 2, 3, true, launch_g<double, 2048, 3, false, 2, 3>},
-    {2048, 3, TFHEB_FP64, 1, 4, true, launch_g<double, 2048, 3, false, 1, 4>},
-    {512, 3, TFHEB_SPLIT_FP32, 8, 4, true, launch_g<float, 512, 3, true, 8, 4>},
-    {512, 3, TFHEB_FP64, 8, 4, true, launch_g<double, 512, 3, false, 8, 4>},
+    {2048, 3, TFHEB_SPLIT_FP32, 3, 6, true, 12.74, launch_paired_il3<2048, 3, 3, 6, 1>, 1},
+    {2048, 3, TFHEB_SPLIT_FP32, 3, 6, true, 13.04, launch_paired_il2<2048, 3, 3, 6, 1>, 1},
+    {2048, 3, TFHEB_SPLIT_FP32, 3, 6, true, 12.79, launch_paired_il<2048, 3, 3, 6, 1>, 1},
+    {2048, 3, TFHEB_SPLIT_FP32, 3, 4, true, 14.11, launch_paired<2048, 3, 3, 4, 1, true>, 1},
+    {2048, 3, TFHEB_SPLIT_FP32, 2, 4, true, 11.26, launch_g<float, 2048, 3, true, 2, 4, false>},
+    {2048, 3, TFHEB_SPLIT_FP32, 2, 4, true, 11.45, launch_g<float, 2048, 3, true, 2, 4>},
+    {2048, 3, TFHEB_SPLIT_FP32, 3, 3, true, 16.81, launch_g<float, 2048, 3, true, 3, 3>},
+    {2048, 3, TFHEB_SPLIT_FP32, 2, 3, true, 11.56, launch_g<float, 2048, 3, true, 2, 3>},
+    {2048, 3, TFHEB_SPLIT_FP32, 1, 3, false, 8.00, launch_g<float, 2048, 3, true, 1, 3>},
+    {2048, 3, TFHEB_SPLIT_FP32, 2, 4, true, 12.86, launch_paired<2048, 3, 2, 4, 2, false>, 1},
+    {2048, 3, TFHEB_SPLIT_FP32, 2, 4, true, 10.56, launch_paired<2048, 3, 2, 4, 2, true>, 1},
+    {2048, 3, TFHEB_FP64, 2, 3, true, 12.94, launch_g<double, 2048, 3, false, 2, 3, false>},
+    {2048, 3, TFHEB_FP64, 2, 3, true, 14.37, launch_g<double, 2048, 3, false, 2, 3>},
+    {2048, 3, TFHEB_FP64, 1, 4, true, 7.66, launch_g<double, 2048, 3, false, 1, 4>},
+    {512, 3, TFHEB_SPLIT_FP32, 8, 4, true, 0, launch_g<float, 512, 3, true, 8, 4>},
+    {512, 3, TFHEB_FP64, 8, 4, true, 0, launch_g<double, 512, 3, false, 8, 4>},
     // the 80-bit parameter set (n = 500, l = 2, Bgbit = 10; tfhe_gate_bootstrapping.cpp:23-48)
-    {1024, 2, TFHEB_SPLIT_FP32, 7, 4, true, launch_g<float, 1024, 2, true, 7, 4>},
-    {1024, 2, TFHEB_SPLIT_FP32, 1, 4, false, launch_g<float, 1024, 2, true, 1, 4>},
-    {1024, 2, TFHEB_SPLIT_FP32, 1, 8, false, launch_wide<float, 1024, 2, true, 8, 2>},
-    {1024, 2, TFHEB_FP64, 4, 4, true, launch_g<double, 1024, 2, false, 4, 4, false>},
-    {1024, 2, TFHEB_FP64, 4, 4, true, launch_g<double, 1024, 2, false, 4, 4>},
-    {1024, 2, TFHEB_FP64, 1, 4, false, launch_g<double, 1024, 2, false, 1, 4>},
-    {1024, 2, TFHEB_FP64, 1, 6, false, launch_wide<double, 1024, 2, false, 6, 2>},
+    {1024, 2, TFHEB_SPLIT_FP32, 7, 4, true, 11.49, launch_g<float, 1024, 2, true, 7, 4>},
+    {1024, 2, TFHEB_SPLIT_FP32, 8, 8, true, 8.60, launch_warp_split2<8>, 1, 23},
+    {1024, 2, TFHEB_SPLIT_FP32, 4, 8, true, 6.12, launch_warp_split2<4>, 1, 23},
+    {1024, 2, TFHEB_SPLIT_FP32, 1, 4, false, 3.77, launch_g<float, 1024, 2, true, 1, 4>},
+    {1024, 2, TFHEB_SPLIT_FP32, 1, 8, false, 2.50, launch_wide<float, 1024, 2, true, 8, 2>},
+    {1024, 2, TFHEB_FP64, 4, 4, true, 7.90, launch_g<double, 1024, 2, false, 4, 4, false>},
+    {1024, 2, TFHEB_FP64, 4, 4, true, 8.38, launch_g<double, 1024, 2, false, 4, 4>},
+    {1024, 2, TFHEB_FP64, 8, 8, true, 11.66, launch_warp<false, 2, 8, 8>},
+    {1024, 2, TFHEB_FP64, 4, 8, true, 7.83, launch_warp<false, 2, 4, 8>},
+    {1024, 2, TFHEB_FP64, 1, 4, false, 3.44, launch_g<double, 1024, 2, false, 1, 4>},
+    {1024, 2, TFHEB_FP64, 1, 6, false, 2.74, launch_wide<double, 1024, 2, false, 6, 2>},
 };
 
 int br_variants(int N, int l, int precision, int *G, int *D, int cap) {
@@ -833,8 +852,8 @@ int br_variants(int N, int l, int precision, int *G, int *D, int cap) {
 static BrArgs br_args(const tfheb_params &p, const DeviceBsk &bsk, const int32_t *bara, int bara_stride, int boots,
                       int nsteps, int32_t mu, const int32_t *acc_in, int32_t *acc_out, int32_t *d_err,
                       int stall_producer, uint64_t timeout_ns) {
-    return BrArgs{bara,       bara_stride, reinterpret_cast<const uint8_t *>(bsk.bsk), bsk.tables, bsk.tables2, acc_in,
-                  acc_out,    boots,       nsteps, mu, p.Bgbit, bsk.split_shift, d_err, timeout_ns, stall_producer};
+    return BrArgs{bara,       bara_stride, reinterpret_cast<const uint8_t *>(bsk.bsk), reinterpret_cast<const uint8_t *>(bsk.bsk2), bsk.tables, bsk.tables2,
+                  acc_in,     acc_out,    boots,       nsteps, mu, p.Bgbit, bsk.split_shift, d_err, timeout_ns, stall_producer, 0};
 }
 
 int br_variant_count() { return (int)(sizeof(kBrVariants) / sizeof(kBrVariants[0])); }
@@ -882,40 +901,98 @@ cudaError_t launch_blind_rotate_exact(const tfheb_params &p, int precision, cons
                             timeout_ns), s);
 }
 
+// Whether the default rule may take a variant for a parameter set.
+static bool br_offered(const BrVariant &v, const tfheb_params &p, int precision) {
+    return v.N == p.N && v.l == p.l && v.precision == precision && p.l * p.Bgbit <= v.most_bits;
+}
+
+int br_chosen_global(const tfheb_params &p, int precision, const BrChoice &choice) {
+    if (choice.tuned >= 0) return br_tuned_global(p.N, p.l, precision, choice.tuned);
+    int best = -1;
+    for (int g = 0; g < br_variant_count(); g++) {
+        const BrVariant &v = kBrVariants[g];
+        if (!v.tuned || !br_offered(v, p, precision)) continue;
+        if (best < 0 || (v.us > 0 && v.us * kBrVariants[best].G < kBrVariants[best].us * v.G)) best = g;
+    }
+    return best;
+}
+
+// The variant for one wave with `need` bootstraps per CTA, given the batch's variant `big`: the autotuner's
+// choice, or else the one with the least measured time that has room for them.
+static int wave_variant(const tfheb_params &p, int big, int need, const BrChoice &choice) {
+    const BrVariant &b = kBrVariants[big];
+    if (need >= b.G || need < 1) return big;
+    if (need < kSmallNeeds && choice.small[need] != -2)
+        return choice.small[need] >= 0 && choice.small[need] < br_variant_count() ? choice.small[need] : big;
+    int pick = big;
+    for (int g = 0; g < br_variant_count(); g++) {
+        const BrVariant &v = kBrVariants[g];
+        if (!br_offered(v, p, b.precision) || v.G < need || v.G >= b.G || v.us == 0) continue;
+        if (kBrVariants[pick].us == 0 || v.us < kBrVariants[pick].us) pick = g;
+    }
+    return pick;
+}
+
+// The first wave, in bootstraps per CTA, of a rest of `need` of them (fewer than `big` packs): all in one wave,
+// or the cut into several with the least sum of measured times (*us).  600 FP64 bootstraps run as 592 + 8 (6.2 +
+// 2.4 ms; 10.1 ms in one wave of eight per CTA).
+static int first_wave(const tfheb_params &p, int big, int need, const BrChoice &choice, float *us) {
+    int first = need;
+    float best = kBrVariants[wave_variant(p, big, need, choice)].us;
+    for (int a = 1; a < need && best > 0; a++) {
+        const float ta = kBrVariants[wave_variant(p, big, a, choice)].us;
+        float rest = 0;
+        if (ta == 0 || ta >= best) continue;
+        first_wave(p, big, need - a, choice, &rest);
+        if (rest > 0 && ta + rest < best) {
+            best = ta + rest;
+            first = a;
+        }
+    }
+    *us = best;
+    return first;
+}
+
+// Full waves of the chosen variant (SMs x G bootstraps each), then the rest in waves of whatever runs that many
+// per CTA fastest: 4096 split bootstraps are 3 waves of 1184 and 544 spread over 4 per CTA (20.7 + 4.95 ms,
+// where a fourth packed wave takes 6.9).  A lone bootstrap per SM runs its 630 steps in 2.0 ms on the
+// digit-parallel kernel.
 cudaError_t launch_blind_rotate(const tfheb_params &p, int precision, const DeviceBsk &bsk, const int32_t *bara,
                                 int bara_stride, int boots, int nsteps, int32_t mu, const int32_t *acc_in,
                                 int32_t *acc_out, cudaStream_t s, int32_t *d_err, int stall_producer,
-                                uint64_t timeout_ns, const BrChoice &choice) {
+                                uint64_t timeout_ns, const BrChoice &choice, int *launches) {
+    if (launches) *launches = 0;
     if (boots <= 0) return cudaSuccess;
-    int g = br_tuned_global(p.N, p.l, precision, choice.tuned);
-    if (g < 0) return cudaErrorInvalidValue;
-    // A batch that fits one wave of CTAs with fewer bootstraps per CTA than the tuned variant packs
-    // may run faster spread thinner: at the default parameters a lone split-FP32 team finishes its
-    // 630 steps in 2.9 ms, while seven sharing an SM take 9.3 ms, so 16 gates packed 7 per CTA onto 3
-    // SMs would wait for the busiest of them.  FP64: 148 gates in 3.1 ms one per CTA, 7.3 ms four per
-    // CTA.
+    const int big = br_chosen_global(p, precision, choice);
+    if (big < 0) return cudaErrorInvalidValue;
     int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-        sms > 0) {
-        const int need = (boots + sms - 1) / sms;  // bootstraps per CTA for one wave
-        if (need < kBrVariants[g].G && need < kSmallNeeds) {
-            const int e = choice.small[need];
-            if (e >= 0 && e < br_variant_count()) {
-                g = e;
-            } else if (e == -2) {  // fewest bootstraps per CTA that fit; of equals, the later entry
-                int pick = -1;
-                for (int i = 0; i < br_variant_count(); i++) {
-                    const BrVariant &v = kBrVariants[i];
-                    if (v.N == p.N && v.l == p.l && v.precision == precision && v.G >= need &&
-                        v.G < kBrVariants[g].G && (pick < 0 || v.G <= kBrVariants[pick].G))
-                        pick = i;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        sms = 0;
+    for (int first = 0; first < boots;) {
+        int g = big, count = boots - first;
+        if (sms > 0) {
+            const int wave = sms * kBrVariants[big].G, rest = count % wave, need = (rest + sms - 1) / sms;
+            float us = 0;
+            const int a = need > 0 ? first_wave(p, big, need, choice, &us) : 0;
+            g = need > 0 ? wave_variant(p, big, a, choice) : big;
+            if (g != big || a < need) {  // the full waves by themselves, then the rest wave by wave
+                if (count > wave) {
+                    g = big;
+                    count -= rest;
+                } else {
+                    count = a < need ? a * sms : rest;
                 }
-                if (pick >= 0) g = pick;
             }
         }
+        const size_t at = (size_t)first * (p.k + 1) * p.N;
+        const cudaError_t e = launch_blind_rotate_exact(
+            p, precision, bsk, bara + (size_t)first * bara_stride, bara_stride, count, nsteps, mu,
+            acc_in ? acc_in + at : nullptr, acc_out + at, s, d_err, stall_producer, timeout_ns, g);
+        if (e != cudaSuccess) return e;
+        if (launches) ++*launches;
+        first += count;
     }
-    return launch_blind_rotate_exact(p, precision, bsk, bara, bara_stride, boots, nsteps, mu, acc_in, acc_out, s, d_err,
-                                     stall_producer, timeout_ns, g);
+    return cudaSuccess;
 }
 
 struct ExtVariant {

@@ -12,6 +12,7 @@ struct BrArgs {
     const int32_t *bara;
     int bara_stride;
     const uint8_t *bsk;
+    const uint8_t *bsk2;  // split: the key with its limbs side by side (DeviceBsk)
     const void *tables;
     const void *tables2;  // split-FP32 twiddles as broadcast pairs (the paired kernel)
     const int32_t *acc_in;
@@ -23,6 +24,7 @@ struct BrArgs {
     int32_t *err;
     uint64_t timeout_ns;
     int stall_producer;
+    int teams;  // bootstraps per CTA, where the kernel takes it at run time (blind_rotate_warp.cu)
 };
 
 // ---- exact conversions without the conversion (XU) pipe ------------------------------------

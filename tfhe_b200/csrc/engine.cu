@@ -158,6 +158,7 @@ static tfheb_status run_pipeline(CloudKey &ck, int precision, int count, int boo
     const tfheb_params &p = ck.p;
     const int bs = bara_stride_of(p);
     const int kN1 = p.k * p.N + 1;
+    int rotations = 0;  // blind-rotation launches
     tfheb_status st;
     if ((st = grow(ck.d_bara, ck.bara_cap, (size_t)boots * bs)) != TFHEB_OK) return st;
     if ((st = grow(ck.d_acc, ck.acc_cap, (size_t)boots * (p.k + 1) * p.N)) != TFHEB_OK) return st;
@@ -166,14 +167,14 @@ static tfheb_status run_pipeline(CloudKey &ck, int precision, int count, int boo
     TFHEB_CUDA(timed(ck, 1, s, [&] {
         return launch_blind_rotate(p, precision, ck.dbsk[precision], ck.d_bara, bs, boots, p.n,
                                    modswitch_to_torus32(1, 8), nullptr, ck.d_acc, s, ck.d_err, ck.stall_producer,
-                                   ck.wait_timeout_ns, ck.br[precision]);
+                                   ck.wait_timeout_ns, ck.br[precision], &rotations);
     }));
     TFHEB_CUDA(timed(ck, 2, s, [&] { return launch_extract(p, ck.d_gdesc, count, ck.d_acc, ck.d_ksin, kN1, s); }));
     TFHEB_CUDA(timed(ck, 3, s, [&] {
         return launch_keyswitch(ck, count, ck.d_ksin, kN1, d_out, s);
     }));
-    g_launches += 4;
-    ck.launches += 4;
+    g_launches += 3 + rotations;
+    ck.launches += 3 + rotations;
     if (d_terms) {
         TFHEB_CUDA(launch_ks_terms(p, count, ck.d_ksin, kN1, d_terms, s));
         g_launches += 1;
@@ -387,6 +388,7 @@ void tfheb_cloud_key_free(tfheb_cloud_key *c) {
         cudaSetDevice(ck.device);
         for (auto &d : ck.dbsk) {
             cudaFree(d.bsk);
+            cudaFree(d.bsk2);
             cudaFree(d.tables);
             cudaFree(d.tables2);
         }
@@ -484,9 +486,10 @@ tfheb_status tfheb_cloud_key_to_device(tfheb_cloud_key *c, int32_t device, int32
         if (d.bsk && (prec == TFHEB_FP64 || d.split_shift == split_shift)) continue;
         if (d.bsk) {
             cudaFree(d.bsk);
+            cudaFree(d.bsk2);
             cudaFree(d.tables);
             cudaFree(d.tables2);
-            d.bsk = d.tables = d.tables2 = nullptr;
+            d.bsk = d.bsk2 = d.tables = d.tables2 = nullptr;
         }
         if (!d_coef.p) {
             TFHEB_CUDA(cudaMalloc(&d_coef.p, ck.bsk_coef.size() * sizeof(int32_t)));
@@ -497,9 +500,10 @@ tfheb_status tfheb_cloud_key_to_device(tfheb_cloud_key *c, int32_t device, int32
         }
         d.bsk_bytes = polys * (size_t)(p.N / 2) * 16;
         TFHEB_CUDA(cudaMalloc(&d.bsk, d.bsk_bytes));
+        if (prec == TFHEB_SPLIT_FP32 && p.N == 1024) TFHEB_CUDA(cudaMalloc(&d.bsk2, d.bsk_bytes));
         d.split_shift = prec == TFHEB_SPLIT_FP32 ? split_shift : 0;
         TFHEB_CUDA(launch_bsk_to_fft(p, prec, static_cast<const int32_t *>(d_coef.p),
-                                     static_cast<const double *>(d_tab64.p), d.bsk, split_shift, ck.stream));
+                                     static_cast<const double *>(d_tab64.p), d.bsk, d.bsk2, split_shift, ck.stream));
         if (prec == TFHEB_FP64) {
             TFHEB_CUDA(cudaMalloc(&d.tables, tab.size() * sizeof(double)));
             TFHEB_CUDA(cudaMemcpy(d.tables, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice));
@@ -623,12 +627,13 @@ static tfheb_status bootstrap_woks_locked(CloudKey &ck, int32_t precision, int32
     const int bs = bara_stride_of(p);
     if ((st = grow(ck.d_bara, ck.bara_cap, (size_t)count * bs)) != TFHEB_OK) return st;
     if ((st = grow(ck.d_acc, ck.acc_cap, (size_t)count * (p.k + 1) * p.N)) != TFHEB_OK) return st;
+    int rotations = 0;
     TFHEB_CUDA(launch_prologue(p, ck.d_bdesc, count, d_in, d_in, d_in, ck.d_bara, bs, s));
     TFHEB_CUDA(launch_blind_rotate(p, precision, ck.dbsk[precision], ck.d_bara, bs, count, p.n, mu, nullptr,
                                    ck.d_acc, s, ck.d_err, ck.stall_producer, ck.wait_timeout_ns,
-                                   ck.br[precision]));
+                                   ck.br[precision], &rotations));
     TFHEB_CUDA(launch_extract(p, ck.d_gdesc, count, ck.d_acc, d_out, p.k * p.N + 1, s));
-    g_launches += 3;
+    g_launches += 2 + rotations;
     return TFHEB_OK;
 }
 
@@ -684,6 +689,7 @@ static DeviceBsk key_from_step(const CloudKey &ck, int precision, int first) {
     const tfheb_params &p = ck.p;
     const size_t step_bytes = (size_t)(p.k + 1) * p.l * (p.k + 1) * (p.N / 2) * 16;
     d.bsk = static_cast<unsigned char *>(d.bsk) + step_bytes * (size_t)first;
+    if (d.bsk2) d.bsk2 = static_cast<unsigned char *>(d.bsk2) + step_bytes * (size_t)first;
     return d;
 }
 
@@ -702,11 +708,12 @@ tfheb_status tfheb_blind_rotate_steps_device(tfheb_cloud_key *c, int32_t precisi
     if ((st = check_device_ptr(ck, d_bara, "d_bara")) != TFHEB_OK || (st = check_device_ptr(ck, d_acc, "d_acc")) != TFHEB_OK)
         return st;
     cudaStream_t s = stream ? (cudaStream_t)stream : ck.stream;
+    int rotations = 0;
     // in place: acc_in == acc_out is safe (each team reads its row fully before writing it back)
     TFHEB_CUDA(launch_blind_rotate(ck.p, precision, key_from_step(ck, precision, first_step), d_bara, nsteps, count,
                                    nsteps, 0, d_acc, d_acc, s, ck.d_err, ck.stall_producer, ck.wait_timeout_ns,
-                                   ck.br[precision]));
-    g_launches += 1;
+                                   ck.br[precision], &rotations));
+    g_launches += rotations;
     return TFHEB_OK;
 }
 
@@ -737,14 +744,15 @@ tfheb_status tfheb_blind_rotate_extract_device(tfheb_cloud_key *c, int32_t preci
     cudaStream_t s = stream ? (cudaStream_t)stream : ck.stream;
     if ((st = scratch_begin(ck, s)) != TFHEB_OK) return st;
     if ((st = grow(ck.d_acc, ck.acc_cap, (size_t)count * (p.k + 1) * p.N)) == TFHEB_OK) {
+        int rotations = 0;
         cudaError_t e = launch_testvec(p, count, d_v, d_barb, ck.d_acc, s);
         if (e == cudaSuccess && nsteps > 0)
             e = launch_blind_rotate(p, precision, key_from_step(ck, precision, first_step), d_bara, nsteps, count,
                                     nsteps, 0, ck.d_acc, ck.d_acc, s, ck.d_err, ck.stall_producer,
-                                    ck.wait_timeout_ns, ck.br[precision]);
+                                    ck.wait_timeout_ns, ck.br[precision], &rotations);
         if (e == cudaSuccess) e = launch_extract(p, nullptr, count, ck.d_acc, d_out, p.k * p.N + 1, s);
         if (e != cudaSuccess) st = cuda_fail(e, "tfheb_blind_rotate_extract_device");
-        g_launches += nsteps > 0 ? 3 : 2;
+        g_launches += 2 + rotations;
     }
     const tfheb_status se = scratch_end(ck, s);
     return st != TFHEB_OK ? st : se;
@@ -877,18 +885,21 @@ tfheb_status tfheb_set_keyswitch_kernel(tfheb_cloud_key *c, int32_t which) {
     return TFHEB_OK;
 }
 
-// Times every compiled blind-rotation variant on `boots` synthetic bootstraps (random rotation
-// amounts, the key's own bootstrapping key) and keeps the fastest for this key and precision.
-// Device time of one blind-rotation launch of compiled variant g over `boots` bootstraps (the second
-// of two runs; the first warms up).
-static tfheb_status time_variant(CloudKey &ck, int precision, int g, int boots, cudaEvent_t e0, cudaEvent_t e1,
-                                 float *ms) {
+// Device time of a blind rotation of `boots` synthetic bootstraps (random rotation amounts, the key's own
+// bootstrapping key), the second of two runs; the first warms up.  g >= 0: one launch of compiled variant
+// g; else the launches that `choice` means for such a batch.
+static tfheb_status time_variant(CloudKey &ck, int precision, int g, const BrChoice &choice, int boots, cudaEvent_t e0,
+                                 cudaEvent_t e1, float *ms) {
     const tfheb_params &p = ck.p;
+    const int32_t mu = modswitch_to_torus32(1, 8);
     for (int rep = 0; rep < 2; rep++) {
         TFHEB_CUDA(cudaEventRecord(e0, ck.stream));
-        TFHEB_CUDA(launch_blind_rotate_exact(p, precision, ck.dbsk[precision], ck.d_bara, bara_stride_of(p), boots, p.n,
-                                             modswitch_to_torus32(1, 8), nullptr, ck.d_acc, ck.stream, ck.d_err, 0,
-                                             ck.wait_timeout_ns, g));
+        if (g >= 0)
+            TFHEB_CUDA(launch_blind_rotate_exact(p, precision, ck.dbsk[precision], ck.d_bara, bara_stride_of(p), boots, p.n,
+                                                 mu, nullptr, ck.d_acc, ck.stream, ck.d_err, 0, ck.wait_timeout_ns, g));
+        else
+            TFHEB_CUDA(launch_blind_rotate(p, precision, ck.dbsk[precision], ck.d_bara, bara_stride_of(p), boots, p.n, mu,
+                                           nullptr, ck.d_acc, ck.stream, ck.d_err, 0, ck.wait_timeout_ns, choice));
         TFHEB_CUDA(cudaEventRecord(e1, ck.stream));
         TFHEB_CUDA(cudaEventSynchronize(e1));
         TFHEB_CUDA(cudaEventElapsedTime(ms, e0, e1));
@@ -934,8 +945,9 @@ tfheb_status tfheb_autotune(tfheb_cloud_key *c, int32_t precision, int32_t boots
     float best_ms = 1e30f;
     for (int v = 0; v < nv; v++) {
         float ms = 0;
-        if ((st = time_variant(ck, precision, br_tuned_global(p.N, p.l, precision, v), boots, ev.a, ev.b, &ms)) != TFHEB_OK)
-            return st;
+        BrChoice trial;  // the candidate for full waves, the default rule for the last one
+        trial.tuned = v;
+        if ((st = time_variant(ck, precision, -1, trial, boots, ev.a, ev.b, &ms)) != TFHEB_OK) return st;
         if (ms_out && v < cap) ms_out[v] = ms;
         if (ms < best_ms) {
             best_ms = ms;
@@ -954,7 +966,7 @@ tfheb_status tfheb_autotune(tfheb_cloud_key *c, int32_t precision, int32_t boots
             br_variant_info(g, &N, &l, &prec, &G, nullptr, nullptr);
             if (N != p.N || l != p.l || prec != precision || G < need || G > best_G) continue;
             float ms = 0;
-            if ((st = time_variant(ck, precision, g, sms * need, ev.a, ev.b, &ms)) != TFHEB_OK) return st;
+            if ((st = time_variant(ck, precision, g, choice, sms * need, ev.a, ev.b, &ms)) != TFHEB_OK) return st;
             if (ms < fastest) {
                 fastest = ms;
                 choice.small[need] = g == best_g ? -1 : g;

@@ -35,6 +35,7 @@ struct GateDesc {
 // Device-side FFT-domain bootstrapping key and tables for one precision.
 struct DeviceBsk {
     void *bsk = nullptr;      // [n][kpl][k+1][R][NT] x 16 bytes (double2, or float4 = hi.re,hi.im,lo.re,lo.im)
+    void *bsk2 = nullptr;     // split, N = 1024: the same key, per slot {hi.re, lo.re, hi.im, lo.im}
     void *tables = nullptr;   // stage twiddles (stage 0 carries the twist), layout of the precision
     void *tables2 = nullptr;  // split only: the FP32 factors as broadcast pairs (build_tables_f32_paired)
     size_t bsk_bytes = 0;
@@ -65,14 +66,14 @@ struct ParamMeta {
 };
 
 // Blind-rotation variant choice of a key for one precision.  `tuned` indexes the autotuner's
-// candidates of (N, l, precision).  A batch that fits one wave of CTAs with g < kSmallNeeds
-// bootstraps per CTA, fewer than the tuned variant packs, runs small[g] instead: a compiled variant
-// (index into the whole table, br_variant_info), -1 for the tuned one, or -2 for the default rule
-// (the variant with the fewest bootstraps per CTA that still fits one wave).  tfheb_autotune fills
-// small[] from one-wave timings.
+// candidates of (N, l, precision); -1 is the default rule (the candidate with the least measured time per
+// bootstrap).  A wave with g < kSmallNeeds bootstraps per CTA, fewer than that variant packs, runs small[g]
+// instead: a compiled variant (index into the whole table, br_variant_info), -1 for the tuned one, or -2
+// for the default rule (the least measured time of those with room).  tfheb_autotune fills small[] from
+// one-wave timings.
 constexpr int kSmallNeeds = 8;
 struct BrChoice {
-    int tuned = 0;
+    int tuned = -1;
     int small[kSmallNeeds] = {-2, -2, -2, -2, -2, -2, -2, -2};
 };
 
@@ -145,9 +146,10 @@ void build_tables_f32(int N, std::vector<float> &tables);    // float4 pairs of 
 void build_tables_f32_paired(int N, std::vector<float> &tables);
 void fill_slot_freq(int N, std::vector<int32_t> &slot_freq); // [R][NT] -> frequency index
 // key_transform.cu: coefficient-domain bootstrapping key [n][kpl][k+1][N] on the device -> the
-// FFT-domain layout of `precision` (d_out: n*kpl*(k+1)*N/2*16 bytes), on stream s.
+// FFT-domain layout of `precision` (d_out: n*kpl*(k+1)*N/2*16 bytes), on stream s; d_out2 (split, may be
+// null): the same in the limbs-side-by-side layout.
 cudaError_t launch_bsk_to_fft(const tfheb_params &p, int precision, const int32_t *d_coef, const double *d_tables64,
-                              void *d_out, int split_shift, cudaStream_t s);
+                              void *d_out, void *d_out2, int split_shift, cudaStream_t s);
 
 // ---- kernel launchers (kernels.cu) ----------------------------------------------------------
 cudaError_t launch_prologue(const tfheb_params &p, const BootDesc *d_desc, int boots, const int32_t *a,
@@ -155,7 +157,9 @@ cudaError_t launch_prologue(const tfheb_params &p, const BootDesc *d_desc, int b
 cudaError_t launch_blind_rotate(const tfheb_params &p, int precision, const DeviceBsk &bsk, const int32_t *bara,
                                 int bara_stride, int boots, int nsteps, int32_t mu, const int32_t *acc_in,
                                 int32_t *acc_out, cudaStream_t s, int32_t *d_err, int stall_producer,
-                                uint64_t timeout_ns, const BrChoice &choice);
+                                uint64_t timeout_ns, const BrChoice &choice, int *launches = nullptr);
+// Index into the whole table of the variant a key's choice means (tuned = -1: the default rule), or -1.
+int br_chosen_global(const tfheb_params &p, int precision, const BrChoice &choice);
 // The same with one compiled variant given by its index into the whole table (for timing).
 cudaError_t launch_blind_rotate_exact(const tfheb_params &p, int precision, const DeviceBsk &bsk, const int32_t *bara,
                                       int bara_stride, int boots, int nsteps, int32_t mu, const int32_t *acc_in,
@@ -203,6 +207,9 @@ template <int N, int L, int G, int D, int XB>
 cudaError_t launch_paired_il3(const BrArgs &a, cudaStream_t s);
 template <int N, int L, int G, int D, int XB>
 cudaError_t launch_paired_il7(const BrArgs &a, cudaStream_t s);
+// blind_rotate_warp.cu: one warp per bootstrap, up to eight per CTA, exchanges in tensor memory (N = 1024)
+template <bool SPLIT, int L, int G, int D>
+cudaError_t launch_warp(const BrArgs &a, cudaStream_t s);
 // keyswitch.cu: device key upload (both layouts) and the keyswitch of `count` extracted samples
 // (rows of in_stride int32) into rows of n+1 int32.
 cudaError_t upload_keyswitch_key(CloudKey &ck);

@@ -8,7 +8,8 @@
 //   FP64:       double2 (re, im) at [R][NT]
 //   split FP32: the polynomial is first cut into limbs c = hi * 2^S + lo, lo in [-2^(S-1), 2^(S-1));
 //               each limb is transformed in FP64 and rounded to float; per register pair (2m, 2m+1)
-//               and limb, float4 {re(2m), re(2m+1), im(2m), im(2m+1)} at [4][2][NT]
+//               and limb, float4 {re(2m), re(2m+1), im(2m), im(2m+1)} at [4][2][NT]; where a second buffer
+//               is given, the same values there as float4 {hi.re, lo.re, hi.im, lo.im} at [R][NT]
 // One team of N/16 threads per polynomial, 4 teams per CTA, twiddles in shared memory.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -34,7 +35,7 @@ struct KtLayout {
 template <int N, bool SPLIT>
 __global__ void __launch_bounds__(kTeams *(N / 16)) bsk_to_fft_kernel(const int32_t *__restrict__ coef, int polys,
                                                                      const double *__restrict__ tables,
-                                                                     uint8_t *__restrict__ out, int split_shift) {
+                                                                     uint8_t *__restrict__ out, uint8_t *__restrict__ out2, int split_shift) {
     using Lay = KtLayout<N>;
     constexpr int M = Lay::M, NT = Lay::NT;
     using F = TeamFft<double, M, kR>;
@@ -86,34 +87,42 @@ __global__ void __launch_bounds__(kTeams *(N / 16)) bsk_to_fft_kernel(const int3
             o[(m * 2 + 1) * NT + t] = make_float4((float)(xl[2 * m].re * scale), (float)(xl[2 * m + 1].re * scale),
                                                   (float)(xl[2 * m].im * scale), (float)(xl[2 * m + 1].im * scale));
         }
+        if (out2) {
+            float4 *o2 = reinterpret_cast<float4 *>(out2 + (size_t)poly * M * 16);
+#pragma unroll
+            for (int r = 0; r < kR; r++)
+                o2[r * NT + t] = make_float4((float)(xh[r].re * scale), (float)(xl[r].re * scale),
+                                             (float)(xh[r].im * scale), (float)(xl[r].im * scale));
+        }
     }
 }
 
 template <int N, bool SPLIT>
-cudaError_t launch_n(const int32_t *coef, int polys, const double *tables, void *out, int split_shift,
-                     cudaStream_t s) {
+cudaError_t launch_n(const int32_t *coef, int polys, const double *tables, void *out, void *out2,
+                     int split_shift, cudaStream_t s) {
     using Lay = KtLayout<N>;
     auto kern = bsk_to_fft_kernel<N, SPLIT>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::bytes);
     if (e != cudaSuccess) return e;
     const int grid = (polys + kTeams - 1) / kTeams;
-    kern<<<grid, kTeams * Lay::NT, Lay::bytes, s>>>(coef, polys, tables, static_cast<uint8_t *>(out), split_shift);
+    kern<<<grid, kTeams * Lay::NT, Lay::bytes, s>>>(coef, polys, tables, static_cast<uint8_t *>(out),
+                                                 static_cast<uint8_t *>(out2), split_shift);
     return cudaGetLastError();
 }
 
 }  // namespace
 
 cudaError_t launch_bsk_to_fft(const tfheb_params &p, int precision, const int32_t *d_coef, const double *d_tables64,
-                              void *d_out, int split_shift, cudaStream_t s) {
+                              void *d_out, void *d_out2, int split_shift, cudaStream_t s) {
     const int polys = p.n * (p.k + 1) * p.l * (p.k + 1);
     const bool split = precision == TFHEB_SPLIT_FP32;
     switch (p.N) {
-        case 512: return split ? launch_n<512, true>(d_coef, polys, d_tables64, d_out, split_shift, s)
-                               : launch_n<512, false>(d_coef, polys, d_tables64, d_out, split_shift, s);
-        case 1024: return split ? launch_n<1024, true>(d_coef, polys, d_tables64, d_out, split_shift, s)
-                                : launch_n<1024, false>(d_coef, polys, d_tables64, d_out, split_shift, s);
-        case 2048: return split ? launch_n<2048, true>(d_coef, polys, d_tables64, d_out, split_shift, s)
-                                : launch_n<2048, false>(d_coef, polys, d_tables64, d_out, split_shift, s);
+        case 512: return split ? launch_n<512, true>(d_coef, polys, d_tables64, d_out, d_out2, split_shift, s)
+                               : launch_n<512, false>(d_coef, polys, d_tables64, d_out, d_out2, split_shift, s);
+        case 1024: return split ? launch_n<1024, true>(d_coef, polys, d_tables64, d_out, d_out2, split_shift, s)
+                                : launch_n<1024, false>(d_coef, polys, d_tables64, d_out, d_out2, split_shift, s);
+        case 2048: return split ? launch_n<2048, true>(d_coef, polys, d_tables64, d_out, d_out2, split_shift, s)
+                                : launch_n<2048, false>(d_coef, polys, d_tables64, d_out, d_out2, split_shift, s);
         default: return cudaErrorInvalidValue;
     }
 }

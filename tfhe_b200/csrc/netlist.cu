@@ -161,19 +161,20 @@ cudaError_t enqueue_level(const Schedule &sc, const Level &L, CloudKey &ck, int 
     const int n1 = p.n + 1, kN1 = p.k * p.N + 1, bs = bara_stride_for(p);
     const uint64_t interv = ((UINT64_C(1) << 63) / (uint64_t)(2 * p.N)) * 2;
     cudaError_t e = cudaSuccess;
+    int rotations = 0;
     if (L.boots > 0) {
         prologue_rows_kernel<<<L.boots, 256, 0, s>>>(sc.d_boot + L.boot_off, reinterpret_cast<const uint32_t *>(w.wires),
                                                      p.n, interv, w.bara, bs);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         e = launch_blind_rotate(p, precision, ck.dbsk[precision], w.bara, bs, L.boots, p.n, modswitch_to_torus32(1, 8),
                                 nullptr, w.acc, s, ck.d_err, ck.stall_producer, ck.wait_timeout_ns,
-                                ck.br[precision]);
+                                ck.br[precision], &rotations);
         if (e != cudaSuccess) return e;
         e = launch_extract(p, sc.d_gate + L.gate_off, L.gates, w.acc, w.ksin, kN1, s);
         if (e != cudaSuccess) return e;
         e = launch_keyswitch(ck, L.gates, w.ksin, kN1, w.wires + (size_t)L.out_row * n1, s);
         if (e != cudaSuccess) return e;
-        launches += 4;
+        launches += 3 + rotations;
     }
     if (L.unaries > 0) {
         unary_rows_kernel<<<L.unaries, 256, 0, s>>>(sc.d_unary + L.unary_off, reinterpret_cast<const uint32_t *>(w.wires),
@@ -211,11 +212,11 @@ cudaError_t enqueue_netlist(tfheb_netlist *nl, CloudKey &ck, int precision, int3
 // Bootstraps one blind-rotation launch runs per wave: SMs x bootstraps per CTA of the key's current
 // variant for `precision`.
 int wave_bootstraps(const CloudKey &ck, int precision) {
-    int sms = 0, G[16] = {0}, D[16] = {0};
+    int sms = 0, G = 1;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ck.device);
-    const int nv = br_variants(ck.p.N, ck.p.l, precision, G, D, 16);
-    const int v = ck.br[precision].tuned;
-    return std::max(1, sms) * (nv > 0 && v < nv ? G[v] : 1);
+    const int g = br_chosen_global(ck.p, precision, ck.br[precision]);
+    if (g >= 0) br_variant_info(g, nullptr, nullptr, nullptr, &G, nullptr, nullptr);
+    return std::max(1, sms) * G;
 }
 
 // Level assignment that fills blind-rotation waves.  `level` holds each gate's earliest level
@@ -620,7 +621,7 @@ tfheb_status tfheb_gate_batch_mixed_device(tfheb_cloud_key *c, int32_t precision
     for (int i = 0; i < 4 && e == cudaSuccess; i++)
         if (bytes[i]) e = cudaMemcpyAsync(buf[i], host[i], bytes[i], cudaMemcpyHostToDevice, s);
     auto *d_tmp = static_cast<int32_t *>(buf[7]);
-    int launches = 0;
+    int launches = 0, rotations = 0;
     if (e == cudaSuccess && nb > 0) {
         const uint64_t interv = ((UINT64_C(1) << 63) / (uint64_t)(2 * p.N)) * 2;
         prologue_rows_kernel<<<boots, 256, 0, s>>>(static_cast<const BootDescRows *>(buf[0]),
@@ -630,12 +631,12 @@ tfheb_status tfheb_gate_batch_mixed_device(tfheb_cloud_key *c, int32_t precision
         if (e == cudaSuccess)
             e = launch_blind_rotate(p, precision, ck.dbsk[precision], static_cast<int32_t *>(buf[4]), bs, boots, p.n,
                                     mu8, nullptr, static_cast<int32_t *>(buf[5]), s, ck.d_err, ck.stall_producer,
-                                    ck.wait_timeout_ns, ck.br[precision]);
+                                    ck.wait_timeout_ns, ck.br[precision], &rotations);
         if (e == cudaSuccess)
             e = launch_extract(p, static_cast<const GateDesc *>(buf[1]), nb, static_cast<int32_t *>(buf[5]),
                                static_cast<int32_t *>(buf[6]), kN1, s);
         if (e == cudaSuccess) e = launch_keyswitch(ck, nb, static_cast<int32_t *>(buf[6]), kN1, d_tmp, s);
-        launches += 4;
+        launches += 3 + rotations;
     }
     if (e == cudaSuccess && nu > 0) {
         unary_rows_kernel<<<nu, 256, 0, s>>>(static_cast<const UnaryDesc *>(buf[2]),
