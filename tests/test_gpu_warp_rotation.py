@@ -1,7 +1,7 @@
 """The one-warp-per-bootstrap blind rotation (eight bootstraps per CTA, FFT exchanges in tensor memory): bit for
 bit the rotation of the team kernels, which the oracle pins, with full, partly filled and single CTAs, over
-the fewest steps, on both gadget lengths; the cut of a batch into waves; digits too wide for its split form;
-and a stalled key stream."""
+the fewest steps, on both gadget lengths; the kernels for a few bootstraps (one per SM, one per cluster of
+two) against it; the cut of a batch into waves; digits too wide for the split form; stalled key streams."""
 import numpy as np
 import pytest
 
@@ -61,6 +61,23 @@ def test_rotation_equals_the_team_kernel(keys, l, Bgbit, precision, nsteps, coun
     ck.set_br_variant(precision, 0)
 
 
+# one bootstrap on two SMs (at most 74 of 148), one per SM, and both in turn
+@pytest.mark.parametrize("count", [1, 2, 74, 75, 148, 149, 230])
+@pytest.mark.parametrize("nsteps", [1, 2, 3, 7])
+@pytest.mark.parametrize("precision", [tb.FP64, tb.SPLIT_FP32])
+@pytest.mark.parametrize("l,Bgbit", [(3, 7), (2, 10)])
+def test_few_bootstraps_equal_a_packed_wave(keys, l, Bgbit, precision, nsteps, count):
+    sk, ck = keys(l, Bgbit)
+    rng = np.random.default_rng(10 * count + nsteps)
+    acc = rng.integers(-2**31, 2**31, (1184, 2, 1024)).astype(np.int32)
+    bara = rng.integers(0, 2048, (1184, nsteps)).astype(np.int32)
+    bara.flat[:4] = [0, 1, 1023, 1024][:min(4, bara.size)]
+    eight = packed_eight(ck, precision)
+    want = rotate(ck, precision, eight, bara, acc, nsteps)
+    assert (rotate(ck, precision, eight, bara[:count], acc[:count], nsteps) == want[:count]).all()
+    ck.set_br_variant(precision, 0)
+
+
 # around the waves' ends: all of the last wave's choices, and a last CTA with one of eight warps at work
 @pytest.mark.parametrize("count", [1033, 1177, 1184, 1185, 1500, 1777])
 @pytest.mark.parametrize("precision", [tb.FP64, tb.SPLIT_FP32])
@@ -77,11 +94,13 @@ def test_batches_cut_into_waves(l, Bgbit, precision, count):
     assert (sk.decrypt(got)[0] == 1 - (x & y)).all()
 
 
+# a packed wave, one bootstrap per SM, one per two SMs (both CTAs of a cluster give up)
+@pytest.mark.parametrize("count", [1184, 100, 3])
 @pytest.mark.parametrize("precision", [tb.FP64, tb.SPLIT_FP32])
-def test_stalled_key_stream_of_a_packed_wave(keys, precision):
+def test_stalled_key_stream(keys, precision, count):
     sk, ck = keys(3, 7)
     rng = np.random.default_rng(5)
-    x = rng.integers(0, 2, 1184)
+    x = rng.integers(0, 2, count)
     a = sk.encrypt(x, seed=9)
     ck.set_br_variant(precision, packed_eight(ck, precision))
     ck.set_wait_timeout(0.05)

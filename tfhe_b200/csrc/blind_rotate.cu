@@ -453,245 +453,6 @@ __global__ void __launch_bounds__(G *(N / 16) + (PW ? 32 : 0), 1) blind_rotate_k
     }
 }
 
-// ---- one bootstrap per CTA, digits in parallel ------------------------------------------------
-//
-// Latency form for batches far below one wave (a single drop-in gate, a few concurrent callers): one
-// CTA per bootstrap, one team per gadget digit ((k+1) * l teams of N/16 threads) plus the producer
-// warp.  Per step:
-//   1. team d rotates polynomial d / l, takes digit d % l and runs its forward transform; the spectra
-//      go to shared memory;
-//   2. jobs (output polynomial v, and in the split form the key limb) run on the first teams: the
-//      multiply-accumulate over the digits in order 0..(k+1)l-1 against the key rows, then the inverse
-//      transform, rounding and accumulation into the accumulator (split: the two limbs' teams add their
-//      parts with shared-memory atomics; integer sums mod 2^32 are order-free).
-// Each accumulator takes the same products in the same order as in blind_rotate_kernel, and each
-// transform runs the same operations, so the results are bit-identical to it.
-template <typename T, int N, int K, int L, int D, int XB>
-struct WideLayout {
-    static constexpr int M = N / 2, NT = M / kR, KP1 = K + 1, KPL = KP1 * L;
-    static constexpr uint32_t chunk = (uint32_t)KP1 * M * 16;
-    static constexpr size_t bars = 0;
-    static constexpr size_t ring = (2 * D * 8 + 4 + 127) / 128 * 128;
-    static constexpr size_t tables = ring + (size_t)D * chunk;
-    static constexpr size_t tables_bytes = tw_table_bytes<T, M>();
-    static constexpr size_t acc = (tables + tables_bytes + 127) / 128 * 128;
-    static constexpr size_t spec = acc + 4 * (size_t)KP1 * N;           // [digit][slot] spectra
-    static constexpr size_t spec_bytes = (size_t)KPL * M * 2 * sizeof(T);
-    static constexpr size_t xbuf_bytes = ((size_t)Exch<T, M>::bytes + 15) / 16 * 16;
-    static constexpr size_t xbufs = spec + spec_bytes;                   // [team][XB] exchange buffers
-    static constexpr size_t bytes = xbufs + (size_t)KPL * XB * xbuf_bytes;
-    static_assert(2 * D * 8 + 4 <= ring, "barrier block");
-    static_assert(bytes <= 227 * 1024, "shared memory of the variant");
-    static_assert(D >= 1 && (XB == 1 || XB == 2), "ring depth and exchange buffers");
-};
-
-template <typename T, int N, int K, int L, bool SPLIT, int D, int XB>
-__global__ void __launch_bounds__((K + 1) * L * (N / 16) + 32, 1) blind_rotate_wide_kernel(const BrArgs args) {
-    using Lay = WideLayout<T, N, K, L, D, XB>;
-    constexpr int M = N / 2, NT = M / kR, KP1 = K + 1, KPL = KP1 * L;
-    constexpr int JOBS = KP1 * (SPLIT ? 2 : 1);  // (output, limb) pairs
-    static_assert(JOBS <= KPL, "every job needs a team");
-    using F = TeamFft<T, M, kR>;
-    extern __shared__ __align__(128) unsigned char smem[];
-
-    const int tid = threadIdx.x;
-    constexpr int consumers = KPL * NT;
-    constexpr int kAllBar = 15;  // named barrier of all consumer teams (teams use 1..KPL)
-    static_assert(KPL < kAllBar, "named barrier ids");
-    const uint32_t bar0 = smem_addr(smem + Lay::bars);
-    auto full_bar = [&](int s) { return bar0 + 8u * s; };
-    auto empty_bar = [&](int s) { return bar0 + 8u * (D + s); };
-    volatile int32_t *abort_flag = reinterpret_cast<volatile int32_t *>(smem + Lay::bars + 16 * D);
-    const uint32_t ring = smem_addr(smem + Lay::ring);
-
-    if (tid == 0) {
-        for (int s = 0; s < D; s++) {
-            mbar_init(full_bar(s), 1);
-            mbar_init(empty_bar(s), (uint32_t)(JOBS * NT));
-        }
-        *abort_flag = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    {
-        const int4 *g_tab = reinterpret_cast<const int4 *>(args.tables);
-        int4 *s_tab4 = reinterpret_cast<int4 *>(smem + Lay::tables);
-        for (int i = tid; i < (int)(Lay::tables_bytes / 16); i += blockDim.x) s_tab4[i] = g_tab[i];
-    }
-    __syncthreads();
-
-    const int total_chunks = args.nsteps * KPL;
-    if (tid >= consumers) {  // producer warp: stream the key rows, as in blind_rotate_kernel
-        if (tid == consumers) {
-            int issued = 0;
-            if (!args.stall_producer) {
-                for (int c = 0; c < total_chunks; c++) {
-                    const int s = c % D;
-                    if (c >= D && !wait_bounded(empty_bar(s), ((c / D) - 1) & 1, abort_flag, args.timeout_ns, args.err))
-                        break;
-                    mbar_arrive_expect_tx(full_bar(s), Lay::chunk);
-                    bulk_copy_g2s(ring + (uint32_t)s * Lay::chunk, args.bsk + (size_t)c * Lay::chunk, Lay::chunk,
-                                  full_bar(s));
-                    issued = c + 1;
-                }
-            }
-            volatile int32_t no_abort = 0;
-            for (int c = (issued > D ? issued - D : 0); c < issued; c++)
-                wait_bounded(full_bar(c % D), (c / D) & 1, &no_abort, args.timeout_ns, args.err);
-        }
-        return;
-    }
-
-    const int team = tid / NT;  // digit of the forward phase; job of the accumulate phase
-    const int t = tid - team * NT;
-    const int bar_id = 1 + team;
-    const int boot = blockIdx.x;
-    uint32_t *s_acc = reinterpret_cast<uint32_t *>(smem + Lay::acc);
-    T *s_spec = reinterpret_cast<T *>(smem + Lay::spec);
-    ExchPair xp{smem + Lay::xbufs + (size_t)team * XB * Lay::xbuf_bytes, XB == 2 ? (uint32_t)Lay::xbuf_bytes : 0u,
-                0u};
-    const cplx<T> *s_tw = reinterpret_cast<const cplx<T> *>(smem + Lay::tables);
-
-    const int32_t *my_bara = args.bara + (size_t)boot * args.bara_stride;
-    if (args.acc_in) {
-        const uint32_t *src = reinterpret_cast<const uint32_t *>(args.acc_in) + (size_t)boot * KP1 * N;
-        for (int i = tid; i < KP1 * N; i += consumers) s_acc[i] = src[i];
-    } else {
-        // acc = (0, X^{2N-barb} * [mu,...,mu])  (lwe-bootstrapping-functions-fft.cpp:142-145)
-        const int e = 2 * N - my_bara[args.nsteps];
-        for (int i = tid; i < K * N; i += consumers) s_acc[i] = 0u;
-        for (int j = tid; j < N; j += consumers) {
-            int src = j - e;
-            uint32_t neg = 0;
-            while (src < 0) {
-                src += N;
-                neg ^= 1u;
-            }
-            s_acc[K * N + j] = neg ? 0u - (uint32_t)args.mu : (uint32_t)args.mu;
-        }
-    }
-    team_sync(kAllBar, consumers);
-
-    // gadget constants (tgsw.cpp:7-29)
-    const int Bgbit = args.Bgbit;
-    uint32_t offset = 0;
-#pragma unroll
-    for (int q = 0; q < L; q++) offset += 1u << (32 - (q + 1) * Bgbit);
-    offset *= 1u << (Bgbit - 1);
-    const uint32_t maskBg = (1u << Bgbit) - 1u;
-    const T digit_bias = DigitConv<T>::base() + T(1 << (Bgbit - 1));
-    const int u_poly = team / L;                     // polynomial of this team's digit
-    const int shift = 32 - (team - u_poly * L + 1) * Bgbit;
-
-    int c = 0;  // first key row of the step
-    int a_next = args.nsteps > 0 ? my_bara[0] : 0;
-    for (int step = 0; step < args.nsteps; step++, c += KPL) {
-        const int ai = a_next & (2 * N - 1);
-        if (step + 1 < args.nsteps) a_next = my_bara[step + 1];
-
-        // 1. this team's digit: (X^a - 1) * poly + offset, digit, forward transform, spectrum out
-        {
-            const uint32_t *poly = s_acc + u_poly * N;
-            cplx<T> z[kR];
-#pragma unroll
-            for (int r = 0; r < kR; r++) {
-                const int j = t + NT * r;
-                const uint32_t v0 = rot_minus_one<N>(poly, j, ai) + offset;
-                const uint32_t v1 = rot_minus_one<N>(poly, j + M, ai) + offset;
-                const T d0 = DigitConv<T>::conv((v0 >> shift) & maskBg, digit_bias);
-                const T d1 = DigitConv<T>::conv((v1 >> shift) & maskBg, digit_bias);
-                z[r] = cplx<T>{d0, -d1};  // a_j - i a_{j+M}; the twist is folded into the FFT
-            }
-            F::forward(z, xp, s_tw, t, bar_id);
-            if constexpr (SPLIT) {
-                // [digit][m][t] float4 {re(2m), re(2m+1), im(2m), im(2m+1)}
-                float4 *sp = reinterpret_cast<float4 *>(s_spec) + (size_t)team * (kR / 2) * NT + t;
-#pragma unroll
-                for (int m = 0; m < kR / 2; m++)
-                    sp[m * NT] = make_float4(z[2 * m].re, z[2 * m + 1].re, z[2 * m].im, z[2 * m + 1].im);
-            } else {
-                double2 *sp = reinterpret_cast<double2 *>(s_spec) + (size_t)team * kR * NT + t;
-#pragma unroll
-                for (int r = 0; r < kR; r++) sp[r * NT] = make_double2(z[r].re, z[r].im);
-            }
-        }
-        team_sync(kAllBar, consumers);
-
-        // 2. job `team`: multiply-accumulate over the digits in order, inverse transform, accumulate
-        if (team < JOBS) {
-            const int v = SPLIT ? team >> 1 : team;
-            if constexpr (SPLIT) {
-                const int limb = team & 1;
-                cpair acc[kR / 2];
-#pragma unroll
-                for (int m = 0; m < kR / 2; m++) acc[m] = {{0.f, 0.f}, {0.f, 0.f}};
-#pragma unroll
-                for (int d = 0; d < KPL; d++) {
-                    const int row = c + d, s = row % D;
-                    wait_bounded(full_bar(s), (row / D) & 1, abort_flag, args.timeout_ns, args.err);
-                    const float4 *kp = reinterpret_cast<const float4 *>(smem + Lay::ring + (size_t)s * Lay::chunk);
-                    const float4 *sp = reinterpret_cast<const float4 *>(s_spec) + (size_t)d * (kR / 2) * NT + t;
-#pragma unroll
-                    for (int m = 0; m < kR / 2; m++) {
-                        const float4 f = sp[m * NT];
-                        const cpair zp{{f.x, f.y}, {f.z, f.w}};
-                        const float2 nzi = neg2(zp.im);
-                        cmac_pair(acc[m], zp, nzi, kp[((v * (kR / 2) + m) * 2 + limb) * NT + t]);
-                    }
-                    mbar_arrive(empty_bar(s));
-                }
-                cplx<T> z[kR];
-#pragma unroll
-                for (int m = 0; m < kR / 2; m++) {
-                    z[2 * m] = {acc[m].re.x, acc[m].im.x};
-                    z[2 * m + 1] = {acc[m].re.y, acc[m].im.y};
-                }
-                F::inverse(z, xp, s_tw, t, bar_id);
-                uint32_t *poly = s_acc + v * N;
-#pragma unroll
-                for (int r = 0; r < kR; r++) {  // (c_j - i c_{j+M}) of this limb
-                    const int j = t + NT * r;
-                    const uint32_t c0 = limb == 0 ? round_f32_mod32(z[r].re) << args.split_shift
-                                                  : (uint32_t)__float2ll_rn(z[r].re);
-                    const uint32_t c1 = limb == 0 ? round_f32_mod32(-z[r].im) << args.split_shift
-                                                  : (uint32_t)__float2ll_rn(-z[r].im);
-                    atomicAdd(poly + j, c0);
-                    atomicAdd(poly + j + M, c1);
-                }
-            } else {
-                cplx<T> acc[kR];
-#pragma unroll
-                for (int r = 0; r < kR; r++) acc[r] = {T(0), T(0)};
-#pragma unroll
-                for (int d = 0; d < KPL; d++) {
-                    const int row = c + d, s = row % D;
-                    wait_bounded(full_bar(s), (row / D) & 1, abort_flag, args.timeout_ns, args.err);
-                    const double2 *kp = reinterpret_cast<const double2 *>(smem + Lay::ring + (size_t)s * Lay::chunk);
-                    const double2 *sp = reinterpret_cast<const double2 *>(s_spec) + (size_t)d * kR * NT + t;
-#pragma unroll
-                    for (int r = 0; r < kR; r++) {
-                        const double2 zz = sp[r * NT];
-                        const double2 b = kp[(v * kR + r) * NT + t];
-                        cmac(acc[r], cplx<T>{(T)zz.x, (T)zz.y}, cplx<T>{(T)b.x, (T)b.y});
-                    }
-                    mbar_arrive(empty_bar(s));
-                }
-                F::inverse(acc, xp, s_tw, t, bar_id);
-                uint32_t *poly = s_acc + v * N;
-#pragma unroll
-                for (int r = 0; r < kR; r++) {
-                    const int j = t + NT * r;
-                    poly[j] += round_f64_mod32(acc[r].re);  // (c_j - i c_{j+M})
-                    poly[j + M] += round_f64_mod32(-acc[r].im);
-                }
-            }
-        }
-        team_sync(kAllBar, consumers);
-    }
-
-    uint32_t *dst = reinterpret_cast<uint32_t *>(args.acc_out) + (size_t)boot * KP1 * N;
-    for (int i = tid; i < KP1 * N; i += consumers) dst[i] = s_acc[i];
-}
-
 // ---- launch -------------------------------------------------------------------------------------
 
 template <typename T, int N, int L, bool SPLIT, int G, int D, bool PW = true>
@@ -703,16 +464,6 @@ static cudaError_t launch_g(const BrArgs &a, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     const int grid = (a.boots + G - 1) / G;
     kern<<<grid, Lay::threads, smem, s>>>(a);
-    return cudaGetLastError();
-}
-
-template <typename T, int N, int L, bool SPLIT, int D, int XB>
-static cudaError_t launch_wide(const BrArgs &a, cudaStream_t s) {
-    using Lay = WideLayout<T, N, 1, L, D, XB>;
-    auto kern = blind_rotate_wide_kernel<T, N, 1, L, SPLIT, D, XB>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::bytes);
-    if (e != cudaSuccess) return e;
-    kern<<<a.boots, 2 * L * (N / 16) + 32, Lay::bytes, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -756,6 +507,7 @@ struct BrVariant {
     cudaError_t (*launch)(const BrArgs &, cudaStream_t);
     int plan = 0;  // 0: one transform per thread; 1: two per thread, spectra in TMEM (blind_rotate_paired.cu)
     int most_bits = 32;  // the default rule takes the variant for l Bgbit up to this
+    int ctas = 1;        // CTAs per bootstrap (a cluster); 2: for waves of at most SMs / 2 bootstraps, `us` of such a one
 };
 static const BrVariant kBrVariants[] = {
     // the split default: two transforms per thread, spectra in TMEM, a 12-half-row key ring; the
@@ -792,7 +544,9 @@ static const BrVariant kBrVariants[] = {
     {1024, 3, TFHEB_SPLIT_FP32, 5, 12, false, 9.57, launch_paired_il3<1024, 3, 5, 12, 1>, 1},
     {1024, 3, TFHEB_SPLIT_FP32, 4, 12, false, 7.86, launch_paired_il3<1024, 3, 4, 12, 1>, 1},
     {1024, 3, TFHEB_SPLIT_FP32, 3, 12, false, 7.51, launch_paired_il3<1024, 3, 3, 12, 1>, 1},
-    {1024, 3, TFHEB_SPLIT_FP32, 1, 8, false, 3.22, launch_wide<float, 1024, 3, true, 8, 2>},
+    // few bootstraps (blind_rotate_latency.cu; D counts 48 KB stages): one per CTA, one per two CTAs
+    {1024, 3, TFHEB_SPLIT_FP32, 1, 2, false, 2.92, launch_latency<float, 3, 1>},
+    {1024, 3, TFHEB_SPLIT_FP32, 1, 2, false, 1.96, launch_latency<float, 3, 2>, 0, 32, 2},
     {1024, 3, TFHEB_FP64, 4, 5, true, 9.85, launch_g<double, 1024, 3, false, 4, 5, false>},
     {1024, 3, TFHEB_FP64, 4, 4, true, 10.18, launch_g<double, 1024, 3, false, 4, 4, false>},
     {1024, 3, TFHEB_FP64, 4, 6, true, 11.18, launch_g<double, 1024, 3, false, 4, 6>},
@@ -801,7 +555,8 @@ static const BrVariant kBrVariants[] = {
     {1024, 3, TFHEB_FP64, 2, 4, true, 5.86, launch_g<double, 1024, 3, false, 2, 4>},
     {1024, 3, TFHEB_FP64, 8, 6, true, 16.08, launch_warp<false, 3, 8, 6>},
     {1024, 3, TFHEB_FP64, 1, 4, false, 4.57, launch_g<double, 1024, 3, false, 1, 4>},
-    {1024, 3, TFHEB_FP64, 1, 6, false, 3.74, launch_wide<double, 1024, 3, false, 6, 1>},
+    {1024, 3, TFHEB_FP64, 1, 2, false, 3.67, launch_latency<double, 3, 1>},
+    {1024, 3, TFHEB_FP64, 1, 1, false, 2.47, launch_latency<double, 3, 2>, 0, 32, 2},
     // the split default at N = 2048: the N = 1024 default's structure with three teams and a 6-deep
     // ring of 16 KB half rows (51.3 ms per 2048 bootstraps; 51.7 ms with output 0's inverse input in
     // registers, 51.9 ms forward interleave only, 53.1 ms no interleave, 54.1 ms rotated words in
@@ -827,13 +582,15 @@ static const BrVariant kBrVariants[] = {
     {1024, 2, TFHEB_SPLIT_FP32, 8, 8, true, 8.60, launch_warp_split2<8>, 1, 23},
     {1024, 2, TFHEB_SPLIT_FP32, 4, 8, true, 6.12, launch_warp_split2<4>, 1, 23},
     {1024, 2, TFHEB_SPLIT_FP32, 1, 4, false, 3.77, launch_g<float, 1024, 2, true, 1, 4>},
-    {1024, 2, TFHEB_SPLIT_FP32, 1, 8, false, 2.50, launch_wide<float, 1024, 2, true, 8, 2>},
+    {1024, 2, TFHEB_SPLIT_FP32, 1, 2, false, 2.58, launch_latency<float, 2, 1>},
+    {1024, 2, TFHEB_SPLIT_FP32, 1, 2, false, 1.82, launch_latency<float, 2, 2>, 0, 32, 2},
     {1024, 2, TFHEB_FP64, 4, 4, true, 7.90, launch_g<double, 1024, 2, false, 4, 4, false>},
     {1024, 2, TFHEB_FP64, 4, 4, true, 8.38, launch_g<double, 1024, 2, false, 4, 4>},
     {1024, 2, TFHEB_FP64, 8, 8, true, 11.66, launch_warp<false, 2, 8, 8>},
     {1024, 2, TFHEB_FP64, 4, 8, true, 7.83, launch_warp<false, 2, 4, 8>},
     {1024, 2, TFHEB_FP64, 1, 4, false, 3.44, launch_g<double, 1024, 2, false, 1, 4>},
-    {1024, 2, TFHEB_FP64, 1, 6, false, 2.74, launch_wide<double, 1024, 2, false, 6, 2>},
+    {1024, 2, TFHEB_FP64, 1, 2, false, 2.98, launch_latency<double, 2, 1>},
+    {1024, 2, TFHEB_FP64, 1, 1, false, 2.10, launch_latency<double, 2, 2>, 0, 32, 2},
 };
 
 int br_variants(int N, int l, int precision, int *G, int *D, int cap) {
@@ -869,6 +626,8 @@ void br_variant_info(int g, int *N, int *l, int *precision, int *G, int *D, int 
 }
 
 int br_variant_plan(int g) { return kBrVariants[g].plan; }
+
+int br_variant_ctas(int g) { return kBrVariants[g].ctas; }
 
 int br_variant_plans(int N, int l, int precision, int *plan, int cap) {
     int n = 0;
@@ -917,46 +676,50 @@ int br_chosen_global(const tfheb_params &p, int precision, const BrChoice &choic
     return best;
 }
 
-// The variant for one wave with `need` bootstraps per CTA, given the batch's variant `big`: the autotuner's
-// choice, or else the one with the least measured time that has room for them.
+// The variant for one wave with `need` bootstraps per SM (0: at most one per two SMs), given the batch's
+// variant `big`: the autotuner's choice, or else the one with the least measured time that has room for them.
 static int wave_variant(const tfheb_params &p, int big, int need, const BrChoice &choice) {
     const BrVariant &b = kBrVariants[big];
-    if (need >= b.G || need < 1) return big;
+    if (need >= b.G || need < 0) return big;
     if (need < kSmallNeeds && choice.small[need] != -2)
         return choice.small[need] >= 0 && choice.small[need] < br_variant_count() ? choice.small[need] : big;
     int pick = big;
     for (int g = 0; g < br_variant_count(); g++) {
         const BrVariant &v = kBrVariants[g];
-        if (!br_offered(v, p, b.precision) || v.G < need || v.G >= b.G || v.us == 0) continue;
+        if (!br_offered(v, p, b.precision) || v.G < need || v.G >= b.G || v.us == 0 || (v.ctas > 1 && need > 0)) continue;
         if (kBrVariants[pick].us == 0 || v.us < kBrVariants[pick].us) pick = g;
     }
     return pick;
 }
 
-// The first wave, in bootstraps per CTA, of a rest of `need` of them (fewer than `big` packs): all in one wave,
-// or the cut into several with the least sum of measured times (*us).  600 FP64 bootstraps run as 592 + 8 (6.2 +
-// 2.4 ms; 10.1 ms in one wave of eight per CTA).
-static int first_wave(const tfheb_params &p, int big, int need, const BrChoice &choice, float *us) {
-    int first = need;
-    float best = kBrVariants[wave_variant(p, big, need, choice)].us;
-    for (int a = 1; a < need && best > 0; a++) {
+// Bootstraps per SM that a wave of `count` needs (0: two SMs for each).
+static int wave_need(int count, int sms) { return 2 * count <= sms ? 0 : (count + sms - 1) / sms; }
+
+// The first wave's bootstraps of a rest of `count` (fewer than a wave of `big`): all of them, or as many whole
+// bootstraps per SM as give the least sum of measured times (*us) over the waves.  600 FP64 bootstraps run as
+// 592 + 8 (6.2 + 1.6 ms; 10.1 ms in one wave of eight per SM), 160 split ones as 148 + 12 (1.84 + 1.24 ms against
+// 3.68 two per SM).
+static int first_wave(const tfheb_params &p, int big, int count, int sms, const BrChoice &choice, float *us) {
+    const int need = wave_need(count, sms);
+    int first = count;
+    *us = kBrVariants[wave_variant(p, big, need, choice)].us;
+    for (int a = 1; a < need && *us > 0; a++) {
         const float ta = kBrVariants[wave_variant(p, big, a, choice)].us;
         float rest = 0;
-        if (ta == 0 || ta >= best) continue;
-        first_wave(p, big, need - a, choice, &rest);
-        if (rest > 0 && ta + rest < best) {
-            best = ta + rest;
-            first = a;
+        if (ta == 0 || ta >= *us) continue;
+        first_wave(p, big, count - a * sms, sms, choice, &rest);
+        if (rest > 0 && ta + rest < *us) {
+            *us = ta + rest;
+            first = a * sms;
         }
     }
-    *us = best;
     return first;
 }
 
 // Full waves of the chosen variant (SMs x G bootstraps each), then the rest in waves of whatever runs that many
 // per CTA fastest: 4096 split bootstraps are 3 waves of 1184 and 544 spread over 4 per CTA (20.7 + 4.95 ms,
-// where a fourth packed wave takes 6.9).  A lone bootstrap per SM runs its 630 steps in 2.0 ms on the
-// digit-parallel kernel.
+// where a fourth packed wave takes 6.9).  A lone bootstrap runs its 630 steps in 1.24 ms on two SMs, 1.84 ms
+// on one.
 cudaError_t launch_blind_rotate(const tfheb_params &p, int precision, const DeviceBsk &bsk, const int32_t *bara,
                                 int bara_stride, int boots, int nsteps, int32_t mu, const int32_t *acc_in,
                                 int32_t *acc_out, cudaStream_t s, int32_t *d_err, int stall_producer,
@@ -970,17 +733,17 @@ cudaError_t launch_blind_rotate(const tfheb_params &p, int precision, const Devi
         sms = 0;
     for (int first = 0; first < boots;) {
         int g = big, count = boots - first;
-        if (sms > 0) {
-            const int wave = sms * kBrVariants[big].G, rest = count % wave, need = (rest + sms - 1) / sms;
+        const int wave = sms * kBrVariants[big].G, rest = sms > 0 ? count % wave : 0;
+        if (rest > 0) {
             float us = 0;
-            const int a = need > 0 ? first_wave(p, big, need, choice, &us) : 0;
-            g = need > 0 ? wave_variant(p, big, a, choice) : big;
-            if (g != big || a < need) {  // the full waves by themselves, then the rest wave by wave
+            const int part = first_wave(p, big, rest, sms, choice, &us);
+            g = wave_variant(p, big, wave_need(part, sms), choice);
+            if (g != big || part < rest) {  // the full waves by themselves, then the rest wave by wave
                 if (count > wave) {
                     g = big;
                     count -= rest;
                 } else {
-                    count = a < need ? a * sms : rest;
+                    count = part;
                 }
             }
         }

@@ -1,0 +1,497 @@
+// blind_rotate_latency.cu -- the blind rotation of few bootstraps (tfhe_blindRotate_FFT,
+// lwe-bootstrapping-functions-fft.cpp:88-112): one bootstrap per CTA, or per cluster of two CTAs; N = 1024.
+//
+// A batch far below one wave (a single drop-in gate, a few dozen concurrent callers) waits for one bootstrap's
+// serial chain of n steps, so a step is spread over as many warps as it has independent work:
+//   1. all warps rotate: (X^a - 1) acc + offset into shared memory;
+//   2. one team of 64 threads per gadget digit runs its forward transform; the spectra go to shared memory;
+//   3. all warps multiply-accumulate: a thread takes two slots of an output polynomial (both key limbs as a
+//      packed pair in the split form) over the digits in order.  Its keys are in registers before the
+//      spectra are there: their shared-memory reads (two thirds of the phase's) are off the chain;
+//   4. one team per (output polynomial, key limb) runs an inverse transform and adds its rounded words to
+//      an accumulator of its own (integer sums mod 2^32: the rotation reads the sum of the two limbs').
+// With C = 2 a cluster shares the bootstrap: CTA v keeps polynomial v of the accumulator, transforms its l digits
+// and computes output v, so the only thing the two exchange is the spectra, once a step: each team also
+// stores its spectrum into the other CTA's shared memory with st.async, which counts the bytes on the other
+// CTA's mbarrier (plain remote stores and a releasing arrival cost the sender 900 cycles of a step's 5,000).
+// The received half alternates between two buffers: a CTA writes step s + 2's half only after its own
+// multiply-accumulate of step s + 1, hence after the other's sending of s + 1, hence after the other's
+// multiply-accumulate of step s, which read the same buffer.
+// Every accumulator takes the same products in the same order as in blind_rotate_kernel, and each transform
+// runs the same operations, so the bits are the same.
+//
+// The key streams through a ring of two stages (48 KB each at l = 3: a step's rows of one output with C = 2,
+// three digits' rows of both with C = 1), issued by a warp of its own.  Waits are bounded as in
+// blind_rotate_kernel.  After one that ran out, all threads of the CTA leave the loop at the end of the same
+// step, the other CTA's next wait runs out too, and the last barrier (all threads of the cluster) keeps
+// each CTA's shared memory alive until the other's stores have landed.
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "async_copy.cuh"
+#include "br_common.cuh"
+#include "fft.cuh"
+#include "internal.h"
+
+namespace tfheb {
+
+namespace {
+
+template <typename T, int L, int C>
+struct LatencyLayout {
+    static constexpr int N = 1024, M = N / 2, NT = M / kR, KP1 = 2, KPL = KP1 * L;
+    static constexpr bool split = sizeof(T) == 4;
+    static constexpr int polys = KP1 / C;                 // polynomials and outputs of a CTA
+    static constexpr int fwd_teams = polys * L;           // 64 threads each
+    static constexpr int inv_teams = polys * (split ? 2 : 1);
+    static constexpr int mac_warps = 8;
+    static constexpr int warps = 2 * fwd_teams > mac_warps ? 2 * fwd_teams : mac_warps;
+    static constexpr int threads = 32 * (warps + 1);
+    static constexpr uint32_t half = (uint32_t)M * 16;    // one output's slots of one key row
+    static constexpr int per_step = C == 2 ? 1 : 2;       // ring stages per step
+    static constexpr int D = !split && C == 2 ? 1 : 2;    // ring stages (FP64 needs the room; a step outlasts a refill)
+    static constexpr int stage_digits = KPL / per_step;
+    static constexpr uint32_t stage = (uint32_t)stage_digits * polys * half;
+    static constexpr size_t spec_bytes = sizeof(cplx<T>) * M;  // one digit's spectrum
+    static constexpr size_t bars = 0;  // full[D], empty[D], remote[2], abort flag, stop
+    static constexpr size_t ring = 128;
+    static constexpr size_t tables = ring + D * (size_t)stage;
+    static constexpr size_t acc = (tables + tw_table_bytes<T, M>() + 127) / 128 * 128;
+    static constexpr size_t acc_bytes = 4 * (size_t)polys * N;
+    static constexpr size_t acc_low = acc + acc_bytes;                             // split: the low limb's sums
+    static constexpr size_t rot = acc_low + (split ? acc_bytes : 0);               // this step's rotated words
+    static constexpr size_t spec = rot + acc_bytes;                                // [team] own digits
+    static constexpr size_t spec_in = spec + fwd_teams * spec_bytes;               // [parity][digit] the other CTA's
+    static constexpr size_t after_spec = spec_in + (C == 2 ? 2 * L * spec_bytes : 0);
+    static constexpr size_t xbuf_bytes = ((size_t)Exch<T, M>::bytes + 15) / 16 * 16;
+    static constexpr int xbufs_of = split || C == 2 ? 2 : 1;  // per team; two save a barrier per exchange
+    static constexpr int teams = fwd_teams > inv_teams ? fwd_teams : inv_teams;
+    // [inverse team] the products' spectra: a region of their own, or (FP64 in one CTA, short of room) the exchange
+    // buffers of the teams that have no inverse transform, idle from the forward transforms on
+    static constexpr bool sums_in_xbufs = !split && C == 1;
+    static constexpr size_t xbufs = after_spec + (sums_in_xbufs ? 0 : inv_teams * spec_bytes);
+    static constexpr size_t sums = sums_in_xbufs ? xbufs + (size_t)inv_teams * xbuf_bytes : after_spec;
+    static constexpr size_t sum_stride = sums_in_xbufs ? xbuf_bytes : spec_bytes;
+    static_assert(!sums_in_xbufs || (teams >= 2 * inv_teams && xbufs_of == 1), "idle exchange buffers");
+    static constexpr size_t bytes = xbufs + (size_t)teams * xbufs_of * xbuf_bytes;
+    static_assert((2 * D + 2) * 8 + 8 <= ring, "barrier block");
+    static_assert(bytes <= 227 * 1024, "shared memory of the variant");
+    static_assert(2 * inv_teams <= warps, "every inverse transform has a team");
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// address of the same shared-memory location in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+// asynchronous store of 16 bytes to the other CTA, counted on its mbarrier
+__device__ __forceinline__ void store_remote(uint32_t addr, float4 v, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr),
+                 "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void store_remote(uint32_t addr, double2 v, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(addr),
+                 "d"(v.x), "d"(v.y), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity, uint32_t hint_ns) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity), "r"(hint_ns)
+        : "memory");
+    return ok != 0;
+}
+// wait_bounded for the other CTA's stores
+__device__ __forceinline__ void wait_bounded_cluster(uint32_t bar, uint32_t parity, volatile int32_t *abort_flag,
+                                                     uint64_t timeout_ns, int32_t *err) {
+    if (mbar_try_wait_cluster(bar, parity, 0)) return;
+    const uint64_t t0 = global_timer_ns();
+    for (;;) {
+        if (*abort_flag) return;
+        if (mbar_try_wait_cluster(bar, parity, kWaitSleepNs)) return;
+        if (global_timer_ns() - t0 > timeout_ns) {
+            *abort_flag = 1;
+            atomicOr(err, 1);
+            return;
+        }
+    }
+}
+
+}  // namespace
+
+template <typename T, int L, int C>
+__global__ void __launch_bounds__(LatencyLayout<T, L, C>::threads, 1) blind_rotate_latency_kernel(const BrArgs args) {
+    using Lay = LatencyLayout<T, L, C>;
+    constexpr int N = Lay::N, M = Lay::M, NT = Lay::NT, KP1 = 2, KPL = Lay::KPL, D = Lay::D;
+    constexpr bool SPLIT = Lay::split;
+    using F = TeamFft<T, M, kR>;
+    extern __shared__ __align__(128) unsigned char smem[];
+
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int rank = C == 2 ? (int)cluster_rank() : 0;
+    const int boot = blockIdx.x / C;
+    constexpr int consumers = 32 * Lay::warps;
+    constexpr int kAllBar = 15;  // teams use 1..KPL
+    const uint32_t bar0 = smem_addr(smem + Lay::bars);
+    auto full_bar = [&](int s) { return bar0 + 8u * s; };
+    auto empty_bar = [&](int s) { return bar0 + 8u * (D + s); };
+    auto remote_bar = [&](int s) { return bar0 + 8u * (2 * D + s); };
+    volatile int32_t *abort_flag = reinterpret_cast<volatile int32_t *>(smem + Lay::bars + 8 * (2 * D + 2));
+    volatile int32_t *stop = abort_flag + 1;  // one thread's reading of the flag, the same for all warps in a step
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < D; s++) {
+            mbar_init(full_bar(s), 1);
+            mbar_init(empty_bar(s), Lay::mac_warps);
+        }
+        for (int s = 0; s < 2; s++) mbar_init(remote_bar(s), 1);
+        *abort_flag = 0;
+        *stop = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    {
+        const int4 *g_tab = reinterpret_cast<const int4 *>(args.tables);
+        int4 *s_tab = reinterpret_cast<int4 *>(smem + Lay::tables);
+        for (int i = threadIdx.x; i < (int)(tw_table_bytes<T, M>() / 16); i += blockDim.x) s_tab[i] = g_tab[i];
+    }
+    __syncthreads();
+    if constexpr (C == 2) cluster_sync();  // both CTAs' barriers exist before either signals
+
+    if (warp == Lay::warps) {  // ---- the key's stream ----
+        if (lane == 0) {
+            const uint8_t *bsk = SPLIT ? args.bsk2 : args.bsk;
+            const int total = args.nsteps * Lay::per_step;
+            int sent = 0;
+            if (!args.stall_producer) {
+                for (int c = 0; c < total; c++) {
+                    const int s = c % D;
+                    if (c >= D && !wait_bounded(empty_bar(s), ((c / D) - 1) & 1, abort_flag, args.timeout_ns, args.err))
+                        break;
+                    mbar_arrive_expect_tx(full_bar(s), Lay::stage);
+                    const uint32_t dst = smem_addr(smem + Lay::ring) + (uint32_t)s * Lay::stage;
+                    for (int d = 0; d < Lay::stage_digits; d++) {  // C = 2: output `rank` of each row
+                        const size_t row = (size_t)c * Lay::stage_digits + d;
+                        bulk_copy_g2s(dst + (uint32_t)d * Lay::polys * Lay::half, bsk + (row * KP1 + rank) * Lay::half,
+                                      Lay::polys * Lay::half, full_bar(s));
+                    }
+                    sent = c + 1;
+                }
+            }
+            volatile int32_t no_abort = 0;
+            for (int c = (sent > D ? sent - D : 0); c < sent; c++)
+                wait_bounded(full_bar(c % D), (c / D) & 1, &no_abort, args.timeout_ns, args.err);
+        }
+        __syncwarp();
+    } else {  // ---- consumer warps ----
+        const int tid = threadIdx.x, team = warp >> 1, t = tid & (NT - 1);
+        uint32_t *s_acc = reinterpret_cast<uint32_t *>(smem + Lay::acc);
+        uint32_t *s_low = reinterpret_cast<uint32_t *>(smem + Lay::acc_low);  // split: acc = s_acc + s_low
+        uint32_t *s_rot = reinterpret_cast<uint32_t *>(smem + Lay::rot);
+        const cplx<T> *s_tw = reinterpret_cast<const cplx<T> *>(smem + Lay::tables);
+        ExchPair xp{smem + Lay::xbufs + (size_t)(team < Lay::teams ? team : 0) * Lay::xbufs_of * Lay::xbuf_bytes,
+                    Lay::xbufs_of == 2 ? (uint32_t)Lay::xbuf_bytes : 0u, 0u};
+        const int32_t *my_bara = args.bara + (size_t)boot * args.bara_stride;
+
+        // the CTA's polynomials: rank .. rank + polys - 1
+        if (args.acc_in) {
+            const uint32_t *src = reinterpret_cast<const uint32_t *>(args.acc_in) + ((size_t)boot * KP1 + rank) * N;
+            for (int i = tid; i < Lay::polys * N; i += consumers) s_acc[i] = src[i];
+        } else {
+            // acc = (0, X^{2N-barb} * [mu,...,mu])  (lwe-bootstrapping-functions-fft.cpp:142-145)
+            const int e = 2 * N - my_bara[args.nsteps];
+            for (int i = tid; i < Lay::polys * N; i += consumers) {
+                const int j = i & (N - 1);
+                int src = j - e;
+                uint32_t neg = 0;
+                while (src < 0) {
+                    src += N;
+                    neg ^= 1u;
+                }
+                const bool last = rank + i / N == KP1 - 1;
+                s_acc[i] = !last ? 0u : neg ? 0u - (uint32_t)args.mu : (uint32_t)args.mu;
+            }
+        }
+        if constexpr (SPLIT)
+            for (int i = tid; i < Lay::polys * N; i += consumers) s_low[i] = 0u;
+        team_sync(kAllBar, consumers);
+
+        // gadget constants (tgsw.cpp:7-29)
+        const int Bgbit = args.Bgbit;
+        uint32_t offset = 0;
+#pragma unroll
+        for (int q = 0; q < L; q++) offset += 1u << (32 - (q + 1) * Bgbit);
+        offset *= 1u << (Bgbit - 1);
+        const uint32_t maskBg = (1u << Bgbit) - 1u;
+        const T digit_bias = DigitConv<T>::base() + T(1 << (Bgbit - 1));
+        const int shift = 32 - (team % L + 1) * Bgbit;
+        // |low-limb sum| <= (k+1) l N 2^(Bgbit-1) 2^(S-1), doubled for FP32's error
+        const bool low_small = (KPL * N <= 8192) && 13 + Bgbit - 1 + args.split_shift - 1 + 1 <= 44;
+        // this team's spectrum here and in the other CTA (per parity)
+        unsigned char *my_spec = smem + Lay::spec + (size_t)(team < Lay::fwd_teams ? team : 0) * Lay::spec_bytes;
+        uint32_t far_spec = 0, far_bar = 0;
+        if constexpr (C == 2) {
+            far_spec = cluster_addr(smem_addr(smem + Lay::spec_in + (size_t)(team < L ? team : 0) * Lay::spec_bytes),
+                                    (uint32_t)(rank ^ 1));
+            far_bar = cluster_addr(remote_bar(0), (uint32_t)(rank ^ 1));
+        }
+
+        int a_next = args.nsteps > 0 ? my_bara[0] : 0;
+        bool aborted = false;
+        for (int step = 0; step < args.nsteps && !aborted; step++) {
+            const int ai = a_next & (2 * N - 1);
+            if (step + 1 < args.nsteps) a_next = my_bara[step + 1];
+            const int parity = step & 1;
+            if (warp == Lay::mac_warps - 1 && lane == 0) {
+                *stop = *abort_flag;
+                if (C == 2) mbar_arrive_expect_tx(remote_bar(parity), (uint32_t)(L * Lay::spec_bytes));
+            }
+
+            // 1. (X^a - 1) acc + offset: coefficient e = j - a mod 2N is e mod N, negated when e has the N bit
+#pragma unroll
+            for (int i0 = 0; i0 < Lay::polys * N; i0 += consumers) {
+                const int i = i0 + tid;
+                if (Lay::polys * N % consumers != 0 && i >= Lay::polys * N) break;
+                const int e = (i & (N - 1)) - ai, src = (i & ~(N - 1)) + (e & (N - 1));
+                const uint32_t neg = (uint32_t)((int32_t)((uint32_t)e << 21) >> 31), on = offset - neg;
+                const uint32_t x = SPLIT ? s_acc[src] + s_low[src] : s_acc[src];
+                const uint32_t y = SPLIT ? s_acc[i] + s_low[i] : s_acc[i];
+                s_rot[i] = (x ^ neg) + (on - y);
+            }
+            team_sync(kAllBar, consumers);
+
+            // the keys of the multiply-accumulate below: thread (m, tm) takes slots 2m, 2m + 1 of virtual thread tm
+            const int m = tid >> 6, tm = tid & (NT - 1);
+            float4 key[Lay::stage_digits][Lay::polys][2];  // split {hi.re, lo.re, hi.im, lo.im}; FP64 {re, im}
+            auto load_keys = [&](int c) {
+                const int s = c % D;
+                wait_bounded(full_bar(s), (c / D) & 1, abort_flag, args.timeout_ns, args.err);
+                const unsigned char *at = smem + Lay::ring + (size_t)s * Lay::stage + 16 * (size_t)(2 * m * NT + tm);
+#pragma unroll
+                for (int dd = 0; dd < Lay::stage_digits; dd++)
+#pragma unroll
+                    for (int v = 0; v < Lay::polys; v++)
+#pragma unroll
+                        for (int i = 0; i < 2; i++)
+                            key[dd][v][i] = *reinterpret_cast<const float4 *>(
+                                at + (size_t)((SPLIT || C == 1 || rank == 0 ? dd : (dd + L) % KPL) * Lay::polys + v) * Lay::half + 16 * i * NT);
+            };
+
+            // 2. digit, forward transform, spectrum out
+            if (team < Lay::fwd_teams) {
+                const uint32_t *w = s_rot + (team / L) * N + t;
+                cplx<T> z[kR];
+#pragma unroll
+                for (int r = 0; r < kR; r++) {
+                    const T d0 = DigitConv<T>::conv((w[NT * r] >> shift) & maskBg, digit_bias);
+                    const T d1 = DigitConv<T>::conv((w[NT * r + M] >> shift) & maskBg, digit_bias);
+                    z[r] = cplx<T>{d0, -d1};  // a_j - i a_{j+M}; the twist is folded into the FFT
+                }
+                F::forward(z, xp, s_tw, t, 1 + team);
+                const uint32_t far = far_spec + (uint32_t)(parity * L * Lay::spec_bytes) + 16u * (uint32_t)t;
+                const uint32_t bar = far_bar + 8u * (uint32_t)parity;
+                if constexpr (SPLIT) {
+                    // [register pair m][t] {re(2m), im(2m), re(2m+1), im(2m+1)}
+#pragma unroll
+                    for (int m = 0; m < kR / 2; m++) {
+                        const float4 v = make_float4(z[2 * m].re, z[2 * m].im, z[2 * m + 1].re, z[2 * m + 1].im);
+                        if constexpr (C == 2) store_remote(far + 16u * (uint32_t)(m * NT), v, bar);
+                        reinterpret_cast<float4 *>(my_spec)[m * NT + t] = v;
+                    }
+                } else {
+                    // [r][t] {re, im}
+#pragma unroll
+                    for (int r = 0; r < kR; r++) {
+                        const double2 v = make_double2(z[r].re, z[r].im);
+                        if constexpr (C == 2) store_remote(far + 16u * (uint32_t)(r * NT), v, bar);
+                        reinterpret_cast<double2 *>(my_spec)[r * NT + t] = v;
+                    }
+                }
+            }
+
+            // 3. multiply-accumulate.  The keys come in while the spectra are on their way to the other CTA; read before
+            // the forward transform they delayed it (2.17 against 1.97 us per step).
+            if (warp < Lay::mac_warps) load_keys(step * Lay::per_step);
+            team_sync(kAllBar, consumers);
+            if (warp < Lay::mac_warps) {
+                auto wait_remote = [&] {
+                    if constexpr (C == 2)
+                        wait_bounded_cluster(remote_bar(parity), (uint32_t)(step >> 1) & 1u, abort_flag, args.timeout_ns, args.err);
+                };
+                // FP64 sums round to the exact integers in any order: the CTA's own digits go first, before the
+                // wait.  The split form's low limb keeps the digits' order.
+                if constexpr (SPLIT) wait_remote();
+                cpair acc2[Lay::polys][2];
+                cplx<double> accd[Lay::polys][2];
+#pragma unroll
+                for (int v = 0; v < Lay::polys; v++)
+#pragma unroll
+                    for (int i = 0; i < 2; i++) {
+                        acc2[v][i] = {{0.f, 0.f}, {0.f, 0.f}};
+                        accd[v][i] = {0.0, 0.0};
+                    }
+#pragma unroll
+                for (int st = 0; st < Lay::per_step; st++) {
+                    const int c = step * Lay::per_step + st;
+                    if (st > 0) load_keys(c);
+#pragma unroll
+                    for (int dd = 0; dd < Lay::stage_digits; dd++) {
+                        if (!SPLIT && C == 2 && dd == L) wait_remote();
+                        const int first = SPLIT || C == 1 ? dd : rank ? (dd + L) % KPL : dd;  // digit of this turn
+                        const int d = st * Lay::stage_digits + first, u = d / L, q = d - u * L;
+                        const unsigned char *sp = smem + Lay::spec + (size_t)d * Lay::spec_bytes;
+                        if constexpr (C == 2)
+                            sp = u == rank ? smem + Lay::spec + (size_t)q * Lay::spec_bytes
+                                           : smem + Lay::spec_in + (size_t)(parity * L + q) * Lay::spec_bytes;
+                        if constexpr (SPLIT) {
+                            const float4 f = reinterpret_cast<const float4 *>(sp)[m * NT + tm];
+#pragma unroll
+                            for (int v = 0; v < Lay::polys; v++)
+#pragma unroll
+                                for (int i = 0; i < 2; i++) {
+                                    const float4 k = key[dd][v][i];
+                                    const float zr = i ? f.z : f.x, zi = i ? f.w : f.y;
+                                    const float2 kr = make_float2(k.x, k.y), ki = make_float2(k.z, k.w);
+                                    cpair &a = acc2[v][i];
+                                    a.re = fma2(bc2(zr), kr, a.re);
+                                    a.im = fma2(bc2(zr), ki, a.im);
+                                    a.re = fma2(bc2(-zi), ki, a.re);
+                                    a.im = fma2(bc2(zi), kr, a.im);
+                                }
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 2; i++) {
+                                const double2 f = reinterpret_cast<const double2 *>(sp)[(2 * m + i) * NT + tm];
+#pragma unroll
+                                for (int v = 0; v < Lay::polys; v++) {
+                                    const float4 k = key[dd][v][i];
+                                    const cplx<double> kd{
+                                        __hiloint2double(__float_as_int(k.y), __float_as_int(k.x)),
+                                        __hiloint2double(__float_as_int(k.w), __float_as_int(k.z))};
+                                    cmac(accd[v][i], cplx<double>{f.x, f.y}, kd);
+                                }
+                            }
+                        }
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(empty_bar(c % D));
+                }
+                // to the inverse teams: (output v, limb) in the layouts of the spectra
+#pragma unroll
+                for (int v = 0; v < Lay::polys; v++) {
+                    if constexpr (SPLIT) {
+                        const cpair &a = acc2[v][0], &b = acc2[v][1];
+                        float4 *hi = reinterpret_cast<float4 *>(smem + Lay::sums + (size_t)(2 * v) * Lay::sum_stride);
+                        float4 *lo = reinterpret_cast<float4 *>(smem + Lay::sums + (size_t)(2 * v + 1) * Lay::sum_stride);
+                        hi[m * NT + tm] = make_float4(a.re.x, a.im.x, b.re.x, b.im.x);
+                        lo[m * NT + tm] = make_float4(a.re.y, a.im.y, b.re.y, b.im.y);
+                    } else {
+                        double2 *o = reinterpret_cast<double2 *>(smem + Lay::sums + (size_t)v * Lay::sum_stride);
+#pragma unroll
+                        for (int i = 0; i < 2; i++) o[(2 * m + i) * NT + tm] = make_double2(accd[v][i].re, accd[v][i].im);
+                    }
+                }
+            }
+            team_sync(kAllBar, consumers);
+
+            // 4. inverse transforms, exact rounding, accumulate
+            if (team < Lay::inv_teams) {
+                const unsigned char *in = smem + Lay::sums + (size_t)team * Lay::sum_stride;
+                cplx<T> z[kR];
+                if constexpr (SPLIT) {
+#pragma unroll
+                    for (int i = 0; i < kR / 2; i++) {
+                        const float4 w = reinterpret_cast<const float4 *>(in)[i * NT + t];
+                        z[2 * i] = {w.x, w.y};
+                        z[2 * i + 1] = {w.z, w.w};
+                    }
+                    F::inverse(z, xp, s_tw, t, 1 + team);
+                    // (c_j - i c_{j+M}) of this limb.  Where no low-limb sum can reach 2^44 it is rounded like the
+                    // high limb's, on the FMA pipe (the same integer; the conversion instruction takes longer)
+                    if ((team & 1) && !low_small) {
+                        uint32_t *poly = s_low + (team >> 1) * N + t;
+#pragma unroll
+                        for (int r = 0; r < kR; r++) {
+                            poly[NT * r] += (uint32_t)__float2ll_rn(z[r].re);
+                            poly[NT * r + M] += (uint32_t)__float2ll_rn(-z[r].im);
+                        }
+                    } else {
+                        uint32_t *poly = (team & 1 ? s_low : s_acc) + (team >> 1) * N + t;
+                        const int weight = team & 1 ? 0 : args.split_shift;
+#pragma unroll
+                        for (int r = 0; r < kR; r++) {
+                            poly[NT * r] += round_f32_mod32(z[r].re) << weight;
+                            poly[NT * r + M] += round_f32_mod32(-z[r].im) << weight;
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int r = 0; r < kR; r++) {
+                        const double2 w = reinterpret_cast<const double2 *>(in)[r * NT + t];
+                        z[r] = {(T)w.x, (T)w.y};
+                    }
+                    F::inverse(z, xp, s_tw, t, 1 + team);
+                    uint32_t *poly = s_acc + team * N + t;
+#pragma unroll
+                    for (int r = 0; r < kR; r++) {
+                        poly[NT * r] += round_f64_mod32(z[r].re);  // (c_j - i c_{j+M})
+                        poly[NT * r + M] += round_f64_mod32(-z[r].im);
+                    }
+                }
+            }
+            aborted = *stop != 0;
+            team_sync(kAllBar, consumers);
+        }
+
+        uint32_t *dst = reinterpret_cast<uint32_t *>(args.acc_out) + ((size_t)boot * KP1 + rank) * N;
+        for (int i = tid; i < Lay::polys * N; i += consumers) dst[i] = s_acc[i] + (SPLIT ? s_low[i] : 0u);
+        if (C == 2 && aborted) __nanosleep(20000);  // stores to the other CTA may still be on their way
+        __syncwarp();
+    }
+    if constexpr (C == 2) cluster_sync();
+}
+
+template <typename T, int L, int C>
+cudaError_t launch_latency(const BrArgs &a, cudaStream_t s) {
+    using Lay = LatencyLayout<T, L, C>;
+    if (Lay::split && !a.bsk2) return cudaErrorInvalidValue;
+    auto kern = blind_rotate_latency_kernel<T, L, C>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::bytes);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(a.boots * C));
+    cfg.blockDim = dim3(Lay::threads);
+    cfg.dynamicSmemBytes = Lay::bytes;
+    cfg.stream = s;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = C;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = C > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, a);
+}
+
+template cudaError_t launch_latency<float, 3, 1>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_latency<float, 3, 2>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_latency<double, 3, 1>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_latency<double, 3, 2>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_latency<float, 2, 1>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_latency<float, 2, 2>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_latency<double, 2, 1>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_latency<double, 2, 2>(const BrArgs &, cudaStream_t);
+
+}  // namespace tfheb

@@ -908,8 +908,8 @@ static tfheb_status time_variant(CloudKey &ck, int precision, int g, const BrCho
 }
 
 // Times every tuned variant on `boots` synthetic bootstraps and keeps the fastest.  Then, for each
-// bootstraps-per-CTA need g below the winner's G, times every compiled variant with g <= G <= the
-// winner's on one full wave (SMs x g bootstraps) and records the fastest in the key's small-batch
+// bootstraps-per-SM need g below the winner's G (0: half a bootstrap per SM), times every compiled variant with
+// room for g and G <= the winner's on one full wave (SMs x g bootstraps) and records the fastest in the key's small-batch
 // table (BrChoice).
 tfheb_status tfheb_autotune(tfheb_cloud_key *c, int32_t precision, int32_t boots, double *ms_out, int32_t cap) {
     if (!c || boots <= 0) return TFHEB_ERR_INVALID;
@@ -959,14 +959,16 @@ tfheb_status tfheb_autotune(tfheb_cloud_key *c, int32_t precision, int32_t boots
     const int best_g = br_tuned_global(p.N, p.l, precision, best);
     int best_G = 0;
     br_variant_info(best_g, nullptr, nullptr, nullptr, &best_G, nullptr, nullptr);
-    for (int need = 1; need < best_G && need < kSmallNeeds; need++) {
+    for (int need = 0; need < best_G && need < kSmallNeeds; need++) {
         float fastest = 1e30f;
         for (int g = 0; g < br_variant_count(); g++) {
             int N = 0, l = 0, prec = 0, G = 0;
             br_variant_info(g, &N, &l, &prec, &G, nullptr, nullptr);
             if (N != p.N || l != p.l || prec != precision || G < need || G > best_G) continue;
+            if (need > 0 ? br_variant_ctas(g) > 1 : G > 1) continue;
             float ms = 0;
-            if ((st = time_variant(ck, precision, g, choice, sms * need, ev.a, ev.b, &ms)) != TFHEB_OK) return st;
+            const int wave = need > 0 ? sms * need : std::max(1, sms / 2);
+            if ((st = time_variant(ck, precision, g, choice, wave, ev.a, ev.b, &ms)) != TFHEB_OK) return st;
             if (ms < fastest) {
                 fastest = ms;
                 choice.small[need] = g == best_g ? -1 : g;

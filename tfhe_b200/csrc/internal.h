@@ -67,8 +67,8 @@ struct ParamMeta {
 
 // Blind-rotation variant choice of a key for one precision.  `tuned` indexes the autotuner's
 // candidates of (N, l, precision); -1 is the default rule (the candidate with the least measured time per
-// bootstrap).  A wave with g < kSmallNeeds bootstraps per CTA, fewer than that variant packs, runs small[g]
-// instead: a compiled variant (index into the whole table, br_variant_info), -1 for the tuned one, or -2
+// bootstrap).  A wave with g < kSmallNeeds bootstraps per SM (0: at most one per two SMs), fewer than that
+// variant packs, runs small[g] instead: a compiled variant (index into the whole table, br_variant_info), -1 for the tuned one, or -2
 // for the default rule (the least measured time of those with room).  tfheb_autotune fills small[] from
 // one-wave timings.
 constexpr int kSmallNeeds = 8;
@@ -171,6 +171,8 @@ void br_variant_info(int global_index, int *N, int *l, int *precision, int *G, i
 // FFT plan of a compiled variant: 0 = one transform per thread (radix-8 team FFT), 1 = two transforms
 // per thread on packed f32x2 with the digit spectra in tensor memory (split-FP32 only)
 int br_variant_plan(int global_index);
+// CTAs that share one bootstrap in a compiled variant (2: a cluster, for waves of at most SMs / 2 bootstraps)
+int br_variant_ctas(int global_index);
 // Plans of the launch variants of (N, l, precision), in the order of br_variants.
 int br_variant_plans(int N, int l, int precision, int *plan, int cap);
 // Index into the whole table of the `tuned`-th autotuner candidate of (N, l, precision), or -1.
@@ -210,6 +212,9 @@ cudaError_t launch_paired_il7(const BrArgs &a, cudaStream_t s);
 // blind_rotate_warp.cu: one warp per bootstrap, up to eight per CTA, exchanges in tensor memory (N = 1024)
 template <bool SPLIT, int L, int G, int D>
 cudaError_t launch_warp(const BrArgs &a, cudaStream_t s);
+// blind_rotate_latency.cu: one bootstrap per CTA (C = 1) or per cluster of two (C = 2), N = 1024
+template <typename T, int L, int C>
+cudaError_t launch_latency(const BrArgs &a, cudaStream_t s);
 // keyswitch.cu: device key upload (both layouts) and the keyswitch of `count` extracted samples
 // (rows of in_stride int32) into rows of n+1 int32.
 cudaError_t upload_keyswitch_key(CloudKey &ck);
