@@ -1,7 +1,7 @@
 """The one-warp-per-bootstrap blind rotation (eight bootstraps per CTA, FFT exchanges in tensor memory): bit for
 bit the rotation of the team kernels, which the oracle pins, with full, partly filled and single CTAs, over
-the fewest steps, on both gadget lengths; the kernels for a few bootstraps (one per SM, one per cluster of
-two) against it; the cut of a batch into waves; digits too wide for the split form; stalled key streams."""
+the fewest steps, on both gadget lengths; its form with two warps per bootstrap and the kernels for a few
+bootstraps (one per SM, one per cluster of two) against it; the cut of a batch into waves; digits too wide for the split form; stalled key streams."""
 import numpy as np
 import pytest
 
@@ -61,8 +61,8 @@ def test_rotation_equals_the_team_kernel(keys, l, Bgbit, precision, nsteps, coun
     ck.set_br_variant(precision, 0)
 
 
-# one bootstrap on two SMs (at most 74 of 148), one per SM, and both in turn
-@pytest.mark.parametrize("count", [1, 2, 74, 75, 148, 149, 230])
+# one bootstrap on two SMs (at most 74 of 148), one per SM, both in turn, and two warps for each of 3 or 4 per SM
+@pytest.mark.parametrize("count", [1, 2, 74, 75, 148, 149, 230, 443, 589, 592])
 @pytest.mark.parametrize("nsteps", [1, 2, 3, 7])
 @pytest.mark.parametrize("precision", [tb.FP64, tb.SPLIT_FP32])
 @pytest.mark.parametrize("l,Bgbit", [(3, 7), (2, 10)])
@@ -94,8 +94,8 @@ def test_batches_cut_into_waves(l, Bgbit, precision, count):
     assert (sk.decrypt(got)[0] == 1 - (x & y)).all()
 
 
-# a packed wave, one bootstrap per SM, one per two SMs (both CTAs of a cluster give up)
-@pytest.mark.parametrize("count", [1184, 100, 3])
+# a packed wave, two warps per bootstrap, one bootstrap per SM, one per two SMs (both CTAs of a cluster give up)
+@pytest.mark.parametrize("count", [1184, 592, 100, 3])
 @pytest.mark.parametrize("precision", [tb.FP64, tb.SPLIT_FP32])
 def test_stalled_key_stream(keys, precision, count):
     sk, ck = keys(3, 7)

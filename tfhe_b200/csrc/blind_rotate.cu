@@ -486,11 +486,11 @@ int blind_rotate_supported(const tfheb_params &p) {
 // The warp kernel's split form keeps a word's digits in a float's mantissa: parameter sets with wider
 // digits (l Bgbit > 23; the reference's sets have 21 and 20) run what was the default before it.
 static cudaError_t launch_warp_split3(const BrArgs &a, cudaStream_t s) {
-    return 3 * a.Bgbit <= 23 ? launch_warp<true, 3, 8, 6>(a, s) : launch_paired_il3<1024, 3, 7, 12, 1>(a, s);
+    return 3 * a.Bgbit <= 23 ? launch_warp<true, 3, 8, 6, false>(a, s) : launch_paired_il3<1024, 3, 7, 12, 1>(a, s);
 }
 template <int G>
 static cudaError_t launch_warp_split2(const BrArgs &a, cudaStream_t s) {
-    return 2 * a.Bgbit <= 23 ? launch_warp<true, 2, G, 8>(a, s) : launch_g<float, 1024, 2, true, 7, 4>(a, s);
+    return 2 * a.Bgbit <= 23 ? launch_warp<true, 2, G, 8, G <= 4>(a, s) : launch_g<float, 1024, 2, true, 7, 4>(a, s);
 }
 
 // Compiled launch variants: (ring degree, gadget length, precision, bootstraps per CTA G, key-ring depth D).
@@ -534,16 +534,16 @@ static const BrVariant kBrVariants[] = {
     {1024, 3, TFHEB_SPLIT_FP32, 6, 6, true, 10.50, launch_paired<1024, 3, 6, 6, 2, true>, 1},
     // one warp per bootstrap, exchanges in TMEM (blind_rotate_warp.cu; D counts 16 KB units): the split default
     {1024, 3, TFHEB_SPLIT_FP32, 8, 6, true, 10.94, launch_warp_split3, 1, 23},
-    {1024, 3, TFHEB_SPLIT_FP32, 3, 4, false, 7.74, launch_g<float, 1024, 3, true, 3, 4>},
     {1024, 3, TFHEB_SPLIT_FP32, 2, 4, false, 5.84, launch_g<float, 1024, 3, true, 2, 4>},
-    {1024, 3, TFHEB_SPLIT_FP32, 1, 4, false, 4.81, launch_g<float, 1024, 3, true, 1, 4>},
-    // the default's kernel with 3-6 teams, for batches of one wave (later than plan 0's equals, so
-    // the default small-batch rule takes them): one wave of 148 G bootstraps in 4.78 / 5.03 / 6.12 /
-    // 6.59 ms at G = 3 / 4 / 5 / 6, against 5.64 (G = 4) and 6.85 ms (G = 5) for plan 0
+    // the paired kernel with 3-6 teams, for waves of that many (3 and 4: for digits the warp kernel does not take)
     {1024, 3, TFHEB_SPLIT_FP32, 6, 12, false, 10.33, launch_paired_il3<1024, 3, 6, 12, 1>, 1},
     {1024, 3, TFHEB_SPLIT_FP32, 5, 12, false, 9.57, launch_paired_il3<1024, 3, 5, 12, 1>, 1},
     {1024, 3, TFHEB_SPLIT_FP32, 4, 12, false, 7.86, launch_paired_il3<1024, 3, 4, 12, 1>, 1},
     {1024, 3, TFHEB_SPLIT_FP32, 3, 12, false, 7.51, launch_paired_il3<1024, 3, 3, 12, 1>, 1},
+    // the warp kernel with two warps per bootstrap: 3.91 ms per wave of four per SM, against 4.95 ms for the paired
+    // kernel and 4.97 ms for one warp per bootstrap (FP64: 5.24 ms against 6.22 and 6.6)
+    {1024, 3, TFHEB_SPLIT_FP32, 4, 6, false, 6.21, launch_warp<true, 3, 4, 6, true>, 1, 23},
+    {1024, 3, TFHEB_SPLIT_FP32, 3, 6, false, 6.14, launch_warp<true, 3, 3, 6, true>, 1, 23},
     // few bootstraps (blind_rotate_latency.cu; D counts 48 KB stages): one per CTA, one per two CTAs
     {1024, 3, TFHEB_SPLIT_FP32, 1, 2, false, 2.92, launch_latency<float, 3, 1>},
     {1024, 3, TFHEB_SPLIT_FP32, 1, 2, false, 1.96, launch_latency<float, 3, 2>, 0, 32, 2},
@@ -553,8 +553,9 @@ static const BrVariant kBrVariants[] = {
     {1024, 3, TFHEB_FP64, 4, 4, true, 11.04, launch_g<double, 1024, 3, false, 4, 4>},
     {1024, 3, TFHEB_FP64, 3, 4, true, 8.58, launch_g<double, 1024, 3, false, 3, 4>},
     {1024, 3, TFHEB_FP64, 2, 4, true, 5.86, launch_g<double, 1024, 3, false, 2, 4>},
-    {1024, 3, TFHEB_FP64, 8, 6, true, 16.08, launch_warp<false, 3, 8, 6>},
-    {1024, 3, TFHEB_FP64, 1, 4, false, 4.57, launch_g<double, 1024, 3, false, 1, 4>},
+    {1024, 3, TFHEB_FP64, 8, 6, true, 16.08, launch_warp<false, 3, 8, 6, false>},
+    {1024, 3, TFHEB_FP64, 4, 6, false, 8.32, launch_warp<false, 3, 4, 6, true>},
+    {1024, 3, TFHEB_FP64, 3, 6, false, 8.34, launch_warp<false, 3, 3, 6, true>},
     {1024, 3, TFHEB_FP64, 1, 2, false, 3.67, launch_latency<double, 3, 1>},
     {1024, 3, TFHEB_FP64, 1, 1, false, 2.47, launch_latency<double, 3, 2>, 0, 32, 2},
     // the split default at N = 2048: the N = 1024 default's structure with three teams and a 6-deep
@@ -580,15 +581,13 @@ static const BrVariant kBrVariants[] = {
     // the 80-bit parameter set (n = 500, l = 2, Bgbit = 10; tfhe_gate_bootstrapping.cpp:23-48)
     {1024, 2, TFHEB_SPLIT_FP32, 7, 4, true, 11.49, launch_g<float, 1024, 2, true, 7, 4>},
     {1024, 2, TFHEB_SPLIT_FP32, 8, 8, true, 8.60, launch_warp_split2<8>, 1, 23},
-    {1024, 2, TFHEB_SPLIT_FP32, 4, 8, true, 6.12, launch_warp_split2<4>, 1, 23},
-    {1024, 2, TFHEB_SPLIT_FP32, 1, 4, false, 3.77, launch_g<float, 1024, 2, true, 1, 4>},
+    {1024, 2, TFHEB_SPLIT_FP32, 4, 8, false, 4.82, launch_warp_split2<4>, 1, 23},
     {1024, 2, TFHEB_SPLIT_FP32, 1, 2, false, 2.58, launch_latency<float, 2, 1>},
     {1024, 2, TFHEB_SPLIT_FP32, 1, 2, false, 1.82, launch_latency<float, 2, 2>, 0, 32, 2},
     {1024, 2, TFHEB_FP64, 4, 4, true, 7.90, launch_g<double, 1024, 2, false, 4, 4, false>},
     {1024, 2, TFHEB_FP64, 4, 4, true, 8.38, launch_g<double, 1024, 2, false, 4, 4>},
-    {1024, 2, TFHEB_FP64, 8, 8, true, 11.66, launch_warp<false, 2, 8, 8>},
-    {1024, 2, TFHEB_FP64, 4, 8, true, 7.83, launch_warp<false, 2, 4, 8>},
-    {1024, 2, TFHEB_FP64, 1, 4, false, 3.44, launch_g<double, 1024, 2, false, 1, 4>},
+    {1024, 2, TFHEB_FP64, 8, 8, true, 11.66, launch_warp<false, 2, 8, 8, false>},
+    {1024, 2, TFHEB_FP64, 4, 8, false, 6.35, launch_warp<false, 2, 4, 8, true>},
     {1024, 2, TFHEB_FP64, 1, 2, false, 2.98, launch_latency<double, 2, 1>},
     {1024, 2, TFHEB_FP64, 1, 1, false, 2.10, launch_latency<double, 2, 2>, 0, 32, 2},
 };
@@ -697,7 +696,7 @@ static int wave_need(int count, int sms) { return 2 * count <= sms ? 0 : (count 
 
 // The first wave's bootstraps of a rest of `count` (fewer than a wave of `big`): all of them, or as many whole
 // bootstraps per SM as give the least sum of measured times (*us) over the waves.  600 FP64 bootstraps run as
-// 592 + 8 (6.2 + 1.6 ms; 10.1 ms in one wave of eight per SM), 160 split ones as 148 + 12 (1.84 + 1.24 ms against
+// 592 + 8 (5.2 + 1.6 ms; 10.1 ms in one wave of eight per SM), 160 split ones as 148 + 12 (1.84 + 1.24 ms against
 // 3.68 two per SM).
 static int first_wave(const tfheb_params &p, int big, int count, int sms, const BrChoice &choice, float *us) {
     const int need = wave_need(count, sms);
@@ -717,7 +716,7 @@ static int first_wave(const tfheb_params &p, int big, int count, int sms, const 
 }
 
 // Full waves of the chosen variant (SMs x G bootstraps each), then the rest in waves of whatever runs that many
-// per CTA fastest: 4096 split bootstraps are 3 waves of 1184 and 544 spread over 4 per CTA (20.7 + 4.95 ms,
+// per CTA fastest: 4096 split bootstraps are 3 waves of 1184 and 544 spread over 4 per CTA (20.7 + 3.9 ms,
 // where a fourth packed wave takes 6.9).  A lone bootstrap runs its 630 steps in 1.24 ms on two SMs, 1.84 ms
 // on one.
 cudaError_t launch_blind_rotate(const tfheb_params &p, int precision, const DeviceBsk &bsk, const int32_t *bara,

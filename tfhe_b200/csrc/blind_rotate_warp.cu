@@ -24,8 +24,9 @@
 // {hi, lo} limb pairs one word at a time.
 // Measured, one wave of 1184 bootstraps (eight per SM): split 6.89 ms against 7.71 ms per 1036 for the paired
 // kernel (1.37 against 1.75 us per bootstrap step and SM), FP64 10.1 ms against 12.4 ms for two waves of 592 on
-// blind_rotate_kernel.  With at most four per SM each scheduler has one warp and its latencies show (split 4.97 ms
-// per 592, FP64 6.6 ms), so smaller waves stay with the other kernels.
+// blind_rotate_kernel.  One warp per bootstrap leaves a scheduler one warp at four per SM, and its latencies
+// show (split 4.97 ms per 592, FP64 6.6 ms); with two warps per bootstrap (DUO) that wave takes 3.91 and 5.24 ms,
+// against 4.95 and 6.22 ms for the paired and the team kernel.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -370,7 +371,9 @@ struct WarpFft {
 // spectra overwrite them once they have been read.  FP64: the two outputs' accumulators, 64 words per lane
 // each, then the rotated words.  Both: the exchange region from 192 on.  The key ring's unit is 16 KB: one
 // output's slots of a digit pair (split), or one digit's row (FP64); the ring holds whole steps.
-template <class Ops, int L, int D>
+// DUO: a quadrant's two warps share one bootstrap and its 512 columns: spectra or (FP64) two outputs'
+// accumulators per warp, rotated words, an exchange region per warp.
+template <class Ops, int L, int D, bool DUO = false>
 struct WarpLayout {
     static constexpr int KP1 = 2, KPL = KP1 * L;
     static constexpr uint32_t half = (uint32_t)kWarpM * 16;  // one output's slots of one key row
@@ -383,7 +386,8 @@ struct WarpLayout {
     static constexpr size_t accs = (mid + Ops::mid_bytes + 127) / 128 * 128;
     static constexpr size_t acc_bytes = 4 * (size_t)KP1 * kWarpN;
     static constexpr size_t bytes(int G) { return accs + (size_t)G * acc_bytes; }
-    static constexpr uint32_t col_xr = 128, col_exch = 192;
+    static constexpr bool split = std::is_same_v<Ops, PairOps>;
+    static constexpr uint32_t col_xr = !DUO ? 128 : split ? 192 : 256, col_exch = !DUO ? 192 : split ? 256 : 320;
     static_assert(D % per_step == 0, "ring slots fixed within a step");
     static_assert(KPL * 32 <= 192 && KPL % 2 == 0, "spectra columns");
     static_assert(bytes(kWarpTeams) <= 227 * 1024, "shared memory of the variant");
@@ -401,10 +405,16 @@ __device__ __forceinline__ float2 digit_pair(uint32_t a, uint32_t b) {
 // Three warpgroups: eight warps of which the first args.teams run a bootstrap each, with 232 registers, and one
 // whose first thread streams the key in the order of the multiply-accumulates (the other three warps
 // only take part in the register split: a ninth warp alone would cap all of them at 168).
-template <bool SPLIT, int L, int D>
+// DUO, for at most four bootstraps per CTA: warps w and w + 4, which share a scheduler and a TMEM quadrant, run one
+// bootstrap together, so that each scheduler still has two warps to choose from.  Warp (role) u keeps
+// polynomial u of the accumulator and computes output u.  Split: the digit pairs go to the two in turn, and both
+// read all spectra from TMEM.  FP64: each transforms its polynomial's digits and multiplies them with the key of
+// both outputs; the two partial sums of an output meet at the end (FP64 sums round to the exact integers in
+// any order).
+template <bool SPLIT, int L, int D, bool DUO>
 __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_kernel(const BrArgs args) {
     using Ops = std::conditional_t<SPLIT, PairOps, DoubleOps>;
-    using Lay = WarpLayout<Ops, L, D>;
+    using Lay = WarpLayout<Ops, L, D, DUO>;
     constexpr int N = kWarpN, M = kWarpM, NT = kWarpNT, KP1 = 2, KPL = KP1 * L;
     using F = WarpFft<Ops>;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -477,24 +487,34 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
         return;
     }
     asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
-    if (warp >= active) return;  // no TMEM use, not counted in any barrier below
+    const int team = DUO ? warp & 3 : warp, role = DUO ? warp >> 2 : 0;
+    if (team >= active) return;  // no TMEM use, not counted in any barrier below
 
     // ---- consumer warps ----
-    const int boot = blockIdx.x * G + warp;
-    uint32_t *s_acc = reinterpret_cast<uint32_t *>(smem + Lay::accs + (size_t)warp * Lay::acc_bytes);
+    const int boot = blockIdx.x * G + team;
+    uint32_t *s_acc = reinterpret_cast<uint32_t *>(smem + Lay::accs + (size_t)team * Lay::acc_bytes);
     const void *s_tab = smem + Lay::tables, *s_mid = smem + Lay::mid;
-    const uint32_t tmem = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * 256);
-    const typename Ops::Exch exch{tmem + Lay::col_exch};
+    const uint32_t tmem = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (DUO ? 0u : (uint32_t)((warp >> 2) * 256));
+    const typename Ops::Exch exch{tmem + Lay::col_exch + (uint32_t)(64 * role)};
+    // DUO: both warps of the bootstrap, their TMEM accesses before it ordered before those after it
+    auto duo_sync = [&] {
+        if constexpr (DUO) {
+            tmem_fence_before_sync();
+            team_sync(2 + team, 64);
+            tmem_fence_after_sync();
+        }
+    };
+    const int first = lane + 32 * role, stride = DUO ? 64 : 32;
 
     const int32_t *my_bara = args.bara + (size_t)boot * args.bara_stride;
     if (args.acc_in) {
         const uint32_t *src = reinterpret_cast<const uint32_t *>(args.acc_in) + (size_t)boot * KP1 * N;
-        for (int i = lane; i < KP1 * N; i += 32) s_acc[i] = src[i];
+        for (int i = first; i < KP1 * N; i += stride) s_acc[i] = src[i];
     } else {
         // acc = (0, X^{2N-barb} * [mu,...,mu])  (lwe-bootstrapping-functions-fft.cpp:142-145)
         const int e = 2 * N - my_bara[args.nsteps];
-        for (int i = lane; i < N; i += 32) s_acc[i] = 0u;
-        for (int j = lane; j < N; j += 32) {
+        for (int i = first; i < N; i += stride) s_acc[i] = 0u;
+        for (int j = first; j < N; j += stride) {
             int src = j - e;
             uint32_t neg = 0;
             while (src < 0) {
@@ -505,6 +525,7 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
         }
     }
     __syncwarp();
+    duo_sync();
 
     // gadget constants (tgsw.cpp:7-29)
     const int Bgbit = args.Bgbit;
@@ -528,30 +549,33 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
         //    scheduler ran 14.9k cycles a step with this loop, 16.0k without).
         {
             const uint32_t rot = 4u * (uint32_t)(lane - ai);  // byte index of e
+            const uint32_t *polys = s_acc + role * N;         // DUO: the warp's own polynomial only
 #pragma unroll 1
             for (int i0 = 0; i0 < 32; i0 += 16) {
                 uint32_t x0[16], x1[16];
-                const uint32_t *own = s_acc + lane + 32 * i0;
+                const uint32_t *own = polys + lane + 32 * i0;
 #pragma unroll
                 for (int i = 0; i < 16; i++) {
                     const uint32_t e = rot + 128u * (uint32_t)(i0 + i);
                     const uint32_t neg = (uint32_t)((int32_t)(e << 19) >> 31);
                     const uint32_t on = offset - neg;
                     const uint32_t *src =
-                        reinterpret_cast<const uint32_t *>(reinterpret_cast<const char *>(s_acc) + (e & 4095u));
+                        reinterpret_cast<const uint32_t *>(reinterpret_cast<const char *>(polys) + (e & 4095u));
                     x0[i] = ((src[0] ^ neg) + (on - own[32 * i])) >> (SPLIT ? kDigitShift : 0);
-                    x1[i] = ((src[N] ^ neg) + (on - own[32 * i + N])) >> (SPLIT ? kDigitShift : 0);
+                    if constexpr (!DUO) x1[i] = ((src[N] ^ neg) + (on - own[32 * i + N])) >> (SPLIT ? kDigitShift : 0);
                 }
-                tmem_st16(tmem + Lay::col_xr + (uint32_t)i0, x0);
-                tmem_st16(tmem + Lay::col_xr + 32u + (uint32_t)i0, x1);
+                tmem_st16(tmem + Lay::col_xr + (uint32_t)(32 * role + i0), x0);
+                if constexpr (!DUO) tmem_st16(tmem + Lay::col_xr + 32u + (uint32_t)i0, x1);
             }
         }
         tmem_wait_st();
 
         if constexpr (SPLIT) {
-            // 2. digits two at a time, forward transforms, spectra to TMEM
+            // 2. digits two at a time, forward transforms, spectra to TMEM (DUO: which the other warp has read
+            //    when it gets here)
+            duo_sync();
 #pragma unroll 1
-            for (int d0 = 0; d0 < KPL; d0 += 2) {
+            for (int d0 = 2 * role; d0 < KPL; d0 += DUO ? 4 : 2) {
                 const int u0 = d0 / L, u1 = (d0 + 1) / L;
                 // digit q of a word: its bits under the exponent of 2^23 are the float 2^23 + d 2^sh; times
                 // 2^-sh, minus (2^23 2^-sh + Bg/2): exact, one operation for the pair
@@ -586,12 +610,13 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
                 }
             }
             tmem_wait_st();
+            duo_sync();
 
             // 3. per output polynomial: multiply-accumulate over the digits against the key, each accumulator the
             //    pair of the key's limbs (hi, lo), then both limbs' inverse transforms as one pair, exact
             //    rounding, accumulate
 #pragma unroll 1
-            for (int v = 0; v < KP1; v++) {
+            for (int v = role; v < (DUO ? role + 1 : KP1); v++) {
                 cpair acc[2][kR];
 #pragma unroll
                 for (int h = 0; h < 2; h++)
@@ -670,13 +695,14 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
             // 2. per digit: forward transform, then its products with the key row, added to both outputs'
             //    accumulators in TMEM (with the 64 registers of a transform, 128 more for accumulators
             //    would not fit); they start at zero
+            const uint32_t sums = tmem + (uint32_t)(128 * role);
             {
                 const uint32_t zero[32] = {};
 #pragma unroll
-                for (int q = 0; q < 4; q++) tmem_st32p(tmem + (uint32_t)(32 * q), zero);
+                for (int q = 0; q < 4; q++) tmem_st32p(sums + (uint32_t)(32 * q), zero);
             }
 #pragma unroll 1
-            for (int d = 0; d < KPL; d++) {
+            for (int d = role * L; d < (DUO ? (role + 1) * L : KPL); d++) {
                 const int u = d / L, sh = 32 - (d - u * L + 1) * Bgbit;
                 // the masked word under the exponent of 2^52 is 1.5 * 2^52 + digit * 2^sh, as in the split form
                 const uint32_t mask = maskBg << sh;
@@ -701,12 +727,12 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
                 const double2 *kp = reinterpret_cast<const double2 *>(smem + Lay::ring + (size_t)slot * Lay::unit) + lane;
                 // quarters (output v, butterfly h), the next one's accumulators loading meanwhile
                 uint32_t a[2][32];
-                tmem_ld32(tmem, a[0]);
+                tmem_ld32(sums, a[0]);
                 tmem_wait_ld32(a[0]);
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
                     uint32_t *acc = a[q & 1];
-                    if (q < 3) tmem_ld32(tmem + (uint32_t)(32 * q + 32), a[(q + 1) & 1]);
+                    if (q < 3) tmem_ld32(sums + (uint32_t)(32 * q + 32), a[(q + 1) & 1]);
                     uint32_t w[32];
 #pragma unroll
                     for (int r = 0; r < kR; r++) {
@@ -716,7 +742,7 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
                         cmac(p, z[q & 1][r], cplx<double>{k.x, k.y});
                         F::put(w, 4 * r, 4 * r + 2, p);
                     }
-                    tmem_st32p(tmem + (uint32_t)(32 * q), w);
+                    tmem_st32p(sums + (uint32_t)(32 * q), w);
                     if (q < 3) tmem_wait_ld32(a[(q + 1) & 1]);
                 }
                 __syncwarp();
@@ -724,17 +750,33 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
                 tmem_wait_st();
             }
             // 3. per output polynomial: inverse transform, exact rounding, accumulate
+            duo_sync();
 #pragma unroll 1
-            for (int v = 0; v < KP1; v++) {
+            for (int v = role; v < (DUO ? role + 1 : KP1); v++) {
                 uint32_t a[64];
-                tmem_ld32(tmem + (uint32_t)(64 * v), a);
-                tmem_ld32(tmem + (uint32_t)(64 * v + 32), a + 32);
+                tmem_ld32(sums + (uint32_t)(64 * v), a);
+                tmem_ld32(sums + (uint32_t)(64 * v + 32), a + 32);
                 tmem_wait_ld64(a);
                 cplx<double> z[2][kR];
 #pragma unroll
                 for (int h = 0; h < 2; h++)
 #pragma unroll
                     for (int r = 0; r < kR; r++) F::get(z[h][r], a, 32 * h + 4 * r, 32 * h + 4 * r + 2);
+                if constexpr (DUO) {  // the other warp's part; its next step's zeros wait for these loads
+                    uint32_t b[64];
+                    tmem_ld32(tmem + (uint32_t)(128 * (role ^ 1) + 64 * v), b);
+                    tmem_ld32(tmem + (uint32_t)(128 * (role ^ 1) + 64 * v + 32), b + 32);
+                    tmem_wait_ld64(b);
+                    duo_sync();
+#pragma unroll
+                    for (int h = 0; h < 2; h++)
+#pragma unroll
+                        for (int r = 0; r < kR; r++) {
+                            cplx<double> p;
+                            F::get(p, b, 32 * h + 4 * r, 32 * h + 4 * r + 2);
+                            z[h][r] = cadd(z[h][r], p);
+                        }
+                }
                 F::inverse(z, exch, s_tab, s_mid, lane);
                 uint32_t *poly = s_acc + v * N + lane;
 #pragma unroll
@@ -751,22 +793,22 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
     }
 
     uint32_t *dst = reinterpret_cast<uint32_t *>(args.acc_out) + (size_t)boot * KP1 * N;
-    for (int i = lane; i < KP1 * N; i += 32) dst[i] = s_acc[i];
+    for (int i = lane + role * N; i < (DUO ? (role + 1) * N : KP1 * N); i += 32) dst[i] = s_acc[i];
 
     // every consumer's TMEM accesses are complete; warp 0 frees the columns
     tmem_fence_before_sync();
-    team_sync(1, active * 32);
+    team_sync(1, active * (DUO ? 64 : 32));
     tmem_fence_after_sync();
     __syncwarp();
     if (warp == 0) tmem_free(tmem_base, 512);
 }
 
-template <bool SPLIT, int L, int G, int D>
+template <bool SPLIT, int L, int G, int D, bool DUO>
 cudaError_t launch_warp(const BrArgs &args, cudaStream_t s) {
-    using Lay = WarpLayout<std::conditional_t<SPLIT, PairOps, DoubleOps>, L, D>;
-    static_assert(G <= kWarpTeams, "one warp per bootstrap");
+    using Lay = WarpLayout<std::conditional_t<SPLIT, PairOps, DoubleOps>, L, D, DUO>;
+    static_assert(G <= (DUO ? kWarpTeams / 2 : kWarpTeams), "one warp per bootstrap, or two");
     if (SPLIT && !args.bsk2) return cudaErrorInvalidValue;
-    auto kern = blind_rotate_warp_kernel<SPLIT, L, D>;
+    auto kern = blind_rotate_warp_kernel<SPLIT, L, D, DUO>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::bytes(kWarpTeams));
     if (e != cudaSuccess) return e;
     BrArgs a = args;
@@ -775,11 +817,15 @@ cudaError_t launch_warp(const BrArgs &args, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-template cudaError_t launch_warp<true, 3, 8, 6>(const BrArgs &, cudaStream_t);
-template cudaError_t launch_warp<false, 3, 8, 6>(const BrArgs &, cudaStream_t);
-template cudaError_t launch_warp<true, 2, 8, 8>(const BrArgs &, cudaStream_t);
-template cudaError_t launch_warp<true, 2, 4, 8>(const BrArgs &, cudaStream_t);
-template cudaError_t launch_warp<false, 2, 8, 8>(const BrArgs &, cudaStream_t);
-template cudaError_t launch_warp<false, 2, 4, 8>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp<true, 3, 8, 6, false>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp<true, 3, 4, 6, true>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp<true, 3, 3, 6, true>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp<false, 3, 8, 6, false>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp<false, 3, 4, 6, true>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp<false, 3, 3, 6, true>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp<true, 2, 8, 8, false>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp<true, 2, 4, 8, true>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp<false, 2, 8, 8, false>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp<false, 2, 4, 8, true>(const BrArgs &, cudaStream_t);
 
 }  // namespace tfheb

@@ -210,7 +210,7 @@ cudaError_t launch_paired_il3(const BrArgs &a, cudaStream_t s);
 template <int N, int L, int G, int D, int XB>
 cudaError_t launch_paired_il7(const BrArgs &a, cudaStream_t s);
 // blind_rotate_warp.cu: one warp per bootstrap, up to eight per CTA, exchanges in tensor memory (N = 1024)
-template <bool SPLIT, int L, int G, int D>
+template <bool SPLIT, int L, int G, int D, bool DUO>
 cudaError_t launch_warp(const BrArgs &a, cudaStream_t s);
 // blind_rotate_latency.cu: one bootstrap per CTA (C = 1) or per cluster of two (C = 2), N = 1024
 template <typename T, int L, int C>
