@@ -1,7 +1,7 @@
 """The one-warp-per-bootstrap blind rotation (eight bootstraps per CTA, FFT exchanges in tensor memory): bit for
 bit the rotation of the team kernels, which the oracle pins, with full, partly filled and single CTAs, over
 the fewest steps, on both gadget lengths; its form with two warps per bootstrap and the kernels for a few
-bootstraps (one per SM, one per cluster of two) against it; the cut of a batch into waves; digits too wide for the split form; stalled key streams."""
+bootstraps (one per SM, one per cluster of two) against it; its form for the larger ring; the cut of a batch into waves; digits too wide for the split form; stalled key streams."""
 import numpy as np
 import pytest
 
@@ -25,6 +25,13 @@ def keys():
             made[l, Bgbit][1].to_device(0)
         return made[l, Bgbit]
     return get
+
+
+@pytest.fixture(scope="module")
+def large_keys():
+    sk, ck = tb.keygen(tb.make_params(9, 2048, 1, 3, 8, 8, 2), seed=79)
+    ck.to_device(0)
+    return sk, ck
 
 
 def packed_eight(ck, precision):
@@ -59,6 +66,23 @@ def test_rotation_equals_the_team_kernel(keys, l, Bgbit, precision, nsteps, coun
     assert (got[:count] == want).all()
     assert (got[count:] == want[0]).all()
     ck.set_br_variant(precision, 0)
+
+
+# N = 2048, two warps per bootstrap, four bootstraps per CTA
+@pytest.mark.parametrize("count", [1, 4, 5, 591])
+@pytest.mark.parametrize("nsteps", [1, 2, 3])
+@pytest.mark.parametrize("precision", [tb.FP64, tb.SPLIT_FP32])
+def test_large_ring_rotation_equals_the_team_kernel(large_keys, precision, nsteps, count):
+    sk, ck = large_keys
+    rng = np.random.default_rng(3 * count + nsteps)
+    acc = rng.integers(-2**31, 2**31, (592, 2, 2048)).astype(np.int32)
+    bara = rng.integers(0, 4096, (592, nsteps)).astype(np.int32)
+    bara.flat[:5] = [0, 1, 2047, 2048, 4095]  # the ends of the rotation's range, both parities
+    acc[count:], bara[count:] = acc[:1], bara[:1]
+    G, D = ck.br_variants(precision)
+    got = rotate(ck, precision, int(np.flatnonzero(G == 4)[0]), bara, acc, nsteps)
+    want = rotate(ck, precision, 0, bara[:count], acc[:count], nsteps)
+    assert (got[:count] == want).all() and (got[count:] == want[0]).all()
 
 
 # one bootstrap on two SMs (at most 74 of 148), one per SM, both in turn, and two warps for each of 3 or 4 per SM

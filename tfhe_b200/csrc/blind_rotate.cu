@@ -486,11 +486,13 @@ int blind_rotate_supported(const tfheb_params &p) {
 // The warp kernel's split form keeps a word's digits in a float's mantissa: parameter sets with wider
 // digits (l Bgbit > 23; the reference's sets have 21 and 20) run what was the default before it.
 static cudaError_t launch_warp_split3(const BrArgs &a, cudaStream_t s) {
-    return 3 * a.Bgbit <= 23 ? launch_warp<true, 3, 8, 6, false>(a, s) : launch_paired_il3<1024, 3, 7, 12, 1>(a, s);
+    return 3 * a.Bgbit <= 23 ? launch_warp<true, 3, 8, 6>(a, s) : launch_paired_il3<1024, 3, 7, 12, 1>(a, s);
 }
 template <int G>
 static cudaError_t launch_warp_split2(const BrArgs &a, cudaStream_t s) {
-    return 2 * a.Bgbit <= 23 ? launch_warp<true, 2, G, 8, G <= 4>(a, s) : launch_g<float, 1024, 2, true, 7, 4>(a, s);
+    if (2 * a.Bgbit > 23) return launch_g<float, 1024, 2, true, 7, 4>(a, s);
+    if constexpr (G == 8) return launch_warp<true, 2, 8, 8>(a, s);
+    else return launch_warp_duo<true, 2, G, 8>(a, s);
 }
 
 // Compiled launch variants: (ring degree, gadget length, precision, bootstraps per CTA G, key-ring depth D).
@@ -542,8 +544,8 @@ static const BrVariant kBrVariants[] = {
     {1024, 3, TFHEB_SPLIT_FP32, 3, 12, false, 7.51, launch_paired_il3<1024, 3, 3, 12, 1>, 1},
     // the warp kernel with two warps per bootstrap: 3.91 ms per wave of four per SM, against 4.95 ms for the paired
     // kernel and 4.97 ms for one warp per bootstrap (FP64: 5.24 ms against 6.22 and 6.6)
-    {1024, 3, TFHEB_SPLIT_FP32, 4, 6, false, 6.21, launch_warp<true, 3, 4, 6, true>, 1, 23},
-    {1024, 3, TFHEB_SPLIT_FP32, 3, 6, false, 6.14, launch_warp<true, 3, 3, 6, true>, 1, 23},
+    {1024, 3, TFHEB_SPLIT_FP32, 4, 6, false, 6.21, launch_warp_duo<true, 3, 4, 6>, 1, 23},
+    {1024, 3, TFHEB_SPLIT_FP32, 3, 6, false, 6.14, launch_warp_duo<true, 3, 3, 6>, 1, 23},
     // few bootstraps (blind_rotate_latency.cu; D counts 48 KB stages): one per CTA, one per two CTAs
     {1024, 3, TFHEB_SPLIT_FP32, 1, 2, false, 2.92, launch_latency<float, 3, 1>},
     {1024, 3, TFHEB_SPLIT_FP32, 1, 2, false, 1.96, launch_latency<float, 3, 2>, 0, 32, 2},
@@ -553,9 +555,9 @@ static const BrVariant kBrVariants[] = {
     {1024, 3, TFHEB_FP64, 4, 4, true, 11.04, launch_g<double, 1024, 3, false, 4, 4>},
     {1024, 3, TFHEB_FP64, 3, 4, true, 8.58, launch_g<double, 1024, 3, false, 3, 4>},
     {1024, 3, TFHEB_FP64, 2, 4, true, 5.86, launch_g<double, 1024, 3, false, 2, 4>},
-    {1024, 3, TFHEB_FP64, 8, 6, true, 16.08, launch_warp<false, 3, 8, 6, false>},
-    {1024, 3, TFHEB_FP64, 4, 6, false, 8.32, launch_warp<false, 3, 4, 6, true>},
-    {1024, 3, TFHEB_FP64, 3, 6, false, 8.34, launch_warp<false, 3, 3, 6, true>},
+    {1024, 3, TFHEB_FP64, 8, 6, true, 16.08, launch_warp<false, 3, 8, 6>},
+    {1024, 3, TFHEB_FP64, 4, 6, false, 8.32, launch_warp_duo<false, 3, 4, 6>},
+    {1024, 3, TFHEB_FP64, 3, 6, false, 8.34, launch_warp_duo<false, 3, 3, 6>},
     {1024, 3, TFHEB_FP64, 1, 2, false, 3.67, launch_latency<double, 3, 1>},
     {1024, 3, TFHEB_FP64, 1, 1, false, 2.47, launch_latency<double, 3, 2>, 0, 32, 2},
     // the split default at N = 2048: the N = 1024 default's structure with three teams and a 6-deep
@@ -573,9 +575,13 @@ static const BrVariant kBrVariants[] = {
     {2048, 3, TFHEB_SPLIT_FP32, 1, 3, false, 8.00, launch_g<float, 2048, 3, true, 1, 3>},
     {2048, 3, TFHEB_SPLIT_FP32, 2, 4, true, 12.86, launch_paired<2048, 3, 2, 4, 2, false>, 1},
     {2048, 3, TFHEB_SPLIT_FP32, 2, 4, true, 10.56, launch_paired<2048, 3, 2, 4, 2, true>, 1},
+    // the warp kernel, D counting 32 KB units: 10.63 ms per wave of 592, against 10.19 ms per 444 for the first entry
+    {2048, 3, TFHEB_SPLIT_FP32, 4, 3, true, 13.28, launch_warp_big<true, 3, 4>, 1},
+    // FP64: the last entry is the default (14.86 ms per wave of 592, against 10.35 ms per 296 for the first)
     {2048, 3, TFHEB_FP64, 2, 3, true, 12.94, launch_g<double, 2048, 3, false, 2, 3, false>},
     {2048, 3, TFHEB_FP64, 2, 3, true, 14.37, launch_g<double, 2048, 3, false, 2, 3>},
     {2048, 3, TFHEB_FP64, 1, 4, true, 7.66, launch_g<double, 2048, 3, false, 1, 4>},
+    {2048, 3, TFHEB_FP64, 4, 3, true, 18.58, launch_warp_big<false, 3, 4>},
     {512, 3, TFHEB_SPLIT_FP32, 8, 4, true, 0, launch_g<float, 512, 3, true, 8, 4>},
     {512, 3, TFHEB_FP64, 8, 4, true, 0, launch_g<double, 512, 3, false, 8, 4>},
     // the 80-bit parameter set (n = 500, l = 2, Bgbit = 10; tfhe_gate_bootstrapping.cpp:23-48)
@@ -586,8 +592,8 @@ static const BrVariant kBrVariants[] = {
     {1024, 2, TFHEB_SPLIT_FP32, 1, 2, false, 1.82, launch_latency<float, 2, 2>, 0, 32, 2},
     {1024, 2, TFHEB_FP64, 4, 4, true, 7.90, launch_g<double, 1024, 2, false, 4, 4, false>},
     {1024, 2, TFHEB_FP64, 4, 4, true, 8.38, launch_g<double, 1024, 2, false, 4, 4>},
-    {1024, 2, TFHEB_FP64, 8, 8, true, 11.66, launch_warp<false, 2, 8, 8, false>},
-    {1024, 2, TFHEB_FP64, 4, 8, false, 6.35, launch_warp<false, 2, 4, 8, true>},
+    {1024, 2, TFHEB_FP64, 8, 8, true, 11.66, launch_warp<false, 2, 8, 8>},
+    {1024, 2, TFHEB_FP64, 4, 8, false, 6.35, launch_warp_duo<false, 2, 4, 8>},
     {1024, 2, TFHEB_FP64, 1, 2, false, 2.98, launch_latency<double, 2, 1>},
     {1024, 2, TFHEB_FP64, 1, 1, false, 2.10, launch_latency<double, 2, 2>, 0, 32, 2},
 };

@@ -27,6 +27,8 @@
 // blind_rotate_kernel.  One warp per bootstrap leaves a scheduler one warp at four per SM, and its latencies
 // show (split 4.97 ms per 592, FP64 6.6 ms); with two warps per bootstrap (DUO) that wave takes 3.91 and 5.24 ms,
 // against 4.95 and 6.22 ms for the paired and the team kernel.
+// N = 2048: two warps per bootstrap, each with half of every transform's points (big below): one wave of 592 takes 10.6 ms
+// split and 14.9 ms FP64, against 10.2 ms per 444 for the paired kernel and 10.35 ms per 296 for the team kernel.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -43,7 +45,11 @@ namespace tfheb {
 namespace {
 
 constexpr int kWarpTeams = 8;  // most bootstraps per CTA
-constexpr int kWarpN = 1024, kWarpM = kWarpN / 2, kWarpNT = kWarpM / kR;  // ring degree, points, virtual team threads
+enum class WarpMode {
+    solo,  // N = 1024, one warp per bootstrap
+    duo,   // N = 1024, two warps per bootstrap, each with half of the transforms
+    big    // N = 2048, two warps per bootstrap, each with half of every transform's points
+};
 
 // ---- the exchange passes -----------------------------------------------------------------------
 // v[64]: the warp's 16 points per lane, 4 words each (two components ri = re, im of two words e: the
@@ -53,9 +59,33 @@ constexpr int kWarpN = 1024, kWarpM = kWarpN / 2, kWarpNT = kWarpM / kR;  // rin
 // S16: 16 words per store instruction instead of 32.  The doubles' results reach the registers of a store with
 // fewer moves that way (8.0k instructions per bootstrap step against 8.7k, 10.1 ms per 1184 bootstraps
 // against 10.5); packed floats need next to none either way.
+// swap() (BIG): the two warps of a team, `half` 0 and 1, trade the group bit of the registers (v[0..31], v[32..63])
+// for their own: warp w gets group w of warp 0, then group w of warp 1.  Every lane keeps its place.
 template <bool S16>
 struct WarpExch {
     uint32_t col;
+    int bar;  // BIG: named barrier of the team's two warps
+    __device__ __forceinline__ void team() const {
+        tmem_fence_before_sync();
+        team_sync(bar, 64);
+        tmem_fence_after_sync();
+    }
+    __device__ __forceinline__ void swap(uint32_t (&v)[64], int half) const {
+        if constexpr (S16) {
+#pragma unroll
+            for (int c = 0; c < 64; c += 16) tmem_st16(col + (uint32_t)c, v + c);
+        } else {
+            tmem_st32p(col, v);
+            tmem_st32p(col + 32u, v + 32);
+        }
+        tmem_wait_st();
+        team();
+        const uint32_t first = col - (uint32_t)(256 * half) + (uint32_t)(32 * half);
+        tmem_ld32(first, v);
+        tmem_ld32(first + 256u, v + 32);
+        tmem_wait_ld64(v);
+        team();  // the regions are free again
+    }
     __device__ __forceinline__ void forward(uint32_t (&v)[64]) const {
         if constexpr (S16) {
 #pragma unroll
@@ -125,7 +155,9 @@ __device__ __forceinline__ void from_words(double &c, uint32_t w0, uint32_t w1) 
 // Arithmetic of one transform of packed FP32 pairs (TeamFft2's) or of doubles (TeamFft<double>'s).  A packed
 // instruction takes one word for both halves of an operand, or its negation, at no cost, so the factors are
 // single words: TeamFft<float>'s table, two factors per 16-byte load.
+template <int M>
 struct PairOps {
+    static constexpr int NT = M / kR, st1 = M / (kR * kR);  // virtual team threads, stage 1's stride
     using point = cpair;
     using factor = float2;
     using Exch = WarpExch<false>;
@@ -153,33 +185,35 @@ struct PairOps {
         a = INV ? pmulconj(a, wr, wi, nwi) : pmul(a, wr, wi, nwi);
     }
     template <bool INV>
-    __device__ static __forceinline__ void fold(point *x) { TeamFft2<kWarpM>::fold_consts<INV>(x); }
-    // tables: stage 0 factors 2 q, 2 q + 1 of virtual thread t; stage 1 factors 2 q + 1, 2 q + 2 of n2; mid-table
-    // factors 2 i, 2 i + 1 of the lane's row
-    static constexpr size_t table_bytes = tw_table_bytes<float, kWarpM>(), mid_bytes = 4 * 9 * 16;
+    __device__ static __forceinline__ void fold(point *x) { TeamFft2<M>::fold_consts<INV>(x); }
+    // tables: stage 0 factors 2 q, 2 q + 1 at t (see WarpFft); stages 1 and 2 factors 2 q + 1, 2 q + 2 at n;
+    // mid-table factors 2 i, 2 i + 1 of a row
+    static constexpr size_t table_bytes = tw_table_bytes<float, M>(), row_bytes = 9 * 16;
     __device__ static __forceinline__ void two(const void *tab, int at, factor &a, factor &b) {
         const float4 w = reinterpret_cast<const float4 *>(tab)[at];
         a = make_float2(w.x, w.y);
         b = make_float2(w.z, w.w);
     }
     __device__ static __forceinline__ void stage0(const void *tab, int q, int t, factor &a, factor &b) {
-        two(tab, q * kWarpNT + t, a, b);
+        two(tab, q * NT + t, a, b);
     }
-    __device__ static __forceinline__ void stage1(const void *tab, int q, int n2, factor &a, factor &b) {
-        two(tab, tw4_offset<kWarpM>(1) + q * kR + n2, a, b);
+    template <int S>
+    __device__ static __forceinline__ void stage(const void *tab, int q, int n, factor &a, factor &b) {
+        two(tab, tw4_offset<M>(S) + q * (S == 1 ? st1 : st1 / kR) + n, a, b);
     }
     __device__ static __forceinline__ void mid(const void *tab, int i, int row, factor &a, factor &b) {
         two(tab, row * 9 + i, a, b);
     }
-    // entry f of a mid-table row = stage 1's factor of (k1, n2), 1 where k1 = 0
-    __device__ static __forceinline__ void put_mid(void *mid_tab, const void *tab, int row, int f, int k1, int n2) {
-        const factor *w = static_cast<const factor *>(tab) + 2 * (tw4_offset<kWarpM>(1) + n2);
+    // entry f of a mid-table row = stage 1's factor of (k1, n), 1 where k1 = 0
+    __device__ static __forceinline__ void put_mid(void *mid_tab, const void *tab, int row, int f, int k1, int n) {
+        const factor *w = static_cast<const factor *>(tab) + 2 * (tw4_offset<M>(1) + n);
         static_cast<factor *>(mid_tab)[row * 18 + f] =
-            k1 ? w[2 * kR * ((k1 - 1) / 2) + (k1 - 1) % 2] : make_float2(1.0f, 0.0f);
+            k1 ? w[2 * st1 * ((k1 - 1) / 2) + (k1 - 1) % 2] : make_float2(1.0f, 0.0f);
     }
 };
-
+template <int M>
 struct DoubleOps {
+    static constexpr int NT = M / kR, st1 = M / (kR * kR);
     using point = cplx<double>;
     using factor = cplx<double>;
     using Exch = WarpExch<true>;
@@ -206,30 +240,42 @@ struct DoubleOps {
     template <bool INV>
     __device__ static __forceinline__ void mul(point &a, factor w) { a = INV ? cmulconj(a, w) : cmul(a, w); }
     template <bool INV>
-    __device__ static __forceinline__ void fold(point *x) { TeamFft<double, kWarpM, kR>::template fold_consts<INV>(x); }
-    static constexpr size_t table_bytes = tw_table_bytes<double, kWarpM>(), mid_bytes = 4 * 17 * 16;
+    __device__ static __forceinline__ void fold(point *x) { TeamFft<double, M, kR>::template fold_consts<INV>(x); }
+    static constexpr size_t table_bytes = tw_table_bytes<double, M>(), row_bytes = 17 * 16;
     __device__ static __forceinline__ void stage0(const void *tab, int q, int t, factor &a, factor &b) {
-        const factor *w = static_cast<const factor *>(tab) + 2 * q * kWarpNT + t;
+        const factor *w = static_cast<const factor *>(tab) + 2 * q * NT + t;
         a = w[0];
-        b = w[kWarpNT];
+        b = w[NT];
     }
-    __device__ static __forceinline__ void stage1(const void *tab, int q, int n2, factor &a, factor &b) {
-        const factor *w = static_cast<const factor *>(tab) + tw_offset<kWarpM>(1) + 2 * q * kR + n2;
+    template <int S>
+    __device__ static __forceinline__ void stage(const void *tab, int q, int n, factor &a, factor &b) {
+        constexpr int st = S == 1 ? st1 : st1 / kR;
+        const factor *w = static_cast<const factor *>(tab) + tw_offset<M>(S) + 2 * q * st + n;
         a = w[0];
-        if (2 * q + 2 < kR) b = w[kR];
+        if (2 * q + 2 < kR) b = w[st];
     }
     __device__ static __forceinline__ void mid(const void *tab, int i, int row, factor &a, factor &b) {
         const factor *w = static_cast<const factor *>(tab) + row * 17 + 2 * i;
         a = w[0];
         b = w[1];
     }
-    __device__ static __forceinline__ void put_mid(void *mid_tab, const void *tab, int row, int f, int k1, int n2) {
-        const factor *w = static_cast<const factor *>(tab) + tw_offset<kWarpM>(1) + n2;
-        static_cast<factor *>(mid_tab)[row * 17 + f] = k1 ? w[(k1 - 1) * kR] : factor{1.0, 0.0};
+    __device__ static __forceinline__ void put_mid(void *mid_tab, const void *tab, int row, int f, int k1, int n) {
+        const factor *w = static_cast<const factor *>(tab) + tw_offset<M>(1) + n;
+        static_cast<factor *>(mid_tab)[row * 17 + f] = k1 ? w[(k1 - 1) * st1] : factor{1.0, 0.0};
     }
 };
 
-template <class Ops>
+__device__ __forceinline__ cpair point_add(const cpair &a, const cpair &b) { return padd(a, b); }
+__device__ __forceinline__ cpair point_sub(const cpair &a, const cpair &b) { return psub(a, b); }
+__device__ __forceinline__ cplx<double> point_add(const cplx<double> &a, const cplx<double> &b) { return cadd(a, b); }
+__device__ __forceinline__ cplx<double> point_sub(const cplx<double> &a, const cplx<double> &b) { return csub(a, b); }
+
+// BIG (N = 2048): the plan 8 x 8 x 8 x 2 over two warps, half = 0 or 1.  Stage 0's butterfly is t = 16 n1 + 2 n2 + n3; a
+// warp starts with n3 = half, so that up to stage 2 both do what one does at N = 1024 (t >> 1 in the place of t, and
+// the factors of their n3: stage 2's are 1 for n3 = 0).  Then WarpExch::swap trades n3 for h, the high bit of k0:
+// stage 3's radix-2 butterfly has its two points in one warp.  Slot (k3, k2) of lane l in warp `half` is position
+// p = 2 (t' + 128 c) + k3 with t' = 64 (l >> 3 & 1) + 8 (l & 7) + k2 and c = 2 half + (l >> 4).
+template <class Ops, bool BIG>
 struct WarpFft {
     using point = typename Ops::point;
     using factor = typename Ops::factor;
@@ -246,8 +292,11 @@ struct WarpFft {
         }
     }
 
-    // In: z[h][r] = a_j - i a_{j+M}, j = lane + 32 h + 64 r.  Out: slot r of virtual thread lane + 32 h.
-    __device__ static __forceinline__ void forward(point (&z)[2][kR], const typename Ops::Exch &x, const void *tab, int lane) {
+    // In: z[h][r] = a_j - i a_{j+M}, j = lane + 32 h + 64 r (BIG: 2 (lane + 32 h) + half + 128 r).  Out: slot r of
+    // virtual thread lane + 32 h (BIG: slot (h, r) as above).
+    __device__ static __forceinline__ void forward(point (&z)[2][kR], const typename Ops::Exch &x, const void *tab, int lane,
+                                                   int half) {
+        const int t0 = lane + (BIG ? 64 * half : 0), n = BIG ? 2 * (lane >> 2) + half : lane >> 2;
         uint32_t v[64], w[64];
 #pragma unroll
         for (int h = 0; h < 2; h++) {
@@ -256,7 +305,7 @@ struct WarpFft {
 #pragma unroll
             for (int q = 0; q < kR / 2; q++) {
                 factor a, b;
-                Ops::stage0(tab, q, lane + 32 * h, a, b);
+                Ops::stage0(tab, q, t0 + 32 * h, a, b);
                 Ops::template mul<false>(z[h][2 * q], a);
                 Ops::template mul<false>(z[h][2 * q + 1], b);
             }
@@ -274,7 +323,7 @@ struct WarpFft {
 #pragma unroll
         for (int q = 0; q < kR / 2; q++) {
             factor a, b;
-            Ops::stage1(tab, q, lane >> 2, a, b);
+            Ops::template stage<1>(tab, q, n, a, b);
 #pragma unroll
             for (int kl = 0; kl < 2; kl++) {
                 Ops::template mul<false>(y[kl][2 * q + 1], a);
@@ -306,12 +355,61 @@ struct WarpFft {
             }
             Ops::combine(z[h], e, o);
         }
+        if constexpr (BIG) {
+            stage2_factors<false>(z, tab, half);
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+#pragma unroll
+                for (int k = 0; k < kR; k++) put(v, 32 * h + 4 * k, 32 * h + 4 * k + 2, z[h][k]);
+            x.swap(v, half);
+            butterflies(z, v);
+        }
+    }
+    // stage 2's factors, 1 in the warp with n3 = 0
+    template <bool INV>
+    __device__ static __forceinline__ void stage2_factors(point (&z)[2][kR], const void *tab, int half) {
+        if (half == 0) return;
+#pragma unroll
+        for (int q = 0; q < kR / 2; q++) {
+            factor a, b;
+            Ops::template stage<2>(tab, q, 1, a, b);
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                Ops::template mul<INV>(z[h][2 * q + 1], a);
+                if (2 * q + 2 < kR) Ops::template mul<INV>(z[h][2 * q + 2], b);
+            }
+        }
+    }
+    // radix 2 over the two groups of v
+    __device__ static __forceinline__ void butterflies(point (&z)[2][kR], const uint32_t *v) {
+#pragma unroll
+        for (int k = 0; k < kR; k++) {
+            point a, b;
+            get(a, v, 4 * k, 4 * k + 2);
+            get(b, v, 32 + 4 * k, 32 + 4 * k + 2);
+            z[0][k] = point_add(a, b);
+            z[1][k] = point_sub(a, b);
+        }
     }
 
     // Slot r of virtual thread lane + 32 h in, z[h][r] = M (c_j - i c_{j+M}) out (the adjoint stages).
     __device__ static __forceinline__ void inverse(point (&z)[2][kR], const typename Ops::Exch &x, const void *tab,
-                                                   const void *mid_tab, int lane) {
+                                                   const void *mid_tab, int lane, int half) {
+        const int t0 = lane + (BIG ? 64 * half : 0);
         uint32_t v[64], w[64];
+        if constexpr (BIG) {
+#pragma unroll
+            for (int k = 0; k < kR; k++) {
+                put(v, 4 * k, 4 * k + 2, point_add(z[0][k], z[1][k]));
+                put(v, 32 + 4 * k, 32 + 4 * k + 2, point_sub(z[0][k], z[1][k]));
+            }
+            x.swap(v, half);
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+#pragma unroll
+                for (int k = 0; k < kR; k++) get(z[h][k], v, 32 * h + 4 * k, 32 * h + 4 * k + 2);
+            stage2_factors<true>(z, tab, half);
+        }
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             Ops::template dft8<true>(z[h]);
@@ -320,7 +418,7 @@ struct WarpFft {
                 put(v, p3_out(h, n & 1, n >> 1, 0, 0), p3_out(h, n & 1, n >> 1, 1, 0), z[h][n]);
         }
         x.backward(v);
-        const int row = 2 * (lane >> 4) + (lane & 1);  // n2 & 1, k1 >> 2
+        const int row = (BIG ? 4 * half : 0) + 2 * (lane >> 4) + (lane & 1);  // (n3,) n2 & 1, k1 >> 2
 #pragma unroll
         for (int i = 0; i < 4; i++)
 #pragma unroll
@@ -352,7 +450,7 @@ struct WarpFft {
 #pragma unroll
             for (int q = 0; q < kR / 2; q++) {
                 factor a, b;
-                Ops::stage0(tab, q, lane + 32 * h, a, b);
+                Ops::stage0(tab, q, t0 + 32 * h, a, b);
 #pragma unroll
                 for (int s = 0; s < 2; s++) {
                     get(z[h][2 * q + s], v, p1_in(h, 2 * q + s, 0, 0), p1_in(h, 2 * q + s, 1, 0));
@@ -373,24 +471,35 @@ struct WarpFft {
 // output's slots of a digit pair (split), or one digit's row (FP64); the ring holds whole steps.
 // DUO: a quadrant's two warps share one bootstrap and its 512 columns: spectra or (FP64) two outputs'
 // accumulators per warp, rotated words, an exchange region per warp.
-template <class Ops, int L, int D, bool DUO = false>
+// big: as solo, with every column count per warp, and the ring holds half a step.
+template <bool SPLIT, int L, int D, WarpMode MODE>
 struct WarpLayout {
+    static constexpr bool duo = MODE == WarpMode::duo, big = MODE == WarpMode::big;
+    static constexpr int N = big ? 2048 : 1024, M = N / 2, NT = M / kR;
+    using Ops = std::conditional_t<SPLIT, PairOps<M>, DoubleOps<M>>;
     static constexpr int KP1 = 2, KPL = KP1 * L;
-    static constexpr uint32_t half = (uint32_t)kWarpM * 16;  // one output's slots of one key row
-    static constexpr uint32_t unit = 2 * half;
-    static constexpr int per_step = KPL, turns = D / per_step;
-    static constexpr size_t bars = 0;  // full[D], empty[D], abort flag, TMEM address
+    static constexpr int teams = MODE == WarpMode::solo ? kWarpTeams : kWarpTeams / 2;  // most bootstraps per CTA
+    static constexpr uint32_t half = (uint32_t)M * 16;  // one output's slots of one key row
+    static constexpr uint32_t unit = 2 * half;          // KPL units per step
+    static constexpr size_t bars = 0;                   // full[D], empty[D], abort flag, TMEM address
     static constexpr size_t ring = (2 * D * 8 + 8 + 127) / 128 * 128;
     static constexpr size_t tables = ring + (size_t)D * unit;
     static constexpr size_t mid = tables + Ops::table_bytes;
-    static constexpr size_t accs = (mid + Ops::mid_bytes + 127) / 128 * 128;
-    static constexpr size_t acc_bytes = 4 * (size_t)KP1 * kWarpN;
+    static constexpr int mid_rows = big ? 8 : 4;
+    static constexpr size_t accs = (mid + mid_rows * Ops::row_bytes + 127) / 128 * 128;
+    static constexpr size_t acc_bytes = 4 * (size_t)KP1 * N;
     static constexpr size_t bytes(int G) { return accs + (size_t)G * acc_bytes; }
-    static constexpr bool split = std::is_same_v<Ops, PairOps>;
-    static constexpr uint32_t col_xr = !DUO ? 128 : split ? 192 : 256, col_exch = !DUO ? 192 : split ? 256 : 320;
-    static_assert(D % per_step == 0, "ring slots fixed within a step");
+    static constexpr uint32_t col_xr = !duo ? 128 : SPLIT ? 192 : 256, col_exch = !duo ? 192 : SPLIT ? 256 : 320;
+    // ring slot and mbarrier phase of unit i of a step: fixed within a step, or within half of one
+    static_assert(D % KPL == 0 || (D == L && KPL == 2 * D), "whole steps, or half a step");
+    __device__ static __forceinline__ int slot(int step, int i) {
+        return D % KPL == 0 ? (step % (D / KPL)) * KPL + i : i % D;
+    }
+    __device__ static __forceinline__ uint32_t phase(int step, int i) {
+        return D % KPL == 0 ? (uint32_t)(step / (D / KPL)) & 1u : (uint32_t)(i / D);  // two turns a step
+    }
     static_assert(KPL * 32 <= 192 && KPL % 2 == 0, "spectra columns");
-    static_assert(bytes(kWarpTeams) <= 227 * 1024, "shared memory of the variant");
+    static_assert(bytes(teams) <= 227 * 1024, "shared memory of the variant");
 };
 
 // the digits' top bits of a rotated word are kept in its low 23 bits
@@ -411,12 +520,17 @@ __device__ __forceinline__ float2 digit_pair(uint32_t a, uint32_t b) {
 // read all spectra from TMEM.  FP64: each transforms its polynomial's digits and multiplies them with the key of
 // both outputs; the two partial sums of an output meet at the end (FP64 sums round to the exact integers in
 // any order).
-template <bool SPLIT, int L, int D, bool DUO>
+//
+// big: warps w and w + 4 hold the two halves of every transform (WarpFft), and of the slots, key rows and accumulator
+// words; the accumulator keeps even and odd coefficients apart, so that a warp's are consecutive.
+template <bool SPLIT, int L, int D, WarpMode MODE>
 __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_kernel(const BrArgs args) {
-    using Ops = std::conditional_t<SPLIT, PairOps, DoubleOps>;
-    using Lay = WarpLayout<Ops, L, D, DUO>;
-    constexpr int N = kWarpN, M = kWarpM, NT = kWarpNT, KP1 = 2, KPL = KP1 * L;
-    using F = WarpFft<Ops>;
+    using Lay = WarpLayout<SPLIT, L, D, MODE>;
+    using Ops = typename Lay::Ops;
+    constexpr bool DUO = Lay::duo, BIG = Lay::big;
+    constexpr int N = Lay::N, NT = Lay::NT, KP1 = 2, KPL = KP1 * L;
+    constexpr bool SHIFTED = SPLIT && !BIG;  // digits from words shifted into a float's mantissa
+    using F = WarpFft<Ops, BIG>;
     extern __shared__ __align__(128) unsigned char smem[];
 
     // the same in every lane, in a way the compiler can see (uniform registers for the TMEM addresses)
@@ -433,7 +547,7 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
     if (threadIdx.x == 0) {
         for (int s = 0; s < D; s++) {
             mbar_init(full_bar(s), 1);
-            mbar_init(empty_bar(s), (uint32_t)active);
+            mbar_init(empty_bar(s), (uint32_t)(BIG ? 2 * active : active));
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -443,11 +557,16 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
     {
         const int4 *g_tab = reinterpret_cast<const int4 *>(args.tables);
         int4 *s_tab4 = reinterpret_cast<int4 *>(smem + Lay::tables);
-        for (int i = threadIdx.x; i < (int)(Ops::table_bytes / 16); i += blockDim.x) s_tab4[i] = g_tab[i];
-        // mid-table row (n2 & 1, k1 >> 2), entry 4 (n2 >> 1) + (k1 & 3)
-        if (threadIdx.x < 64) {
-            const int row = threadIdx.x >> 4, f = threadIdx.x & 15;
-            Ops::put_mid(smem + Lay::mid, args.tables, row, f, 4 * (row & 1) + (f & 3), 2 * (f >> 2) + (row >> 1));
+        constexpr int stage0 = (SPLIT ? kR / 2 : kR) * NT;
+        for (int i = threadIdx.x; i < (int)(Ops::table_bytes / 16); i += blockDim.x) {
+            int at = i;  // big: stage 0's factors of even t, then of odd t
+            if (BIG && i < stage0) at = (i & ~(NT - 1)) + (i & 1) * (NT / 2) + ((i & (NT - 1)) >> 1);
+            s_tab4[at] = g_tab[i];
+        }
+        // mid-table row (n3, n2 & 1, k1 >> 2), entry 4 (n2 >> 1) + (k1 & 3)
+        if (threadIdx.x < 16 * Lay::mid_rows) {
+            const int row = threadIdx.x >> 4, f = threadIdx.x & 15, n2 = 2 * (f >> 2) + (row >> 1 & 1);
+            Ops::put_mid(smem + Lay::mid, args.tables, row, f, 4 * (row & 1) + (f & 3), BIG ? 2 * n2 + (row >> 2) : n2);
         }
     }
     tmem_fence_before_sync();
@@ -458,8 +577,8 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
     if (warp >= kWarpTeams) {  // ---- producer ----
         asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
         if (threadIdx.x == kWarpTeams * 32) {
-            constexpr int per_step = Lay::per_step;
-            const int total = args.nsteps * per_step;
+            const uint8_t *bsk = SPLIT || BIG ? args.bsk2 : args.bsk;
+            const int total = args.nsteps * KPL;
             int sent = 0;
             if (!args.stall_producer) {
                 for (int c = 0; c < total; c++) {
@@ -469,13 +588,13 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
                     const uint32_t dst = ring + (uint32_t)s * Lay::unit;
                     mbar_arrive_expect_tx(full_bar(s), Lay::unit);
                     if constexpr (SPLIT) {
-                        const int step = c / per_step, rem = c - step * per_step;
+                        const int step = c / KPL, rem = c - step * KPL;
                         const int v = rem / L, d = 2 * (rem - v * L);
-                        const uint8_t *src = args.bsk2 + ((size_t)(step * KPL + d) * KP1 + v) * Lay::half;
+                        const uint8_t *src = bsk + ((size_t)(step * KPL + d) * KP1 + v) * Lay::half;
                         bulk_copy_g2s(dst, src, Lay::half, full_bar(s));
                         bulk_copy_g2s(dst + Lay::half, src + (size_t)KP1 * Lay::half, Lay::half, full_bar(s));
                     } else {
-                        bulk_copy_g2s(dst, args.bsk + (size_t)c * Lay::unit, Lay::unit, full_bar(s));
+                        bulk_copy_g2s(dst, bsk + (size_t)c * Lay::unit, Lay::unit, full_bar(s));
                     }
                     sent = c + 1;
                 }
@@ -487,7 +606,7 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
         return;
     }
     asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
-    const int team = DUO ? warp & 3 : warp, role = DUO ? warp >> 2 : 0;
+    const int team = DUO || BIG ? warp & 3 : warp, role = DUO ? warp >> 2 : 0, half = BIG ? warp >> 2 : 0;
     if (team >= active) return;  // no TMEM use, not counted in any barrier below
 
     // ---- consumer warps ----
@@ -495,21 +614,19 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
     uint32_t *s_acc = reinterpret_cast<uint32_t *>(smem + Lay::accs + (size_t)team * Lay::acc_bytes);
     const void *s_tab = smem + Lay::tables, *s_mid = smem + Lay::mid;
     const uint32_t tmem = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (DUO ? 0u : (uint32_t)((warp >> 2) * 256));
-    const typename Ops::Exch exch{tmem + Lay::col_exch + (uint32_t)(64 * role)};
+    const typename Ops::Exch exch{tmem + Lay::col_exch + (uint32_t)(64 * role), 2 + team};
     // DUO: both warps of the bootstrap, their TMEM accesses before it ordered before those after it
     auto duo_sync = [&] {
-        if constexpr (DUO) {
-            tmem_fence_before_sync();
-            team_sync(2 + team, 64);
-            tmem_fence_after_sync();
-        }
+        if constexpr (DUO) exch.team();
     };
-    const int first = lane + 32 * role, stride = DUO ? 64 : 32;
+    const int first = lane + 32 * (role + half), stride = DUO || BIG ? 64 : 32;
+    // place of coefficient j of a polynomial (i over both)
+    auto place = [](int i) { return BIG ? (i & ~(N - 1)) + ((i & 1) << 10) + ((i & (N - 1)) >> 1) : i; };
 
     const int32_t *my_bara = args.bara + (size_t)boot * args.bara_stride;
     if (args.acc_in) {
         const uint32_t *src = reinterpret_cast<const uint32_t *>(args.acc_in) + (size_t)boot * KP1 * N;
-        for (int i = first; i < KP1 * N; i += stride) s_acc[i] = src[i];
+        for (int i = first; i < KP1 * N; i += stride) s_acc[place(i)] = src[i];
     } else {
         // acc = (0, X^{2N-barb} * [mu,...,mu])  (lwe-bootstrapping-functions-fft.cpp:142-145)
         const int e = 2 * N - my_bara[args.nsteps];
@@ -521,11 +638,11 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
                 src += N;
                 neg ^= 1u;
             }
-            s_acc[N + j] = neg ? 0u - (uint32_t)args.mu : (uint32_t)args.mu;
+            s_acc[N + place(j)] = neg ? 0u - (uint32_t)args.mu : (uint32_t)args.mu;
         }
     }
     __syncwarp();
-    duo_sync();
+    if constexpr (DUO || BIG) team_sync(2 + team, 64);
 
     // gadget constants (tgsw.cpp:7-29)
     const int Bgbit = args.Bgbit;
@@ -548,21 +665,23 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
         //    A loop of two halves: the whole step unrolled misses the instruction cache (one warp per
         //    scheduler ran 14.9k cycles a step with this loop, 16.0k without).
         {
-            const uint32_t rot = 4u * (uint32_t)(lane - ai);  // byte index of e
-            const uint32_t *polys = s_acc + role * N;         // DUO: the warp's own polynomial only
+            // byte index of e; big: of e's place among the even or odd coefficients, the same for all of the warp's j
+            const uint32_t rot = 4u * (uint32_t)(BIG ? (2 * lane + half - ai) >> 1 : lane - ai);
+            const uint32_t *polys = s_acc + role * N;  // DUO: the warp's own polynomial only
+            const uint32_t *from = BIG ? polys + (((half - ai) & 1) << 10) : polys;
 #pragma unroll 1
             for (int i0 = 0; i0 < 32; i0 += 16) {
                 uint32_t x0[16], x1[16];
-                const uint32_t *own = polys + lane + 32 * i0;
+                const uint32_t *own = polys + 1024 * half + lane + 32 * i0;
 #pragma unroll
                 for (int i = 0; i < 16; i++) {
                     const uint32_t e = rot + 128u * (uint32_t)(i0 + i);
                     const uint32_t neg = (uint32_t)((int32_t)(e << 19) >> 31);
                     const uint32_t on = offset - neg;
                     const uint32_t *src =
-                        reinterpret_cast<const uint32_t *>(reinterpret_cast<const char *>(polys) + (e & 4095u));
-                    x0[i] = ((src[0] ^ neg) + (on - own[32 * i])) >> (SPLIT ? kDigitShift : 0);
-                    if constexpr (!DUO) x1[i] = ((src[N] ^ neg) + (on - own[32 * i + N])) >> (SPLIT ? kDigitShift : 0);
+                        reinterpret_cast<const uint32_t *>(reinterpret_cast<const char *>(from) + (e & 4095u));
+                    x0[i] = ((src[0] ^ neg) + (on - own[32 * i])) >> (SHIFTED ? kDigitShift : 0);
+                    if constexpr (!DUO) x1[i] = ((src[N] ^ neg) + (on - own[32 * i + N])) >> (SHIFTED ? kDigitShift : 0);
                 }
                 tmem_st16(tmem + Lay::col_xr + (uint32_t)(32 * role + i0), x0);
                 if constexpr (!DUO) tmem_st16(tmem + Lay::col_xr + 32u + (uint32_t)i0, x1);
@@ -579,9 +698,11 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
                 const int u0 = d0 / L, u1 = (d0 + 1) / L;
                 // digit q of a word: its bits under the exponent of 2^23 are the float 2^23 + d 2^sh; times
                 // 2^-sh, minus (2^23 2^-sh + Bg/2): exact, one operation for the pair
-                const int sh0 = 32 - (d0 - u0 * L + 1) * Bgbit - kDigitShift, sh1 = 32 - (d0 + 1 - u1 * L + 1) * Bgbit - kDigitShift;
-                const uint32_t m0 = maskBg << sh0, m1 = maskBg << sh1;
-                const float2 sc = make_float2(__int_as_float((127 - sh0) << 23), __int_as_float((127 - sh1) << 23));
+                const int sh0 = 32 - (d0 - u0 * L + 1) * Bgbit - (SHIFTED ? kDigitShift : 0);
+                const int sh1 = 32 - (d0 + 1 - u1 * L + 1) * Bgbit - (SHIFTED ? kDigitShift : 0);
+                const uint32_t m0 = SHIFTED ? maskBg << sh0 : maskBg, m1 = SHIFTED ? maskBg << sh1 : maskBg;
+                const float2 sc = SHIFTED ? make_float2(__int_as_float((127 - sh0) << 23), __int_as_float((127 - sh1) << 23))
+                                          : make_float2(1.0f, 1.0f);
                 const float half_bg = float(1 << (Bgbit - 1));
                 const float2 bias = make_float2(8388608.0f * sc.x + half_bg, 8388608.0f * sc.y + half_bg);
                 uint32_t xa[32], xb[32];
@@ -595,11 +716,13 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
 #pragma unroll
                     for (int r = 0; r < kR; r++) {  // j = lane + 32 (h + 2 r); j + M is word 16 on
                         const int i = h + 2 * r;
-                        const float2 lo = digit_pair(xa[i] & m0, xb[i] & m1);
-                        const float2 hi = digit_pair(xa[i + 16] & m0, xb[i + 16] & m1);
-                        z[h][r] = {fma2(lo, sc, neg2(bias)), fma2(neg2(hi), sc, bias)};
+                        const int s0 = SHIFTED ? 0 : sh0, s1 = SHIFTED ? 0 : sh1;
+                        const float2 lo = digit_pair((xa[i] >> s0) & m0, (xb[i] >> s1) & m1);
+                        const float2 hi = digit_pair((xa[i + 16] >> s0) & m0, (xb[i + 16] >> s1) & m1);
+                        if constexpr (SHIFTED) z[h][r] = {fma2(lo, sc, neg2(bias)), fma2(neg2(hi), sc, bias)};
+                        else z[h][r] = {sub2(lo, bias), sub2(bias, hi)};
                     }
-                F::forward(z, exch, s_tab, lane);
+                F::forward(z, exch, s_tab, lane, half);
                 // per butterfly h and slot r: re of both digits, im of both
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
@@ -625,9 +748,10 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
                 // keys of butterfly h and digit dd of the ring unit at `at`: {hi.re, lo.re, hi.im, lo.im} per slot.  Each
                 // quarter of a unit is loaded while the one before is multiplied.
                 auto load = [&](float4(&k)[kR], const unsigned char *at, int h, int dd) {
-                    const float4 *kp = reinterpret_cast<const float4 *>(at + dd * Lay::half) + lane + 32 * h;
+                    const float4 *kp = reinterpret_cast<const float4 *>(at + dd * Lay::half) + lane +
+                                       (BIG ? 512 * half + 256 * h : 32 * h);
 #pragma unroll
-                    for (int r = 0; r < kR; r++) k[r] = kp[r * NT];
+                    for (int r = 0; r < kR; r++) k[r] = kp[r * (BIG ? 32 : NT)];
                 };
                 auto mac = [&](cpair(&a)[kR], const uint32_t(&f)[32], int dd, const float4(&k)[kR]) {
 #pragma unroll
@@ -643,8 +767,8 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
                 auto ring_at = [&](int s) { return smem + Lay::ring + (size_t)s * Lay::unit; };
                 uint32_t f0[32], f1[32];
                 float4 ka[kR], kb[kR];
-                int slot = (step % Lay::turns) * Lay::per_step + v * (KPL / 2);
-                const uint32_t phase = (uint32_t)(step / Lay::turns) & 1u;
+                int slot = Lay::slot(step, v * L);
+                const uint32_t phase = Lay::phase(step, v * L);
                 tmem_ld32(tmem, f0);
                 tmem_ld32(tmem + 32u, f1);
                 wait_bounded(full_bar(slot), phase, abort_flag, args.timeout_ns, args.err);
@@ -679,15 +803,15 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
                         tmem_tie32(f1);
                     }
                 }
-                F::inverse(acc, exch, s_tab, s_mid, lane);
-                uint32_t *poly = s_acc + v * N + lane;
+                F::inverse(acc, exch, s_tab, s_mid, lane, half);
+                uint32_t *poly = s_acc + v * N + 1024 * half + lane;
 #pragma unroll
                 for (int h = 0; h < 2; h++)
 #pragma unroll
                     for (int r = 0; r < kR; r++) {  // (c_j - i c_{j+M}) of each limb, the high limb weighted 2^S
                         const int j = 32 * h + 64 * r;
                         poly[j] += ((uint32_t)__float2ll_rn(acc[h][r].re.x) << split_shift) + (uint32_t)__float2ll_rn(acc[h][r].re.y);
-                        poly[j + M] +=
+                        poly[j + 512] +=
                             ((uint32_t)__float2ll_rn(-acc[h][r].im.x) << split_shift) + (uint32_t)__float2ll_rn(-acc[h][r].im.y);
                     }
             }
@@ -720,11 +844,11 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
                         const double hi = __hiloint2double(0x43380000, (int)(x[h + 2 * r + 16] & mask));
                         z[h][r] = {fma(lo, scale, -bias), fma(-hi, scale, bias)};
                     }
-                F::forward(z, exch, s_tab, lane);
-                const int slot = (step % Lay::turns) * Lay::per_step + d;
-                wait_bounded(full_bar(slot), (uint32_t)(step / Lay::turns) & 1u, abort_flag, args.timeout_ns, args.err);
+                F::forward(z, exch, s_tab, lane, half);
+                const int slot = Lay::slot(step, d);
+                wait_bounded(full_bar(slot), Lay::phase(step, d), abort_flag, args.timeout_ns, args.err);
                 __syncwarp();
-                const double2 *kp = reinterpret_cast<const double2 *>(smem + Lay::ring + (size_t)slot * Lay::unit) + lane;
+                const double2 *kp = reinterpret_cast<const double2 *>(smem + Lay::ring + (size_t)slot * Lay::unit) + lane + 512 * half;
                 // quarters (output v, butterfly h), the next one's accumulators loading meanwhile
                 uint32_t a[2][32];
                 tmem_ld32(sums, a[0]);
@@ -736,7 +860,7 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
                     uint32_t w[32];
 #pragma unroll
                     for (int r = 0; r < kR; r++) {
-                        const double2 k = kp[((q >> 1) * kR + r) * NT + 32 * (q & 1)];
+                        const double2 k = BIG ? kp[1024 * (q >> 1) + 256 * (q & 1) + 32 * r] : kp[((q >> 1) * kR + r) * NT + 32 * (q & 1)];
                         cplx<double> p;
                         F::get(p, acc, 4 * r, 4 * r + 2);
                         cmac(p, z[q & 1][r], cplx<double>{k.x, k.y});
@@ -777,55 +901,74 @@ __global__ void __launch_bounds__((kWarpTeams + 4) * 32, 1) blind_rotate_warp_ke
                             z[h][r] = cadd(z[h][r], p);
                         }
                 }
-                F::inverse(z, exch, s_tab, s_mid, lane);
-                uint32_t *poly = s_acc + v * N + lane;
+                F::inverse(z, exch, s_tab, s_mid, lane, half);
+                uint32_t *poly = s_acc + v * N + 1024 * half + lane;
 #pragma unroll
                 for (int h = 0; h < 2; h++)
 #pragma unroll
                     for (int r = 0; r < kR; r++) {  // (c_j - i c_{j+M})
                         const int j = 32 * h + 64 * r;
                         poly[j] += round_f64_mod32(z[h][r].re);
-                        poly[j + M] += round_f64_mod32(-z[h][r].im);
+                        poly[j + 512] += round_f64_mod32(-z[h][r].im);
                     }
             }
         }
-        __syncwarp();
+        if constexpr (BIG) team_sync(2 + team, 64);  // the other warp rotates these words too
+        else __syncwarp();
     }
 
     uint32_t *dst = reinterpret_cast<uint32_t *>(args.acc_out) + (size_t)boot * KP1 * N;
-    for (int i = lane + role * N; i < (DUO ? (role + 1) * N : KP1 * N); i += 32) dst[i] = s_acc[i];
+    if constexpr (BIG) {
+        for (int i = first; i < KP1 * N; i += stride) dst[i] = s_acc[place(i)];
+    } else {
+        for (int i = lane + role * N; i < (DUO ? (role + 1) * N : KP1 * N); i += 32) dst[i] = s_acc[i];
+    }
 
     // every consumer's TMEM accesses are complete; warp 0 frees the columns
     tmem_fence_before_sync();
-    team_sync(1, active * (DUO ? 64 : 32));
+    team_sync(1, active * (DUO || BIG ? 64 : 32));
     tmem_fence_after_sync();
     __syncwarp();
     if (warp == 0) tmem_free(tmem_base, 512);
 }
 
-template <bool SPLIT, int L, int G, int D, bool DUO>
-cudaError_t launch_warp(const BrArgs &args, cudaStream_t s) {
-    using Lay = WarpLayout<std::conditional_t<SPLIT, PairOps, DoubleOps>, L, D, DUO>;
-    static_assert(G <= (DUO ? kWarpTeams / 2 : kWarpTeams), "one warp per bootstrap, or two");
-    if (SPLIT && !args.bsk2) return cudaErrorInvalidValue;
-    auto kern = blind_rotate_warp_kernel<SPLIT, L, D, DUO>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::bytes(kWarpTeams));
+template <bool SPLIT, int L, int G, int D, WarpMode MODE>
+static cudaError_t launch_warp_impl(const BrArgs &args, cudaStream_t s) {
+    using Lay = WarpLayout<SPLIT, L, D, MODE>;
+    static_assert(G <= Lay::teams, "one warp per bootstrap, or two");
+    if ((SPLIT || Lay::big) && !args.bsk2) return cudaErrorInvalidValue;
+    auto kern = blind_rotate_warp_kernel<SPLIT, L, D, MODE>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::bytes(Lay::teams));
     if (e != cudaSuccess) return e;
     BrArgs a = args;
     a.teams = G;
     kern<<<(a.boots + G - 1) / G, 32 * (kWarpTeams + 4), Lay::bytes(G), s>>>(a);
     return cudaGetLastError();
 }
+template <bool SPLIT, int L, int G, int D>
+cudaError_t launch_warp(const BrArgs &a, cudaStream_t s) {
+    return launch_warp_impl<SPLIT, L, G, D, WarpMode::solo>(a, s);
+}
+template <bool SPLIT, int L, int G, int D>
+cudaError_t launch_warp_duo(const BrArgs &a, cudaStream_t s) {
+    return launch_warp_impl<SPLIT, L, G, D, WarpMode::duo>(a, s);
+}
+template <bool SPLIT, int L, int G>
+cudaError_t launch_warp_big(const BrArgs &a, cudaStream_t s) {
+    return launch_warp_impl<SPLIT, L, G, L, WarpMode::big>(a, s);
+}
 
-template cudaError_t launch_warp<true, 3, 8, 6, false>(const BrArgs &, cudaStream_t);
-template cudaError_t launch_warp<true, 3, 4, 6, true>(const BrArgs &, cudaStream_t);
-template cudaError_t launch_warp<true, 3, 3, 6, true>(const BrArgs &, cudaStream_t);
-template cudaError_t launch_warp<false, 3, 8, 6, false>(const BrArgs &, cudaStream_t);
-template cudaError_t launch_warp<false, 3, 4, 6, true>(const BrArgs &, cudaStream_t);
-template cudaError_t launch_warp<false, 3, 3, 6, true>(const BrArgs &, cudaStream_t);
-template cudaError_t launch_warp<true, 2, 8, 8, false>(const BrArgs &, cudaStream_t);
-template cudaError_t launch_warp<true, 2, 4, 8, true>(const BrArgs &, cudaStream_t);
-template cudaError_t launch_warp<false, 2, 8, 8, false>(const BrArgs &, cudaStream_t);
-template cudaError_t launch_warp<false, 2, 4, 8, true>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp<true, 3, 8, 6>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp<false, 3, 8, 6>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp<true, 2, 8, 8>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp<false, 2, 8, 8>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp_duo<true, 3, 4, 6>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp_duo<true, 3, 3, 6>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp_duo<false, 3, 4, 6>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp_duo<false, 3, 3, 6>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp_duo<true, 2, 4, 8>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp_duo<false, 2, 4, 8>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp_big<true, 3, 4>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_warp_big<false, 3, 4>(const BrArgs &, cudaStream_t);
 
 }  // namespace tfheb

@@ -12,7 +12,7 @@ struct BrArgs {
     const int32_t *bara;
     int bara_stride;
     const uint8_t *bsk;
-    const uint8_t *bsk2;  // split: the key with its limbs side by side (DeviceBsk)
+    const uint8_t *bsk2;  // the key's second layout (DeviceBsk), or null
     const void *tables;
     const void *tables2;  // split-FP32 twiddles as broadcast pairs (the paired kernel)
     const int32_t *acc_in;

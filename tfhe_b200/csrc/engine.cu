@@ -500,7 +500,7 @@ tfheb_status tfheb_cloud_key_to_device(tfheb_cloud_key *c, int32_t device, int32
         }
         d.bsk_bytes = polys * (size_t)(p.N / 2) * 16;
         TFHEB_CUDA(cudaMalloc(&d.bsk, d.bsk_bytes));
-        if (prec == TFHEB_SPLIT_FP32 && p.N == 1024) TFHEB_CUDA(cudaMalloc(&d.bsk2, d.bsk_bytes));
+        if (p.N == 2048 || (p.N == 1024 && prec == TFHEB_SPLIT_FP32)) TFHEB_CUDA(cudaMalloc(&d.bsk2, d.bsk_bytes));
         d.split_shift = prec == TFHEB_SPLIT_FP32 ? split_shift : 0;
         TFHEB_CUDA(launch_bsk_to_fft(p, prec, static_cast<const int32_t *>(d_coef.p),
                                      static_cast<const double *>(d_tab64.p), d.bsk, d.bsk2, split_shift, ck.stream));

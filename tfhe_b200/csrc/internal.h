@@ -35,7 +35,8 @@ struct GateDesc {
 // Device-side FFT-domain bootstrapping key and tables for one precision.
 struct DeviceBsk {
     void *bsk = nullptr;      // [n][kpl][k+1][R][NT] x 16 bytes (double2, or float4 = hi.re,hi.im,lo.re,lo.im)
-    void *bsk2 = nullptr;     // split, N = 1024: the same key, per slot {hi.re, lo.re, hi.im, lo.im}
+    // the same key as the newer kernels read it (key_transform.cu): split at N = 1024, both forms at N = 2048
+    void *bsk2 = nullptr;
     void *tables = nullptr;   // stage twiddles (stage 0 carries the twist), layout of the precision
     void *tables2 = nullptr;  // split only: the FP32 factors as broadcast pairs (build_tables_f32_paired)
     size_t bsk_bytes = 0;
@@ -146,8 +147,8 @@ void build_tables_f32(int N, std::vector<float> &tables);    // float4 pairs of 
 void build_tables_f32_paired(int N, std::vector<float> &tables);
 void fill_slot_freq(int N, std::vector<int32_t> &slot_freq); // [R][NT] -> frequency index
 // key_transform.cu: coefficient-domain bootstrapping key [n][kpl][k+1][N] on the device -> the
-// FFT-domain layout of `precision` (d_out: n*kpl*(k+1)*N/2*16 bytes), on stream s; d_out2 (split, may be
-// null): the same in the limbs-side-by-side layout.
+// FFT-domain layout of `precision` (d_out: n*kpl*(k+1)*N/2*16 bytes), on stream s; d_out2 (may be
+// null): the same in the second layout.
 cudaError_t launch_bsk_to_fft(const tfheb_params &p, int precision, const int32_t *d_coef, const double *d_tables64,
                               void *d_out, void *d_out2, int split_shift, cudaStream_t s);
 
@@ -209,9 +210,14 @@ template <int N, int L, int G, int D, int XB>
 cudaError_t launch_paired_il3(const BrArgs &a, cudaStream_t s);
 template <int N, int L, int G, int D, int XB>
 cudaError_t launch_paired_il7(const BrArgs &a, cudaStream_t s);
-// blind_rotate_warp.cu: one warp per bootstrap, up to eight per CTA, exchanges in tensor memory (N = 1024)
-template <bool SPLIT, int L, int G, int D, bool DUO>
+// blind_rotate_warp.cu: exchanges in tensor memory; N = 1024 with one warp per bootstrap, up to eight per CTA, or
+// two (duo), up to four; N = 2048 with two, up to four (big)
+template <bool SPLIT, int L, int G, int D>
 cudaError_t launch_warp(const BrArgs &a, cudaStream_t s);
+template <bool SPLIT, int L, int G, int D>
+cudaError_t launch_warp_duo(const BrArgs &a, cudaStream_t s);
+template <bool SPLIT, int L, int G>
+cudaError_t launch_warp_big(const BrArgs &a, cudaStream_t s);
 // blind_rotate_latency.cu: one bootstrap per CTA (C = 1) or per cluster of two (C = 2), N = 1024
 template <typename T, int L, int C>
 cudaError_t launch_latency(const BrArgs &a, cudaStream_t s);

@@ -8,8 +8,10 @@
 //   FP64:       double2 (re, im) at [R][NT]
 //   split FP32: the polynomial is first cut into limbs c = hi * 2^S + lo, lo in [-2^(S-1), 2^(S-1));
 //               each limb is transformed in FP64 and rounded to float; per register pair (2m, 2m+1)
-//               and limb, float4 {re(2m), re(2m+1), im(2m), im(2m+1)} at [4][2][NT]; where a second buffer
-//               is given, the same values there as float4 {hi.re, lo.re, hi.im, lo.im} at [R][NT]
+//               and limb, float4 {re(2m), re(2m+1), im(2m), im(2m+1)} at [4][2][NT]
+// A second buffer, where given, takes the same values as double2 (re, im) or float4 {hi.re, lo.re, hi.im, lo.im},
+// at [R][NT] for N <= 1024 and for N = 2048 in the order of blind_rotate_warp.cu's lanes: slot r = 2c + k3 of thread
+// t = 64 x + 8 k1 + k2 at [c >> 1][k3][k2][16 (c & 1) + 8 x + k1].
 // One team of N/16 threads per polynomial, 4 teams per CTA, twiddles in shared memory.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -24,6 +26,15 @@ namespace {
 constexpr int kTeams = 4;
 
 template <int N>
+__device__ __forceinline__ int second_index(int r, int t) {
+    if constexpr (N == 2048) {
+        const int c = r >> 1, lane = 16 * (c & 1) + 8 * (t >> 6) + (t >> 3 & 7);
+        return (((c >> 1) * 2 + (r & 1)) * 8 + (t & 7)) * 32 + lane;
+    }
+    return r * (N / 2 / kR) + t;
+}
+
+template <int N>
 struct KtLayout {
     static constexpr int M = N / 2, NT = M / kR;
     static constexpr int TW = tw_offset<M>(FftPlan<M>::NS);
@@ -35,7 +46,8 @@ struct KtLayout {
 template <int N, bool SPLIT>
 __global__ void __launch_bounds__(kTeams *(N / 16)) bsk_to_fft_kernel(const int32_t *__restrict__ coef, int polys,
                                                                      const double *__restrict__ tables,
-                                                                     uint8_t *__restrict__ out, uint8_t *__restrict__ out2, int split_shift) {
+                                                                     uint8_t *__restrict__ out,
+                                                                     uint8_t *__restrict__ out2, int split_shift) {
     using Lay = KtLayout<N>;
     constexpr int M = Lay::M, NT = Lay::NT;
     using F = TeamFft<double, M, kR>;
@@ -66,6 +78,11 @@ __global__ void __launch_bounds__(kTeams *(N / 16)) bsk_to_fft_kernel(const int3
         double2 *o = reinterpret_cast<double2 *>(out + (size_t)poly * M * 16);
 #pragma unroll
         for (int r = 0; r < kR; r++) o[r * NT + t] = make_double2(x[r].re * scale, x[r].im * scale);
+        if (out2) {
+            double2 *o2 = reinterpret_cast<double2 *>(out2 + (size_t)poly * M * 16);
+#pragma unroll
+            for (int r = 0; r < kR; r++) o2[second_index<N>(r, t)] = make_double2(x[r].re * scale, x[r].im * scale);
+        }
     } else {
         const int64_t half = (int64_t)1 << (split_shift - 1), mask = ((int64_t)1 << split_shift) - 1;
         cplx<double> xh[kR], xl[kR];
@@ -91,8 +108,8 @@ __global__ void __launch_bounds__(kTeams *(N / 16)) bsk_to_fft_kernel(const int3
             float4 *o2 = reinterpret_cast<float4 *>(out2 + (size_t)poly * M * 16);
 #pragma unroll
             for (int r = 0; r < kR; r++)
-                o2[r * NT + t] = make_float4((float)(xh[r].re * scale), (float)(xl[r].re * scale),
-                                             (float)(xh[r].im * scale), (float)(xl[r].im * scale));
+                o2[second_index<N>(r, t)] = make_float4((float)(xh[r].re * scale), (float)(xl[r].re * scale),
+                                                        (float)(xh[r].im * scale), (float)(xl[r].im * scale));
         }
     }
 }
