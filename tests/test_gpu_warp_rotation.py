@@ -1,7 +1,7 @@
 """The one-warp-per-bootstrap blind rotation (eight bootstraps per CTA, FFT exchanges in tensor memory): bit for
 bit the rotation of the team kernels, which the oracle pins, with full, partly filled and single CTAs, over
 the fewest steps, on both gadget lengths; its form with two warps per bootstrap and the kernels for a few
-bootstraps (one per SM, one per cluster of two) against it; its form for the larger ring; the cut of a batch into waves; digits too wide for the split form; stalled key streams."""
+bootstraps (one per SM, one per cluster of two) against it; their forms for the larger ring; the cut of a batch into waves; digits too wide for the split form; stalled key streams."""
 import numpy as np
 import pytest
 
@@ -102,6 +102,20 @@ def test_few_bootstraps_equal_a_packed_wave(keys, l, Bgbit, precision, nsteps, c
     ck.set_br_variant(precision, 0)
 
 
+# N = 2048: one bootstrap on two SMs (at most 74 of 148); a step takes six rows through a ring of five
+@pytest.mark.parametrize("count", [1, 2, 73, 74, 75])
+@pytest.mark.parametrize("nsteps", [1, 2, 5, 9])
+def test_large_ring_few_bootstraps_equal_a_packed_wave(large_keys, nsteps, count):
+    sk, ck = large_keys
+    rng = np.random.default_rng(7 * count + nsteps)
+    acc = rng.integers(-2**31, 2**31, (592, 2, 2048)).astype(np.int32)
+    bara = rng.integers(0, 4096, (592, nsteps)).astype(np.int32)
+    bara.flat[:5] = [0, 1, 2047, 2048, 4095]
+    four = int(np.flatnonzero(ck.br_variants(tb.SPLIT_FP32)[0] == 4)[0])
+    want = rotate(ck, tb.SPLIT_FP32, four, bara, acc, nsteps)
+    assert (rotate(ck, tb.SPLIT_FP32, four, bara[:count], acc[:count], nsteps) == want[:count]).all()
+
+
 # around the waves' ends: all of the last wave's choices, and a last CTA with one of eight warps at work
 @pytest.mark.parametrize("count", [1033, 1177, 1184, 1185, 1500, 1777])
 @pytest.mark.parametrize("precision", [tb.FP64, tb.SPLIT_FP32])
@@ -136,3 +150,16 @@ def test_stalled_key_stream(keys, precision, count):
     ck.set_wait_timeout(1.0)
     assert (sk.decrypt(ck.gate(tb.api.NAND, a, a, precision=precision))[0] == 1 - x).all()
     ck.set_br_variant(precision, 0)
+
+
+def test_stalled_key_stream_large_ring(large_keys):
+    sk, ck = large_keys
+    bara, acc = np.zeros((3, 2), np.int32), np.zeros((3, 2, 2048), np.int32)
+    ck.set_wait_timeout(0.05)
+    ck.test_stall_key_stream(True)
+    with pytest.raises(tb.api.TfhebError) as exc:
+        rotate(ck, tb.SPLIT_FP32, 0, bara, acc, 2)
+    assert exc.value.status == tb.api.TIMEOUT
+    ck.test_stall_key_stream(False)
+    ck.set_wait_timeout(1.0)
+    rotate(ck, tb.SPLIT_FP32, 0, bara, acc, 2)

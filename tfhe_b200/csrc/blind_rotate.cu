@@ -247,7 +247,9 @@ __global__ void __launch_bounds__(G *(N / 16) + (PW ? 32 : 0), 1) blind_rotate_k
 #pragma unroll
                 for (int m = 0; m < kR / 2; m++) {
                     const cpair zp = make_cpair(z[2 * m], z[2 * m + 1]);
-                    const float2 nzi = neg2(zp.im);
+                    // the same bits; one team alone runs faster with the product (6.30 against 6.40 ms per wave of 148
+                    // at N = 2048), five at N = 1024 with the sign flips (6.71 against 6.84 ms)
+                    const float2 nzi = G == 1 ? mul2(zp.im, make_float2(-1.f, -1.f)) : neg2(zp.im);
 #pragma unroll
                     for (int v = 0; v < KP1; v++) {
                         const float4 *kp = reinterpret_cast<const float4 *>(
@@ -547,8 +549,8 @@ static const BrVariant kBrVariants[] = {
     {1024, 3, TFHEB_SPLIT_FP32, 4, 6, false, 6.21, launch_warp_duo<true, 3, 4, 6>, 1, 23},
     {1024, 3, TFHEB_SPLIT_FP32, 3, 6, false, 6.14, launch_warp_duo<true, 3, 3, 6>, 1, 23},
     // few bootstraps (blind_rotate_latency.cu; D counts 48 KB stages): one per CTA, one per two CTAs
-    {1024, 3, TFHEB_SPLIT_FP32, 1, 2, false, 2.92, launch_latency<float, 3, 1>},
-    {1024, 3, TFHEB_SPLIT_FP32, 1, 2, false, 1.96, launch_latency<float, 3, 2>, 0, 32, 2},
+    {1024, 3, TFHEB_SPLIT_FP32, 1, 2, false, 2.92, launch_latency<float, 3, 1, 1024>},
+    {1024, 3, TFHEB_SPLIT_FP32, 1, 2, false, 1.96, launch_latency<float, 3, 2, 1024>, 0, 32, 2},
     {1024, 3, TFHEB_FP64, 4, 5, true, 9.85, launch_g<double, 1024, 3, false, 4, 5, false>},
     {1024, 3, TFHEB_FP64, 4, 4, true, 10.18, launch_g<double, 1024, 3, false, 4, 4, false>},
     {1024, 3, TFHEB_FP64, 4, 6, true, 11.18, launch_g<double, 1024, 3, false, 4, 6>},
@@ -558,8 +560,8 @@ static const BrVariant kBrVariants[] = {
     {1024, 3, TFHEB_FP64, 8, 6, true, 16.08, launch_warp<false, 3, 8, 6>},
     {1024, 3, TFHEB_FP64, 4, 6, false, 8.32, launch_warp_duo<false, 3, 4, 6>},
     {1024, 3, TFHEB_FP64, 3, 6, false, 8.34, launch_warp_duo<false, 3, 3, 6>},
-    {1024, 3, TFHEB_FP64, 1, 2, false, 3.67, launch_latency<double, 3, 1>},
-    {1024, 3, TFHEB_FP64, 1, 1, false, 2.47, launch_latency<double, 3, 2>, 0, 32, 2},
+    {1024, 3, TFHEB_FP64, 1, 2, false, 3.67, launch_latency<double, 3, 1, 1024>},
+    {1024, 3, TFHEB_FP64, 1, 1, false, 2.47, launch_latency<double, 3, 2, 1024>, 0, 32, 2},
     // the split default at N = 2048: the N = 1024 default's structure with three teams and a 6-deep
     // ring of 16 KB half rows (51.3 ms per 2048 bootstraps; 51.7 ms with output 0's inverse input in
     // registers, 51.9 ms forward interleave only, 53.1 ms no interleave, 54.1 ms rotated words in
@@ -572,7 +574,9 @@ static const BrVariant kBrVariants[] = {
     {2048, 3, TFHEB_SPLIT_FP32, 2, 4, true, 11.45, launch_g<float, 2048, 3, true, 2, 4>},
     {2048, 3, TFHEB_SPLIT_FP32, 3, 3, true, 16.81, launch_g<float, 2048, 3, true, 3, 3>},
     {2048, 3, TFHEB_SPLIT_FP32, 2, 3, true, 11.56, launch_g<float, 2048, 3, true, 2, 3>},
-    {2048, 3, TFHEB_SPLIT_FP32, 1, 3, false, 8.00, launch_g<float, 2048, 3, true, 1, 3>},
+    {2048, 3, TFHEB_SPLIT_FP32, 1, 3, false, 7.86, launch_g<float, 2048, 3, true, 1, 3>},
+    // one bootstrap on two SMs, D counting 16 KB rows: 3.46 ms per wave of 74, where the entry above takes 5.9
+    {2048, 3, TFHEB_SPLIT_FP32, 1, 5, false, 4.33, launch_latency<float, 3, 2, 2048>, 0, 32, 2},
     {2048, 3, TFHEB_SPLIT_FP32, 2, 4, true, 12.86, launch_paired<2048, 3, 2, 4, 2, false>, 1},
     {2048, 3, TFHEB_SPLIT_FP32, 2, 4, true, 10.56, launch_paired<2048, 3, 2, 4, 2, true>, 1},
     // the warp kernel, D counting 32 KB units: 10.63 ms per wave of 592, against 10.19 ms per 444 for the first entry
@@ -588,14 +592,14 @@ static const BrVariant kBrVariants[] = {
     {1024, 2, TFHEB_SPLIT_FP32, 7, 4, true, 11.49, launch_g<float, 1024, 2, true, 7, 4>},
     {1024, 2, TFHEB_SPLIT_FP32, 8, 8, true, 8.60, launch_warp_split2<8>, 1, 23},
     {1024, 2, TFHEB_SPLIT_FP32, 4, 8, false, 4.82, launch_warp_split2<4>, 1, 23},
-    {1024, 2, TFHEB_SPLIT_FP32, 1, 2, false, 2.58, launch_latency<float, 2, 1>},
-    {1024, 2, TFHEB_SPLIT_FP32, 1, 2, false, 1.82, launch_latency<float, 2, 2>, 0, 32, 2},
+    {1024, 2, TFHEB_SPLIT_FP32, 1, 2, false, 2.58, launch_latency<float, 2, 1, 1024>},
+    {1024, 2, TFHEB_SPLIT_FP32, 1, 2, false, 1.82, launch_latency<float, 2, 2, 1024>, 0, 32, 2},
     {1024, 2, TFHEB_FP64, 4, 4, true, 7.90, launch_g<double, 1024, 2, false, 4, 4, false>},
     {1024, 2, TFHEB_FP64, 4, 4, true, 8.38, launch_g<double, 1024, 2, false, 4, 4>},
     {1024, 2, TFHEB_FP64, 8, 8, true, 11.66, launch_warp<false, 2, 8, 8>},
     {1024, 2, TFHEB_FP64, 4, 8, false, 6.35, launch_warp_duo<false, 2, 4, 8>},
-    {1024, 2, TFHEB_FP64, 1, 2, false, 2.98, launch_latency<double, 2, 1>},
-    {1024, 2, TFHEB_FP64, 1, 1, false, 2.10, launch_latency<double, 2, 2>, 0, 32, 2},
+    {1024, 2, TFHEB_FP64, 1, 2, false, 2.98, launch_latency<double, 2, 1, 1024>},
+    {1024, 2, TFHEB_FP64, 1, 1, false, 2.10, launch_latency<double, 2, 2, 1024>, 0, 32, 2},
 };
 
 int br_variants(int N, int l, int precision, int *G, int *D, int cap) {

@@ -1,5 +1,6 @@
 // blind_rotate_latency.cu -- the blind rotation of few bootstraps (tfhe_blindRotate_FFT,
-// lwe-bootstrapping-functions-fft.cpp:88-112): one bootstrap per CTA, or per cluster of two CTAs; N = 1024.
+// lwe-bootstrapping-functions-fft.cpp:88-112): one bootstrap per CTA, or per cluster of two CTAs; N = 1024, and the
+// split form at N = 2048 on two CTAs (3.46 ms per wave of 74, against 5.9 ms for one team of blind_rotate_kernel).
 //
 // A batch far below one wave (a single drop-in gate, a few dozen concurrent callers) waits for one bootstrap's
 // serial chain of n steps, so a step is spread over as many warps as it has independent work:
@@ -20,9 +21,10 @@
 // Every accumulator takes the same products in the same order as in blind_rotate_kernel, and each transform
 // runs the same operations, so the bits are the same.
 //
-// The key streams through a ring of two stages (48 KB each at l = 3: a step's rows of one output with C = 2,
-// three digits' rows of both with C = 1), issued by a warp of its own.  Waits are bounded as in
-// blind_rotate_kernel.  After one that ran out, all threads of the CTA leave the loop at the end of the same
+// The key streams through a ring, issued by a warp of its own: two stages of 48 KB at l = 3 (a step's rows of one
+// output with C = 2, three digits' rows of both with C = 1).  N = 2048 has room for five of one digit's row (16 KB),
+// each given back as soon as its words are in registers (after the products instead: 3.70 ms).
+// Waits are bounded as in blind_rotate_kernel.  After one that ran out, all threads of the CTA leave the loop at the end of the same
 // step, the other CTA's next wait runs out too, and the last barrier (all threads of the cluster) keeps
 // each CTA's shared memory alive until the other's stores have landed.
 #include <cuda_runtime.h>
@@ -37,20 +39,23 @@ namespace tfheb {
 
 namespace {
 
-template <typename T, int L, int C>
+template <typename T, int L, int C, int N_>
 struct LatencyLayout {
-    static constexpr int N = 1024, M = N / 2, NT = M / kR, KP1 = 2, KPL = KP1 * L;
-    static constexpr bool split = sizeof(T) == 4;
+    static constexpr int N = N_, M = N / 2, NT = M / kR, KP1 = 2, KPL = KP1 * L;
+    static constexpr bool split = sizeof(T) == 4, big = N == 2048;
+    static_assert(!big || (split && C == 2 && L == 3), "N = 2048: shared memory for the split form on two CTAs only");
     static constexpr int polys = KP1 / C;                 // polynomials and outputs of a CTA
-    static constexpr int fwd_teams = polys * L;           // 64 threads each
+    static constexpr int fwd_teams = polys * L;           // NT threads each
     static constexpr int inv_teams = polys * (split ? 2 : 1);
-    static constexpr int mac_warps = 8;
-    static constexpr int warps = 2 * fwd_teams > mac_warps ? 2 * fwd_teams : mac_warps;
+    static constexpr int mac_warps = 8, pairs = 4 * NT / (32 * mac_warps);  // slot pairs of a thread per output
+    static constexpr int team_warps = NT / 32;
+    static constexpr int warps = team_warps * fwd_teams > mac_warps ? team_warps * fwd_teams : mac_warps;
     static constexpr int threads = 32 * (warps + 1);
     static constexpr uint32_t half = (uint32_t)M * 16;    // one output's slots of one key row
-    static constexpr int per_step = C == 2 ? 1 : 2;       // ring stages per step
-    static constexpr int D = !split && C == 2 ? 1 : 2;    // ring stages (FP64 needs the room; a step outlasts a refill)
-    static constexpr int stage_digits = KPL / per_step;
+    // ring: D stages of stage_digits digits' rows of the CTA's outputs; the first `early` digits' keys of a step go to
+    // registers before the spectra have arrived
+    static constexpr int stage_digits = big ? 1 : C == 2 ? KPL : L, early = big || C == 1 ? L : KPL;
+    static constexpr int D = big ? 5 : !split && C == 2 ? 1 : 2;  // FP64 needs the room; a step outlasts a refill
     static constexpr uint32_t stage = (uint32_t)stage_digits * polys * half;
     static constexpr size_t spec_bytes = sizeof(cplx<T>) * M;  // one digit's spectrum
     static constexpr size_t bars = 0;  // full[D], empty[D], remote[2], abort flag, stop
@@ -64,19 +69,32 @@ struct LatencyLayout {
     static constexpr size_t spec_in = spec + fwd_teams * spec_bytes;               // [parity][digit] the other CTA's
     static constexpr size_t after_spec = spec_in + (C == 2 ? 2 * L * spec_bytes : 0);
     static constexpr size_t xbuf_bytes = ((size_t)Exch<T, M>::bytes + 15) / 16 * 16;
-    static constexpr int xbufs_of = split || C == 2 ? 2 : 1;  // per team; two save a barrier per exchange
+    static constexpr int xbufs_of = !big && (split || C == 2) ? 2 : 1;  // per team; two save a barrier per exchange
     static constexpr int teams = fwd_teams > inv_teams ? fwd_teams : inv_teams;
-    // [inverse team] the products' spectra: a region of their own, or (FP64 in one CTA, short of room) the exchange
-    // buffers of the teams that have no inverse transform, idle from the forward transforms on
+    // [inverse team] the products' spectra: a region of their own, or where room is short the exchange buffers of
+    // the teams that have no inverse transform, idle from the forward transforms on (FP64 in one CTA), or that of
+    // the last team and the rotated words, which the digits were taken from (N = 2048)
     static constexpr bool sums_in_xbufs = !split && C == 1;
-    static constexpr size_t xbufs = after_spec + (sums_in_xbufs ? 0 : inv_teams * spec_bytes);
-    static constexpr size_t sums = sums_in_xbufs ? xbufs + (size_t)inv_teams * xbuf_bytes : after_spec;
-    static constexpr size_t sum_stride = sums_in_xbufs ? xbuf_bytes : spec_bytes;
+    static constexpr size_t xbufs = after_spec + (sums_in_xbufs || big ? 0 : inv_teams * spec_bytes);
+    __host__ __device__ static constexpr size_t sums(int team) {
+        return sums_in_xbufs ? xbufs + (size_t)(inv_teams + team) * xbuf_bytes
+               : !big        ? after_spec + team * spec_bytes
+               : team == 0   ? rot
+                             : xbufs + (size_t)(teams - 1) * xbufs_of * xbuf_bytes;
+    }
     static_assert(!sums_in_xbufs || (teams >= 2 * inv_teams && xbufs_of == 1), "idle exchange buffers");
+    static_assert(!big || (acc_bytes >= spec_bytes && xbuf_bytes >= spec_bytes && teams > inv_teams), "places of the sums");
     static constexpr size_t bytes = xbufs + (size_t)teams * xbufs_of * xbuf_bytes;
     static_assert((2 * D + 2) * 8 + 8 <= ring, "barrier block");
     static_assert(bytes <= 227 * 1024, "shared memory of the variant");
-    static_assert(2 * inv_teams <= warps, "every inverse transform has a team");
+    static_assert(team_warps * inv_teams <= warps && KPL % stage_digits == 0, "every inverse transform has a team");
+    // place (in float4) of slots 2c, 2c + 1 of thread t in a spectrum.  N = 2048: the multiply-accumulate follows the
+    // key's second layout (key_transform.cu), whose lanes hold t's 8 apart; the low three bits are XORed so that
+    // both sides hit 8 different bank groups
+    __host__ __device__ static constexpr int pair_at(int c, int t) {
+        if (!big) return c * NT + t;
+        return (((c >> 1) * 8 + (t & 7)) * 32 + 16 * (c & 1) + 8 * (t >> 6) + (t >> 3 & 7)) ^ (t & 7);
+    }
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -133,10 +151,10 @@ __device__ __forceinline__ void wait_bounded_cluster(uint32_t bar, uint32_t pari
 
 }  // namespace
 
-template <typename T, int L, int C>
-__global__ void __launch_bounds__(LatencyLayout<T, L, C>::threads, 1) blind_rotate_latency_kernel(const BrArgs args) {
-    using Lay = LatencyLayout<T, L, C>;
-    constexpr int N = Lay::N, M = Lay::M, NT = Lay::NT, KP1 = 2, KPL = Lay::KPL, D = Lay::D;
+template <typename T, int L, int C, int N>
+__global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_rotate_latency_kernel(const BrArgs args) {
+    using Lay = LatencyLayout<T, L, C, N>;
+    constexpr int M = Lay::M, NT = Lay::NT, KP1 = 2, KPL = Lay::KPL, D = Lay::D;
     constexpr bool SPLIT = Lay::split;
     using F = TeamFft<T, M, kR>;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -174,7 +192,7 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C>::threads, 1) blind_rota
     if (warp == Lay::warps) {  // ---- the key's stream ----
         if (lane == 0) {
             const uint8_t *bsk = SPLIT ? args.bsk2 : args.bsk;
-            const int total = args.nsteps * Lay::per_step;
+            const int total = args.nsteps * (KPL / Lay::stage_digits);
             int sent = 0;
             if (!args.stall_producer) {
                 for (int c = 0; c < total; c++) {
@@ -197,7 +215,7 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C>::threads, 1) blind_rota
         }
         __syncwarp();
     } else {  // ---- consumer warps ----
-        const int tid = threadIdx.x, team = warp >> 1, t = tid & (NT - 1);
+        const int tid = threadIdx.x, team = warp / Lay::team_warps, t = tid & (NT - 1);
         uint32_t *s_acc = reinterpret_cast<uint32_t *>(smem + Lay::acc);
         uint32_t *s_low = reinterpret_cast<uint32_t *>(smem + Lay::acc_low);  // split: acc = s_acc + s_low
         uint32_t *s_rot = reinterpret_cast<uint32_t *>(smem + Lay::rot);
@@ -266,29 +284,12 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C>::threads, 1) blind_rota
                 const int i = i0 + tid;
                 if (Lay::polys * N % consumers != 0 && i >= Lay::polys * N) break;
                 const int e = (i & (N - 1)) - ai, src = (i & ~(N - 1)) + (e & (N - 1));
-                const uint32_t neg = (uint32_t)((int32_t)((uint32_t)e << 21) >> 31), on = offset - neg;
+                const uint32_t neg = (uint32_t)((int32_t)((uint32_t)e << (N == 2048 ? 20 : 21)) >> 31), on = offset - neg;
                 const uint32_t x = SPLIT ? s_acc[src] + s_low[src] : s_acc[src];
                 const uint32_t y = SPLIT ? s_acc[i] + s_low[i] : s_acc[i];
                 s_rot[i] = (x ^ neg) + (on - y);
             }
             team_sync(kAllBar, consumers);
-
-            // the keys of the multiply-accumulate below: thread (m, tm) takes slots 2m, 2m + 1 of virtual thread tm
-            const int m = tid >> 6, tm = tid & (NT - 1);
-            float4 key[Lay::stage_digits][Lay::polys][2];  // split {hi.re, lo.re, hi.im, lo.im}; FP64 {re, im}
-            auto load_keys = [&](int c) {
-                const int s = c % D;
-                wait_bounded(full_bar(s), (c / D) & 1, abort_flag, args.timeout_ns, args.err);
-                const unsigned char *at = smem + Lay::ring + (size_t)s * Lay::stage + 16 * (size_t)(2 * m * NT + tm);
-#pragma unroll
-                for (int dd = 0; dd < Lay::stage_digits; dd++)
-#pragma unroll
-                    for (int v = 0; v < Lay::polys; v++)
-#pragma unroll
-                        for (int i = 0; i < 2; i++)
-                            key[dd][v][i] = *reinterpret_cast<const float4 *>(
-                                at + (size_t)((SPLIT || C == 1 || rank == 0 ? dd : (dd + L) % KPL) * Lay::polys + v) * Lay::half + 16 * i * NT);
-            };
 
             // 2. digit, forward transform, spectrum out
             if (team < Lay::fwd_teams) {
@@ -301,71 +302,108 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C>::threads, 1) blind_rota
                     z[r] = cplx<T>{d0, -d1};  // a_j - i a_{j+M}; the twist is folded into the FFT
                 }
                 F::forward(z, xp, s_tw, t, 1 + team);
-                const uint32_t far = far_spec + (uint32_t)(parity * L * Lay::spec_bytes) + 16u * (uint32_t)t;
+                const uint32_t far = far_spec + (uint32_t)(parity * L * Lay::spec_bytes);
                 const uint32_t bar = far_bar + 8u * (uint32_t)parity;
                 if constexpr (SPLIT) {
-                    // [register pair m][t] {re(2m), im(2m), re(2m+1), im(2m+1)}
+                    // per register pair m {re(2m), im(2m), re(2m+1), im(2m+1)}
 #pragma unroll
                     for (int m = 0; m < kR / 2; m++) {
                         const float4 v = make_float4(z[2 * m].re, z[2 * m].im, z[2 * m + 1].re, z[2 * m + 1].im);
-                        if constexpr (C == 2) store_remote(far + 16u * (uint32_t)(m * NT), v, bar);
-                        reinterpret_cast<float4 *>(my_spec)[m * NT + t] = v;
+                        if constexpr (C == 2) store_remote(far + 16u * (uint32_t)Lay::pair_at(m, t), v, bar);
+                        reinterpret_cast<float4 *>(my_spec)[Lay::pair_at(m, t)] = v;
                     }
                 } else {
                     // [r][t] {re, im}
 #pragma unroll
                     for (int r = 0; r < kR; r++) {
                         const double2 v = make_double2(z[r].re, z[r].im);
-                        if constexpr (C == 2) store_remote(far + 16u * (uint32_t)(r * NT), v, bar);
+                        if constexpr (C == 2) store_remote(far + 16u * (uint32_t)(r * NT + t), v, bar);
                         reinterpret_cast<double2 *>(my_spec)[r * NT + t] = v;
                     }
                 }
             }
 
-            // 3. multiply-accumulate.  The keys come in while the spectra are on their way to the other CTA; read before
-            // the forward transform they delayed it (2.17 against 1.97 us per step).
-            if (warp < Lay::mac_warps) load_keys(step * Lay::per_step);
+            // 3. multiply-accumulate: a thread takes slots 2c, 2c + 1 of one virtual thread t (N = 2048: of two, c 2
+            //    apart, in the order of the key's second layout).  The keys of the first digits come in while the
+            //    spectra are on their way to the other CTA; read before the forward transform they delayed it
+            //    (2.17 against 1.97 us per step).
+            auto pair = [&](int i) { return Lay::big ? (i * 256 + tid) ^ (warp & 7) : tid; };  // Lay::pair_at of pair i
+            auto key_at = [&](int i, int k) {  // slot 2c + k of pair i in a key row's half
+                if constexpr (Lay::big) return i * 512 + k * 256 + tid;
+                else return (2 * (tid / NT) + k) * NT + (tid & (NT - 1));
+            };
+            // the step's digit at turn dd.  FP64 sums round to the exact integers in any order: there the CTA's own
+            // digits go first, before the wait.  The split form's low limb keeps the digits' order.
+            auto digit = [&](int dd) { return SPLIT || C == 1 || rank == 0 ? dd : (dd + L) % KPL; };
+            float4 key[Lay::early][Lay::polys][Lay::pairs][2];  // split {hi.re, lo.re, hi.im, lo.im}; FP64 {re, im}
+            auto load_key = [&](int dd) {
+                const int c = (step * KPL + dd) / Lay::stage_digits, s = c % D;
+                if (dd % Lay::stage_digits == 0)
+                    wait_bounded(full_bar(s), (c / D) & 1, abort_flag, args.timeout_ns, args.err);
+                const unsigned char *row = smem + Lay::ring + (size_t)s * Lay::stage +
+                                           (size_t)(digit(dd) % Lay::stage_digits) * Lay::polys * Lay::half;
+#pragma unroll
+                for (int v = 0; v < Lay::polys; v++)
+#pragma unroll
+                    for (int i = 0; i < Lay::pairs; i++)
+#pragma unroll
+                        for (int e = 0; e < 2; e++)
+                            key[dd % Lay::early][v][i][e] = reinterpret_cast<const float4 *>(row + v * Lay::half)[key_at(i, e)];
+            };
+            auto release = [&](int dd) {  // after the last digit of a stage
+                if ((dd + 1) % Lay::stage_digits != 0) return;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(empty_bar((step * KPL + dd) / Lay::stage_digits % D));
+            };
+            if (warp < Lay::mac_warps) {
+#pragma unroll
+                for (int dd = 0; dd < Lay::early; dd++) {
+                    load_key(dd);
+                    if (Lay::big) release(dd);
+                }
+            }
             team_sync(kAllBar, consumers);
             if (warp < Lay::mac_warps) {
                 auto wait_remote = [&] {
                     if constexpr (C == 2)
                         wait_bounded_cluster(remote_bar(parity), (uint32_t)(step >> 1) & 1u, abort_flag, args.timeout_ns, args.err);
                 };
-                // FP64 sums round to the exact integers in any order: the CTA's own digits go first, before the
-                // wait.  The split form's low limb keeps the digits' order.
                 if constexpr (SPLIT) wait_remote();
-                cpair acc2[Lay::polys][2];
-                cplx<double> accd[Lay::polys][2];
+                cpair acc2[Lay::polys][Lay::pairs][2];
+                cplx<double> accd[Lay::polys][Lay::pairs][2];
 #pragma unroll
                 for (int v = 0; v < Lay::polys; v++)
 #pragma unroll
-                    for (int i = 0; i < 2; i++) {
-                        acc2[v][i] = {{0.f, 0.f}, {0.f, 0.f}};
-                        accd[v][i] = {0.0, 0.0};
+                    for (int i = 0; i < 2 * Lay::pairs; i++) {
+                        acc2[v][i / 2][i % 2] = {{0.f, 0.f}, {0.f, 0.f}};
+                        accd[v][i / 2][i % 2] = {0.0, 0.0};
                     }
 #pragma unroll
-                for (int st = 0; st < Lay::per_step; st++) {
-                    const int c = step * Lay::per_step + st;
-                    if (st > 0) load_keys(c);
+                for (int dd = 0; dd < KPL; dd++) {
+                    if (!SPLIT && C == 2 && dd == L) wait_remote();
+                    if (dd > 0 && dd % Lay::early == 0)
 #pragma unroll
-                    for (int dd = 0; dd < Lay::stage_digits; dd++) {
-                        if (!SPLIT && C == 2 && dd == L) wait_remote();
-                        const int first = SPLIT || C == 1 ? dd : rank ? (dd + L) % KPL : dd;  // digit of this turn
-                        const int d = st * Lay::stage_digits + first, u = d / L, q = d - u * L;
-                        const unsigned char *sp = smem + Lay::spec + (size_t)d * Lay::spec_bytes;
-                        if constexpr (C == 2)
-                            sp = u == rank ? smem + Lay::spec + (size_t)q * Lay::spec_bytes
-                                           : smem + Lay::spec_in + (size_t)(parity * L + q) * Lay::spec_bytes;
+                        for (int e = 0; e < Lay::early; e++) {
+                            load_key(dd + e);
+                            if (Lay::big) release(dd + e);
+                        }
+                    const int d = digit(dd), u = d / L, q = d - u * L;
+                    const unsigned char *sp = smem + Lay::spec + (size_t)d * Lay::spec_bytes;
+                    if constexpr (C == 2)
+                        sp = u == rank ? smem + Lay::spec + (size_t)q * Lay::spec_bytes
+                                       : smem + Lay::spec_in + (size_t)(parity * L + q) * Lay::spec_bytes;
+#pragma unroll
+                    for (int i = 0; i < Lay::pairs; i++) {
                         if constexpr (SPLIT) {
-                            const float4 f = reinterpret_cast<const float4 *>(sp)[m * NT + tm];
+                            const float4 f = reinterpret_cast<const float4 *>(sp)[pair(i)];
 #pragma unroll
                             for (int v = 0; v < Lay::polys; v++)
 #pragma unroll
-                                for (int i = 0; i < 2; i++) {
-                                    const float4 k = key[dd][v][i];
-                                    const float zr = i ? f.z : f.x, zi = i ? f.w : f.y;
+                                for (int e = 0; e < 2; e++) {
+                                    const float4 k = key[dd % Lay::early][v][i][e];
+                                    const float zr = e ? f.z : f.x, zi = e ? f.w : f.y;
                                     const float2 kr = make_float2(k.x, k.y), ki = make_float2(k.z, k.w);
-                                    cpair &a = acc2[v][i];
+                                    cpair &a = acc2[v][i][e];
                                     a.re = fma2(bc2(zr), kr, a.re);
                                     a.im = fma2(bc2(zr), ki, a.im);
                                     a.re = fma2(bc2(-zi), ki, a.re);
@@ -373,48 +411,49 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C>::threads, 1) blind_rota
                                 }
                         } else {
 #pragma unroll
-                            for (int i = 0; i < 2; i++) {
-                                const double2 f = reinterpret_cast<const double2 *>(sp)[(2 * m + i) * NT + tm];
+                            for (int e = 0; e < 2; e++) {
+                                const double2 f = reinterpret_cast<const double2 *>(sp)[key_at(i, e)];
 #pragma unroll
                                 for (int v = 0; v < Lay::polys; v++) {
-                                    const float4 k = key[dd][v][i];
+                                    const float4 k = key[dd % Lay::early][v][i][e];
                                     const cplx<double> kd{
                                         __hiloint2double(__float_as_int(k.y), __float_as_int(k.x)),
                                         __hiloint2double(__float_as_int(k.w), __float_as_int(k.z))};
-                                    cmac(accd[v][i], cplx<double>{f.x, f.y}, kd);
+                                    cmac(accd[v][i][e], cplx<double>{f.x, f.y}, kd);
                                 }
                             }
                         }
                     }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(empty_bar(c % D));
+                    if (!Lay::big) release(dd);
                 }
                 // to the inverse teams: (output v, limb) in the layouts of the spectra
 #pragma unroll
-                for (int v = 0; v < Lay::polys; v++) {
-                    if constexpr (SPLIT) {
-                        const cpair &a = acc2[v][0], &b = acc2[v][1];
-                        float4 *hi = reinterpret_cast<float4 *>(smem + Lay::sums + (size_t)(2 * v) * Lay::sum_stride);
-                        float4 *lo = reinterpret_cast<float4 *>(smem + Lay::sums + (size_t)(2 * v + 1) * Lay::sum_stride);
-                        hi[m * NT + tm] = make_float4(a.re.x, a.im.x, b.re.x, b.im.x);
-                        lo[m * NT + tm] = make_float4(a.re.y, a.im.y, b.re.y, b.im.y);
-                    } else {
-                        double2 *o = reinterpret_cast<double2 *>(smem + Lay::sums + (size_t)v * Lay::sum_stride);
+                for (int v = 0; v < Lay::polys; v++)
 #pragma unroll
-                        for (int i = 0; i < 2; i++) o[(2 * m + i) * NT + tm] = make_double2(accd[v][i].re, accd[v][i].im);
+                    for (int i = 0; i < Lay::pairs; i++) {
+                        if constexpr (SPLIT) {
+                            const cpair &a = acc2[v][i][0], &b = acc2[v][i][1];
+                            reinterpret_cast<float4 *>(smem + Lay::sums(2 * v))[pair(i)] =
+                                make_float4(a.re.x, a.im.x, b.re.x, b.im.x);
+                            reinterpret_cast<float4 *>(smem + Lay::sums(2 * v + 1))[pair(i)] =
+                                make_float4(a.re.y, a.im.y, b.re.y, b.im.y);
+                        } else {
+                            double2 *o = reinterpret_cast<double2 *>(smem + Lay::sums(v));
+#pragma unroll
+                            for (int e = 0; e < 2; e++) o[key_at(i, e)] = make_double2(accd[v][i][e].re, accd[v][i][e].im);
+                        }
                     }
-                }
             }
             team_sync(kAllBar, consumers);
 
             // 4. inverse transforms, exact rounding, accumulate
             if (team < Lay::inv_teams) {
-                const unsigned char *in = smem + Lay::sums + (size_t)team * Lay::sum_stride;
+                const unsigned char *in = smem + Lay::sums(team);
                 cplx<T> z[kR];
                 if constexpr (SPLIT) {
 #pragma unroll
                     for (int i = 0; i < kR / 2; i++) {
-                        const float4 w = reinterpret_cast<const float4 *>(in)[i * NT + t];
+                        const float4 w = reinterpret_cast<const float4 *>(in)[Lay::pair_at(i, t)];
                         z[2 * i] = {w.x, w.y};
                         z[2 * i + 1] = {w.z, w.w};
                     }
@@ -464,11 +503,11 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C>::threads, 1) blind_rota
     if constexpr (C == 2) cluster_sync();
 }
 
-template <typename T, int L, int C>
+template <typename T, int L, int C, int N>
 cudaError_t launch_latency(const BrArgs &a, cudaStream_t s) {
-    using Lay = LatencyLayout<T, L, C>;
+    using Lay = LatencyLayout<T, L, C, N>;
     if (Lay::split && !a.bsk2) return cudaErrorInvalidValue;
-    auto kern = blind_rotate_latency_kernel<T, L, C>;
+    auto kern = blind_rotate_latency_kernel<T, L, C, N>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::bytes);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
@@ -485,13 +524,14 @@ cudaError_t launch_latency(const BrArgs &a, cudaStream_t s) {
     return cudaLaunchKernelEx(&cfg, kern, a);
 }
 
-template cudaError_t launch_latency<float, 3, 1>(const BrArgs &, cudaStream_t);
-template cudaError_t launch_latency<float, 3, 2>(const BrArgs &, cudaStream_t);
-template cudaError_t launch_latency<double, 3, 1>(const BrArgs &, cudaStream_t);
-template cudaError_t launch_latency<double, 3, 2>(const BrArgs &, cudaStream_t);
-template cudaError_t launch_latency<float, 2, 1>(const BrArgs &, cudaStream_t);
-template cudaError_t launch_latency<float, 2, 2>(const BrArgs &, cudaStream_t);
-template cudaError_t launch_latency<double, 2, 1>(const BrArgs &, cudaStream_t);
-template cudaError_t launch_latency<double, 2, 2>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_latency<float, 3, 1, 1024>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_latency<float, 3, 2, 1024>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_latency<double, 3, 1, 1024>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_latency<double, 3, 2, 1024>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_latency<float, 2, 1, 1024>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_latency<float, 2, 2, 1024>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_latency<double, 2, 1, 1024>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_latency<double, 2, 2, 1024>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_latency<float, 3, 2, 2048>(const BrArgs &, cudaStream_t);
 
 }  // namespace tfheb

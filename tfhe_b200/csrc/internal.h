@@ -218,8 +218,8 @@ template <bool SPLIT, int L, int G, int D>
 cudaError_t launch_warp_duo(const BrArgs &a, cudaStream_t s);
 template <bool SPLIT, int L, int G>
 cudaError_t launch_warp_big(const BrArgs &a, cudaStream_t s);
-// blind_rotate_latency.cu: one bootstrap per CTA (C = 1) or per cluster of two (C = 2), N = 1024
-template <typename T, int L, int C>
+// blind_rotate_latency.cu: one bootstrap per CTA (C = 1) or per cluster of two (C = 2)
+template <typename T, int L, int C, int N>
 cudaError_t launch_latency(const BrArgs &a, cudaStream_t s);
 // keyswitch.cu: device key upload (both layouts) and the keyswitch of `count` extracted samples
 // (rows of in_stride int32) into rows of n+1 int32.
