@@ -106,3 +106,30 @@ def test_mixed_batch_rejects_bad_rows(keys):
         ck.gate_mixed_device(g, [0, 1], [2, 3], None, [3, 3], d, 4)
     with pytest.raises(tb.api.TfhebError, match="output row out of range"):
         ck.gate_mixed_device(g, [0, 1], [2, 3], None, [0, -1], d, 4)
+
+
+# ragged levels from a few gates to several waves' worth: whichever assignment of gates to levels is taken, each wire
+# has the bits of its gate evaluated by itself
+@pytest.mark.parametrize("precision", [tb.FP64, tb.SPLIT_FP32])
+@pytest.mark.parametrize("levels,width", [(1, 1), (4, 30), (8, 100), (6, 300), (5, 700), (6, 1200), (2, 2600)])
+def test_netlist_wires_equal_gates_one_layer_at_a_time(levels, width, precision):
+    sk, ck = tb.keygen(tb.make_params(12, 1024, 1, 3, 7, 8, 2), seed=31)
+    ck.to_device(0, precisions=(precision,))
+    rng = np.random.default_rng(width)
+    ni, gates, ia, ib, ic = random_netlist(rng, levels, max(1, width // 16), width, mix=ALL_GATES)
+    depth = np.zeros(ni + len(gates), np.int64)
+    for g, code in enumerate(gates):
+        srcs = (ia[g],) if code >= tb.api.NOT else ((ia[g], ib[g], ic[g]) if code == tb.api.MUX else (ia[g], ib[g]))
+        depth[ni + g] = 1 + max(depth[s] for s in srcs)
+    wires = torch.zeros((ni + len(gates), 13), dtype=torch.int32, device="cuda")
+    wires[:ni] = torch.from_numpy(sk.encrypt(rng.integers(0, 2, ni), seed=9))
+    want = wires.clone()
+    nl = Netlist(ck, ni, gates, ia, ib, ic)
+    nl.run(wires, precision=precision, use_graph=True)
+    for lv in range(1, depth.max() + 1):
+        g = np.flatnonzero(depth[ni:] == lv)
+        ck.gate_mixed_device(*(x[g].astype(np.int32) for x in (gates, ia, ib, ic)), (ni + g).astype(np.int32), want,
+                             len(want), precision=precision)
+    ck.synchronize()
+    assert torch.equal(wires, want)
+    nl.free()

@@ -725,6 +725,13 @@ static int first_wave(const tfheb_params &p, int big, int count, int sms, const 
     return first;
 }
 
+float br_rest_us(const tfheb_params &p, int precision, const BrChoice &choice, int sms, int count) {
+    const int big = br_chosen_global(p, precision, choice);
+    float us = 0;
+    if (big >= 0 && count > 0) first_wave(p, big, count, sms, choice, &us);
+    return us;
+}
+
 // Full waves of the chosen variant (SMs x G bootstraps each), then the rest in waves of whatever runs that many
 // per CTA fastest: 4096 split bootstraps are 3 waves of 1184 and 544 spread over 4 per CTA (20.7 + 3.9 ms,
 // where a fourth packed wave takes 6.9).  A lone bootstrap runs its 630 steps in 1.24 ms on two SMs, 1.84 ms

@@ -161,7 +161,9 @@ cudaError_t launch_blind_rotate(const tfheb_params &p, int precision, const Devi
                                 uint64_t timeout_ns, const BrChoice &choice, int *launches = nullptr);
 // Index into the whole table of the variant a key's choice means (tuned = -1: the default rule), or -1.
 int br_chosen_global(const tfheb_params &p, int precision, const BrChoice &choice);
-// The same with one compiled variant given by its index into the whole table (for timing).
+// Measured time (us per step, 0 if not known) of launch_blind_rotate's waves for a rest of `count`, at most one wave.
+float br_rest_us(const tfheb_params &p, int precision, const BrChoice &choice, int sms, int count);
+// launch_blind_rotate with one compiled variant given by its index into the whole table (for timing).
 cudaError_t launch_blind_rotate_exact(const tfheb_params &p, int precision, const DeviceBsk &bsk, const int32_t *bara,
                                       int bara_stride, int boots, int nsteps, int32_t mu, const int32_t *acc_in,
                                       int32_t *acc_out, cudaStream_t s, int32_t *d_err, int stall_producer,

@@ -3,7 +3,7 @@
 // The reference evaluates circuits one gate call at a time (e.g. test-long-run.cpp:61-185,
 // test-addition-boot.cpp); here the whole circuit is scheduled at creation:
 //   * each gate gets a level: the earliest is 1 + the deepest level among its inputs (primary inputs
-//     are level 0); gates with slack then move later to fill blind-rotation waves (pack_levels),
+//     are level 0); gates with slack then move later to levels where the blind rotation has room (pack_levels),
 //     keeping the number of levels at the critical path length;
 //   * gates are renumbered level by level into an internal wire array, bootstrapped gates first in
 //     each level, so a level's outputs are one contiguous block of rows;
@@ -91,7 +91,7 @@ struct Level {
 namespace tfheb {
 namespace {
 // One level schedule of a netlist: levels, their descriptors and the internal row order.  Each
-// precision has its own, packed for the wave of that precision's blind-rotation variant.
+// precision has its own, packed by the times of that precision's blind-rotation variants.
 struct Schedule {
     std::vector<Level> levels;
     int max_boots = 0, max_gates = 0;
@@ -209,27 +209,54 @@ cudaError_t enqueue_netlist(tfheb_netlist *nl, CloudKey &ck, int precision, int3
     return e;
 }
 
-// Bootstraps one blind-rotation launch runs per wave: SMs x bootstraps per CTA of the key's current
-// variant for `precision`.
-int wave_bootstraps(const CloudKey &ck, int precision) {
-    int sms = 0, G = 1;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ck.device);
-    const int g = br_chosen_global(ck.p, precision, ck.br[precision]);
-    if (g >= 0) br_variant_info(g, nullptr, nullptr, nullptr, &G, nullptr, nullptr);
-    return std::max(1, sms) * G;
-}
+// What the blind rotation of a level of `boots` bootstraps takes, in us per step as the variant table has it: whole
+// waves, and the rest by steps of half an SM count (a rest's variants depend on no more than that).  With `shards`
+// keys a level is spread evenly over them.
+struct LevelCost {
+    int sms = 1, wave = 1, shards = 1;  // wave: bootstraps a launch of one key's variant runs at once
+    float full = 0;                     // a whole wave; 0: not known
+    std::vector<float> rest;            // a rest of up to a SMs + half of them, and of up to a + 1 SMs
 
-// Level assignment that fills blind-rotation waves.  `level` holds each gate's earliest level
-// (1 + its deepest input) on entry.  Every gate gets a deadline, its latest level that keeps the
-// number of levels at nlev (1 below the earliest deadline among its consumers; nlev without
-// consumers).  Level s then takes every ready gate whose deadline is s, and tops the level up with
-// other ready gates, earliest deadline first, while its bootstraps stay within the waves the
-// mandatory gates already start (a multiple of `wave`).  A gate is ready once all its inputs sit on
-// earlier levels, so the evaluation order stays valid; NOT/COPY gates (no bootstrap) go on the
-// first level where they are ready.
+    LevelCost(const CloudKey &ck, int precision, int shards_) : shards(shards_) {
+        int G = 1;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ck.device);
+        sms = std::max(1, sms);
+        const int g = br_chosen_global(ck.p, precision, ck.br[precision]);
+        if (g >= 0) br_variant_info(g, nullptr, nullptr, nullptr, &G, nullptr, nullptr);
+        wave = sms * G;
+        for (int a = 0; a < G; a++)
+            for (int end : {a * sms + std::max(1, sms / 2), (a + 1) * sms})
+                rest.push_back(br_rest_us(ck.p, precision, ck.br[precision], sms, end));
+        full = rest.back();
+        if (*std::min_element(rest.begin(), rest.end()) <= 0) full = 0;
+    }
+    int64_t one(int64_t boots) const { return (boots + shards - 1) / shards; }
+    double operator()(int64_t boots) const {
+        const int64_t b = one(boots), waves = b / wave;
+        const int left = (int)(b - waves * wave), a = left > 0 ? (left - 1) / sms : 0;
+        return (double)waves * full + (left == 0 ? 0.f : rest[2 * a + (left - a * sms > std::max(1, sms / 2))]);
+    }
+    // the most bootstraps that cost no more than `boots`
+    int64_t step_end(int64_t boots) const {
+        const int64_t b = std::max<int64_t>(1, one(boots)), whole = (b - 1) / sms * sms;
+        return (whole + (b - whole <= sms / 2 ? sms / 2 : sms)) * shards;
+    }
+};
+
+// Level assignment by the blind rotation's cost.  `level` holds each gate's earliest level (1 + its deepest input)
+// on entry.  Every gate gets a deadline, its latest level that keeps the number of levels at nlev (1 below the
+// earliest deadline among its consumers; nlev without consumers).  Level s then takes every ready gate whose
+// deadline is s, and tops the level up with other ready gates, earliest deadline first, up to a cap.  A gate is
+// ready once all its inputs sit on earlier levels, so the evaluation order stays valid; NOT/COPY gates (no
+// bootstrap) go on the first level where they are ready.
+// The cap is the end of the waves that the mandatory gates start, waves being counted in the variant's, in half of
+// them, in SMs or in half SMs; or it is where topping up pays most, at a full wave's cost per bootstrap.  No one of
+// them is best throughout, so each is tried and the assignment with the least sum of costs taken.  Measured, split
+// form: ten levels of 75 to 1200 gates 42.6 ms (by half waves; 52.1 by whole ones), six of 18 to 300 11.2 (by SMs;
+// 13.1 by the costs), eight of 6 to 100 10.1 (by half SMs; 11.9).  Creation takes 3.7 instead of 2.4 ms for 5775 gates.
 void pack_levels(int num_inputs, int num_gates, const int32_t *gates, const int32_t *in_a, const int32_t *in_b,
-                 const int32_t *in_c, int nlev, int wave, std::vector<int> &level) {
-    if (num_gates == 0 || wave <= 1) return;
+                 const int32_t *in_c, int nlev, const LevelCost &cost, std::vector<int> &level) {
+    if (num_gates == 0 || cost.wave * cost.shards <= 1) return;
     const int32_t *ins[3] = {in_a, in_b, in_c};
     auto nin = [&](int g) { return gates[g] == TFHEB_MUX ? 3 : (gates[g] >= TFHEB_NOT ? 1 : 2); };
     auto boots = [&](int g) { return gates[g] == TFHEB_MUX ? 2 : (gates[g] >= TFHEB_NOT ? 0 : 1); };
@@ -241,11 +268,11 @@ void pack_levels(int num_inputs, int num_gates, const int32_t *gates, const int3
             if (src >= 0) deadline[src] = std::min(deadline[src], deadline[g] - 1);
         }
     // consumer lists and unscheduled-input counts
-    std::vector<int> cons_off(num_gates + 1, 0), waiting(num_gates, 0);
+    std::vector<int> cons_off(num_gates + 1, 0), inputs(num_gates, 0);
     for (int g = 0; g < num_gates; g++)
         for (int k = 0; k < nin(g); k++) {
             const int src = ins[k][g] - num_inputs;
-            if (src >= 0) cons_off[src + 1]++, waiting[g]++;
+            if (src >= 0) cons_off[src + 1]++, inputs[g]++;
         }
     for (int g = 0; g < num_gates; g++) cons_off[g + 1] += cons_off[g];
     std::vector<int> cons(cons_off[num_gates]), fill(cons_off.begin(), cons_off.end() - 1);
@@ -254,40 +281,71 @@ void pack_levels(int num_inputs, int num_gates, const int32_t *gates, const int3
             const int src = ins[k][g] - num_inputs;
             if (src >= 0) cons[fill[src]++] = g;
         }
-    // ready gates bucketed by deadline; unary gates in their own list
-    std::vector<std::vector<int>> bucket(nlev + 2);
-    std::vector<size_t> head(nlev + 2, 0);
-    std::vector<int> unary_ready;
-    auto make_ready = [&](int g) {
-        if (boots(g) == 0) unary_ready.push_back(g);
-        else bucket[deadline[g]].push_back(g);
-    };
-    for (int g = 0; g < num_gates; g++)
-        if (waiting[g] == 0) make_ready(g);
-    std::vector<int> placed;
-    for (int s = 1; s <= nlev; s++) {
-        placed.clear();
-        std::vector<int> un;
-        un.swap(unary_ready);
-        for (int g : un) placed.push_back(g);
-        int used = 0;
-        for (; head[s] < bucket[s].size(); head[s]++) {  // mandatory: deadline s
-            const int g = bucket[s][head[s]];
-            placed.push_back(g);
-            used += boots(g);
-        }
-        const int cap = (std::max(used, 1) + wave - 1) / wave * wave;
-        for (int t = s + 1; t <= nlev && used < cap; t++)
-            for (; head[t] < bucket[t].size() && used + boots(bucket[t][head[t]]) <= cap; head[t]++) {
-                const int g = bucket[t][head[t]];
+    // one assignment; cap(used, ready) for `used` mandatory and `ready` possible bootstraps.  Returns its cost.
+    auto assign = [&](auto &&cap_of, std::vector<int> &out) {
+        // ready gates bucketed by deadline; unary gates in their own list
+        std::vector<std::vector<int>> bucket(nlev + 2);
+        std::vector<size_t> head(nlev + 2, 0);
+        std::vector<int> unary_ready, placed, un, waiting(inputs);
+        int64_t ready = 0;  // bootstraps in the buckets
+        auto make_ready = [&](int g) {
+            if (boots(g) == 0) unary_ready.push_back(g);
+            else bucket[deadline[g]].push_back(g), ready += boots(g);
+        };
+        for (int g = 0; g < num_gates; g++)
+            if (waiting[g] == 0) make_ready(g);
+        double total = 0;
+        for (int s = 1; s <= nlev; s++) {
+            placed.clear();
+            un.clear();
+            un.swap(unary_ready);
+            for (int g : un) placed.push_back(g);
+            int64_t used = 0;
+            for (; head[s] < bucket[s].size(); head[s]++) {  // mandatory: deadline s
+                const int g = bucket[s][head[s]];
                 placed.push_back(g);
                 used += boots(g);
             }
-        for (int g : placed) level[num_inputs + g] = s;
-        for (int g : placed)
-            for (int i = cons_off[g]; i < cons_off[g + 1]; i++)
-                if (--waiting[cons[i]] == 0) make_ready(cons[i]);
-    }
+            const int64_t cap = cap_of(used, ready);
+            for (int t = s + 1; t <= nlev && used < cap; t++)
+                for (; head[t] < bucket[t].size() && used + boots(bucket[t][head[t]]) <= cap; head[t]++) {
+                    const int g = bucket[t][head[t]];
+                    placed.push_back(g);
+                    used += boots(g);
+                }
+            ready -= used;
+            total += cost(used);
+            for (int g : placed) out[num_inputs + g] = s;
+            for (int g : placed)
+                for (int i = cons_off[g]; i < cons_off[g + 1]; i++)
+                    if (--waiting[cons[i]] == 0) make_ready(cons[i]);
+        }
+        return total;
+    };
+    const int64_t wave = (int64_t)cost.wave * cost.shards, per_sm = (int64_t)cost.sms * cost.shards;
+    auto waves_of = [](int64_t w) {
+        return [w](int64_t used, int64_t) { return (std::max<int64_t>(used, 1) + w - 1) / w * w; };
+    };
+    double least = assign(waves_of(wave), level);
+    if (cost.full <= 0) return;  // no measured times: the variant's waves
+    auto consider = [&](auto &&cap_of) {
+        std::vector<int> other(level);
+        const double t = assign(cap_of, other);
+        if (t < least) least = t, level.swap(other);
+    };
+    for (int64_t w : {wave / 2, per_sm})
+        if (w < wave) consider(waves_of(w));
+    consider([&](int64_t used, int64_t) { return cost.step_end(used); });
+    consider([&](int64_t used, int64_t ready) {
+        int64_t best = used;
+        double gain = 0;
+        for (int64_t x = used; x < std::min(ready, used + wave);) {
+            x = std::min(ready, cost.step_end(x + 1));
+            const double v = (double)(x - used) * cost.full / (double)wave - (cost(x) - cost(used));
+            if (v >= gain) gain = v, best = x;
+        }
+        return best;
+    });
 }
 
 // Internal order (by level, bootstrapped gates before NOT/COPY in each level), descriptors and the
@@ -434,7 +492,7 @@ tfheb_status tfheb_netlist_create(tfheb_cloud_key *c, int32_t num_inputs, int32_
     cudaError_t e = cudaSetDevice(ck.device);
     for (int prec = 0; prec < 2 && e == cudaSuccess; prec++) {
         std::vector<int> lv(level);
-        pack_levels(num_inputs, num_gates, gates, in_a, in_b, in_c, nlev, wave_bootstraps(ck, prec), lv);
+        pack_levels(num_inputs, num_gates, gates, in_a, in_b, in_c, nlev, LevelCost(ck, prec, 1), lv);
         e = build_schedule(num_inputs, num_gates, gates, in_a, in_b, in_c, nlev, lv, nl->sched[prec]);
     }
     const tfheb_params &p = ck.p;
@@ -692,11 +750,9 @@ tfheb_status tfheb_netlist_multi_create(tfheb_cloud_key *const *cks, int32_t nke
     const size_t rows = (size_t)num_inputs + num_gates;
     cudaError_t e = cudaSuccess;
     for (int prec = 0; prec < 2 && e == cudaSuccess; prec++) {
-        // the levels are packed for the waves of all keys together
-        int wave = 0;
-        for (int k = 0; k < nkeys; k++) wave += wave_bootstraps(cks[k]->ck, prec);
+        // the levels are packed for the waves of all keys together (the keys' devices are alike)
         std::vector<int> lv(level);
-        pack_levels(num_inputs, num_gates, gates, in_a, in_b, in_c, nlev, wave, lv);
+        pack_levels(num_inputs, num_gates, gates, in_a, in_b, in_c, nlev, LevelCost(cks[0]->ck, prec, nkeys), lv);
         for (int k = 0; k < nkeys && e == cudaSuccess; k++) {
             e = cudaSetDevice(cks[k]->ck.device);
             if (e == cudaSuccess)
