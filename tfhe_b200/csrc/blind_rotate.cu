@@ -538,7 +538,6 @@ static const BrVariant kBrVariants[] = {
     {1024, 3, TFHEB_SPLIT_FP32, 6, 6, true, 10.50, launch_paired<1024, 3, 6, 6, 2, true>, 1},
     // one warp per bootstrap, exchanges in TMEM (blind_rotate_warp.cu; D counts 16 KB units): the split default
     {1024, 3, TFHEB_SPLIT_FP32, 8, 6, true, 10.94, launch_warp_split3, 1, 23},
-    {1024, 3, TFHEB_SPLIT_FP32, 2, 4, false, 5.84, launch_g<float, 1024, 3, true, 2, 4>},
     // the paired kernel with 3-6 teams, for waves of that many (3 and 4: for digits the warp kernel does not take)
     {1024, 3, TFHEB_SPLIT_FP32, 6, 12, false, 10.33, launch_paired_il3<1024, 3, 6, 12, 1>, 1},
     {1024, 3, TFHEB_SPLIT_FP32, 5, 12, false, 9.57, launch_paired_il3<1024, 3, 5, 12, 1>, 1},
@@ -549,8 +548,8 @@ static const BrVariant kBrVariants[] = {
     {1024, 3, TFHEB_SPLIT_FP32, 4, 6, false, 6.21, launch_warp_duo<true, 3, 4, 6>, 1, 23},
     {1024, 3, TFHEB_SPLIT_FP32, 3, 6, false, 6.14, launch_warp_duo<true, 3, 3, 6>, 1, 23},
     // few bootstraps (blind_rotate_latency.cu; D counts 48 KB stages): one per CTA, one per two CTAs
-    {1024, 3, TFHEB_SPLIT_FP32, 1, 2, false, 2.92, launch_latency<float, 3, 1, 1024>},
-    {1024, 3, TFHEB_SPLIT_FP32, 1, 2, false, 1.96, launch_latency<float, 3, 2, 1024>, 0, 32, 2},
+    {1024, 3, TFHEB_SPLIT_FP32, 1, 2, false, 2.65, launch_latency<float, 3, 1, 1024>},
+    {1024, 3, TFHEB_SPLIT_FP32, 1, 2, false, 1.81, launch_latency<float, 3, 2, 1024>, 0, 32, 2},
     {1024, 3, TFHEB_FP64, 4, 5, true, 9.85, launch_g<double, 1024, 3, false, 4, 5, false>},
     {1024, 3, TFHEB_FP64, 4, 4, true, 10.18, launch_g<double, 1024, 3, false, 4, 4, false>},
     {1024, 3, TFHEB_FP64, 4, 6, true, 11.18, launch_g<double, 1024, 3, false, 4, 6>},
@@ -575,8 +574,8 @@ static const BrVariant kBrVariants[] = {
     {2048, 3, TFHEB_SPLIT_FP32, 3, 3, true, 16.81, launch_g<float, 2048, 3, true, 3, 3>},
     {2048, 3, TFHEB_SPLIT_FP32, 2, 3, true, 11.56, launch_g<float, 2048, 3, true, 2, 3>},
     {2048, 3, TFHEB_SPLIT_FP32, 1, 3, false, 7.86, launch_g<float, 2048, 3, true, 1, 3>},
-    // one bootstrap on two SMs, D counting 16 KB rows: 3.46 ms per wave of 74, where the entry above takes 5.9
-    {2048, 3, TFHEB_SPLIT_FP32, 1, 5, false, 4.33, launch_latency<float, 3, 2, 2048>, 0, 32, 2},
+    // one bootstrap on two SMs, D counting 16 KB rows: 3.42 ms per wave of 74, where the entry above takes 5.9
+    {2048, 3, TFHEB_SPLIT_FP32, 1, 5, false, 4.28, launch_latency<float, 3, 2, 2048>, 0, 32, 2},
     {2048, 3, TFHEB_SPLIT_FP32, 2, 4, true, 12.86, launch_paired<2048, 3, 2, 4, 2, false>, 1},
     {2048, 3, TFHEB_SPLIT_FP32, 2, 4, true, 10.56, launch_paired<2048, 3, 2, 4, 2, true>, 1},
     // the warp kernel, D counting 32 KB units: 10.63 ms per wave of 592, against 10.19 ms per 444 for the first entry
@@ -592,13 +591,13 @@ static const BrVariant kBrVariants[] = {
     {1024, 2, TFHEB_SPLIT_FP32, 7, 4, true, 11.49, launch_g<float, 1024, 2, true, 7, 4>},
     {1024, 2, TFHEB_SPLIT_FP32, 8, 8, true, 8.60, launch_warp_split2<8>, 1, 23},
     {1024, 2, TFHEB_SPLIT_FP32, 4, 8, false, 4.82, launch_warp_split2<4>, 1, 23},
-    {1024, 2, TFHEB_SPLIT_FP32, 1, 2, false, 2.58, launch_latency<float, 2, 1, 1024>},
-    {1024, 2, TFHEB_SPLIT_FP32, 1, 2, false, 1.82, launch_latency<float, 2, 2, 1024>, 0, 32, 2},
+    {1024, 2, TFHEB_SPLIT_FP32, 1, 2, false, 2.37, launch_latency<float, 2, 1, 1024>},
+    {1024, 2, TFHEB_SPLIT_FP32, 1, 2, false, 1.70, launch_latency<float, 2, 2, 1024>, 0, 32, 2},
     {1024, 2, TFHEB_FP64, 4, 4, true, 7.90, launch_g<double, 1024, 2, false, 4, 4, false>},
     {1024, 2, TFHEB_FP64, 4, 4, true, 8.38, launch_g<double, 1024, 2, false, 4, 4>},
     {1024, 2, TFHEB_FP64, 8, 8, true, 11.66, launch_warp<false, 2, 8, 8>},
     {1024, 2, TFHEB_FP64, 4, 8, false, 6.35, launch_warp_duo<false, 2, 4, 8>},
-    {1024, 2, TFHEB_FP64, 1, 2, false, 2.98, launch_latency<double, 2, 1, 1024>},
+    {1024, 2, TFHEB_FP64, 1, 2, false, 2.74, launch_latency<double, 2, 1, 1024>},
     {1024, 2, TFHEB_FP64, 1, 1, false, 2.10, launch_latency<double, 2, 2, 1024>, 0, 32, 2},
 };
 
@@ -706,7 +705,7 @@ static int wave_need(int count, int sms) { return 2 * count <= sms ? 0 : (count 
 
 // The first wave's bootstraps of a rest of `count` (fewer than a wave of `big`): all of them, or as many whole
 // bootstraps per SM as give the least sum of measured times (*us) over the waves.  600 FP64 bootstraps run as
-// 592 + 8 (5.2 + 1.6 ms; 10.1 ms in one wave of eight per SM), 160 split ones as 148 + 12 (1.84 + 1.24 ms against
+// 592 + 8 (5.2 + 1.6 ms; 10.1 ms in one wave of eight per SM), 296 split ones as two of 148 (1.67 ms each, against
 // 3.68 two per SM).
 static int first_wave(const tfheb_params &p, int big, int count, int sms, const BrChoice &choice, float *us) {
     const int need = wave_need(count, sms);
@@ -734,7 +733,7 @@ float br_rest_us(const tfheb_params &p, int precision, const BrChoice &choice, i
 
 // Full waves of the chosen variant (SMs x G bootstraps each), then the rest in waves of whatever runs that many
 // per CTA fastest: 4096 split bootstraps are 3 waves of 1184 and 544 spread over 4 per CTA (20.7 + 3.9 ms,
-// where a fourth packed wave takes 6.9).  A lone bootstrap runs its 630 steps in 1.24 ms on two SMs, 1.84 ms
+// where a fourth packed wave takes 6.9).  A lone bootstrap runs its 630 steps in 1.14 ms on two SMs, 1.67 ms
 // on one.
 cudaError_t launch_blind_rotate(const tfheb_params &p, int precision, const DeviceBsk &bsk, const int32_t *bara,
                                 int bara_stride, int boots, int nsteps, int32_t mu, const int32_t *acc_in,

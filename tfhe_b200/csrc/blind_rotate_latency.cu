@@ -1,6 +1,6 @@
 // blind_rotate_latency.cu -- the blind rotation of few bootstraps (tfhe_blindRotate_FFT,
 // lwe-bootstrapping-functions-fft.cpp:88-112): one bootstrap per CTA, or per cluster of two CTAs; N = 1024, and the
-// split form at N = 2048 on two CTAs (3.46 ms per wave of 74, against 5.9 ms for one team of blind_rotate_kernel).
+// split form at N = 2048 on two CTAs (3.42 ms per wave of 74, against 5.9 ms for one team of blind_rotate_kernel).
 //
 // A batch far below one wave (a single drop-in gate, a few dozen concurrent callers) waits for one bootstrap's
 // serial chain of n steps, so a step is spread over as many warps as it has independent work:
@@ -10,7 +10,11 @@
 //      packed pair in the split form) over the digits in order.  Its keys are in registers before the
 //      spectra are there: their shared-memory reads (two thirds of the phase's) are off the chain;
 //   4. one team per (output polynomial, key limb) runs an inverse transform and adds its rounded words to
-//      an accumulator of its own (integer sums mod 2^32: the rotation reads the sum of the two limbs').
+//      the accumulator, the two limbs' teams by shared-memory atomics (integer sums mod 2^32, in any order).
+// A thread's twiddles stay in registers where there is room (N = 1024 split, and FP64 at l = 2 on one CTA).  These two
+// steps took a wave of 148 from 1.84 to 1.67 ms, one of 74 from 1.23 to 1.14 (split, l = 3): the shared-memory pipe is
+// busy three quarters of a step.  Slower: the rotation by each team for itself instead of once (1.24 ms of 1.14),
+// warps of their own for the multiply-accumulate (1.35).
 // With C = 2 a cluster shares the bootstrap: CTA v keeps polynomial v of the accumulator, transforms its l digits
 // and computes output v, so the only thing the two exchange is the spectra, once a step: each team also
 // stores its spectrum into the other CTA's shared memory with st.async, which counts the bytes on the other
@@ -56,6 +60,8 @@ struct LatencyLayout {
     // registers before the spectra have arrived
     static constexpr int stage_digits = big ? 1 : C == 2 ? KPL : L, early = big || C == 1 ? L : KPL;
     static constexpr int D = big ? 5 : !split && C == 2 ? 1 : 2;  // FP64 needs the room; a step outlasts a refill
+    // stages whose twiddles a thread keeps (more spilled, and ran slower: FP64 at l = 3 2.89 against 2.32 ms)
+    static constexpr int own_stages = big ? 0 : split || (C == 1 && L == 2) ? 2 : 0;
     static constexpr uint32_t stage = (uint32_t)stage_digits * polys * half;
     static constexpr size_t spec_bytes = sizeof(cplx<T>) * M;  // one digit's spectrum
     static constexpr size_t bars = 0;  // full[D], empty[D], remote[2], abort flag, stop
@@ -63,8 +69,7 @@ struct LatencyLayout {
     static constexpr size_t tables = ring + D * (size_t)stage;
     static constexpr size_t acc = (tables + tw_table_bytes<T, M>() + 127) / 128 * 128;
     static constexpr size_t acc_bytes = 4 * (size_t)polys * N;
-    static constexpr size_t acc_low = acc + acc_bytes;                             // split: the low limb's sums
-    static constexpr size_t rot = acc_low + (split ? acc_bytes : 0);               // this step's rotated words
+    static constexpr size_t rot = acc + acc_bytes;                                 // this step's rotated words
     static constexpr size_t spec = rot + acc_bytes;                                // [team] own digits
     static constexpr size_t spec_in = spec + fwd_teams * spec_bytes;               // [parity][digit] the other CTA's
     static constexpr size_t after_spec = spec_in + (C == 2 ? 2 * L * spec_bytes : 0);
@@ -217,7 +222,6 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
     } else {  // ---- consumer warps ----
         const int tid = threadIdx.x, team = warp / Lay::team_warps, t = tid & (NT - 1);
         uint32_t *s_acc = reinterpret_cast<uint32_t *>(smem + Lay::acc);
-        uint32_t *s_low = reinterpret_cast<uint32_t *>(smem + Lay::acc_low);  // split: acc = s_acc + s_low
         uint32_t *s_rot = reinterpret_cast<uint32_t *>(smem + Lay::rot);
         const cplx<T> *s_tw = reinterpret_cast<const cplx<T> *>(smem + Lay::tables);
         ExchPair xp{smem + Lay::xbufs + (size_t)(team < Lay::teams ? team : 0) * Lay::xbufs_of * Lay::xbuf_bytes,
@@ -243,8 +247,6 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
                 s_acc[i] = !last ? 0u : neg ? 0u - (uint32_t)args.mu : (uint32_t)args.mu;
             }
         }
-        if constexpr (SPLIT)
-            for (int i = tid; i < Lay::polys * N; i += consumers) s_low[i] = 0u;
         team_sync(kAllBar, consumers);
 
         // gadget constants (tgsw.cpp:7-29)
@@ -267,6 +269,8 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
             far_bar = cluster_addr(remote_bar(0), (uint32_t)(rank ^ 1));
         }
 
+        const typename F::template OwnTwiddles<Lay::own_stages> own_tw(s_tw, t);
+
         int a_next = args.nsteps > 0 ? my_bara[0] : 0;
         bool aborted = false;
         for (int step = 0; step < args.nsteps && !aborted; step++) {
@@ -285,8 +289,7 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
                 if (Lay::polys * N % consumers != 0 && i >= Lay::polys * N) break;
                 const int e = (i & (N - 1)) - ai, src = (i & ~(N - 1)) + (e & (N - 1));
                 const uint32_t neg = (uint32_t)((int32_t)((uint32_t)e << (N == 2048 ? 20 : 21)) >> 31), on = offset - neg;
-                const uint32_t x = SPLIT ? s_acc[src] + s_low[src] : s_acc[src];
-                const uint32_t y = SPLIT ? s_acc[i] + s_low[i] : s_acc[i];
+                const uint32_t x = s_acc[src], y = s_acc[i];
                 s_rot[i] = (x ^ neg) + (on - y);
             }
             team_sync(kAllBar, consumers);
@@ -301,7 +304,7 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
                     const T d1 = DigitConv<T>::conv((w[NT * r + M] >> shift) & maskBg, digit_bias);
                     z[r] = cplx<T>{d0, -d1};  // a_j - i a_{j+M}; the twist is folded into the FFT
                 }
-                F::forward(z, xp, s_tw, t, 1 + team);
+                F::forward(z, xp, own_tw, t, 1 + team);
                 const uint32_t far = far_spec + (uint32_t)(parity * L * Lay::spec_bytes);
                 const uint32_t bar = far_bar + 8u * (uint32_t)parity;
                 if constexpr (SPLIT) {
@@ -457,23 +460,23 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
                         z[2 * i] = {w.x, w.y};
                         z[2 * i + 1] = {w.z, w.w};
                     }
-                    F::inverse(z, xp, s_tw, t, 1 + team);
+                    F::inverse(z, xp, own_tw, t, 1 + team);
                     // (c_j - i c_{j+M}) of this limb.  Where no low-limb sum can reach 2^44 it is rounded like the
                     // high limb's, on the FMA pipe (the same integer; the conversion instruction takes longer)
                     if ((team & 1) && !low_small) {
-                        uint32_t *poly = s_low + (team >> 1) * N + t;
+                        uint32_t *poly = s_acc + (team >> 1) * N + t;
 #pragma unroll
                         for (int r = 0; r < kR; r++) {
-                            poly[NT * r] += (uint32_t)__float2ll_rn(z[r].re);
-                            poly[NT * r + M] += (uint32_t)__float2ll_rn(-z[r].im);
+                            atomicAdd(poly + NT * r, (uint32_t)__float2ll_rn(z[r].re));
+                            atomicAdd(poly + NT * r + M, (uint32_t)__float2ll_rn(-z[r].im));
                         }
                     } else {
-                        uint32_t *poly = (team & 1 ? s_low : s_acc) + (team >> 1) * N + t;
+                        uint32_t *poly = s_acc + (team >> 1) * N + t;
                         const int weight = team & 1 ? 0 : args.split_shift;
 #pragma unroll
                         for (int r = 0; r < kR; r++) {
-                            poly[NT * r] += round_f32_mod32(z[r].re) << weight;
-                            poly[NT * r + M] += round_f32_mod32(-z[r].im) << weight;
+                            atomicAdd(poly + NT * r, round_f32_mod32(z[r].re) << weight);
+                            atomicAdd(poly + NT * r + M, round_f32_mod32(-z[r].im) << weight);
                         }
                     }
                 } else {
@@ -482,7 +485,7 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
                         const double2 w = reinterpret_cast<const double2 *>(in)[r * NT + t];
                         z[r] = {(T)w.x, (T)w.y};
                     }
-                    F::inverse(z, xp, s_tw, t, 1 + team);
+                    F::inverse(z, xp, own_tw, t, 1 + team);
                     uint32_t *poly = s_acc + team * N + t;
 #pragma unroll
                     for (int r = 0; r < kR; r++) {
@@ -496,7 +499,7 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
         }
 
         uint32_t *dst = reinterpret_cast<uint32_t *>(args.acc_out) + ((size_t)boot * KP1 + rank) * N;
-        for (int i = tid; i < Lay::polys * N; i += consumers) dst[i] = s_acc[i] + (SPLIT ? s_low[i] : 0u);
+        for (int i = tid; i < Lay::polys * N; i += consumers) dst[i] = s_acc[i];
         if (C == 2 && aborted) __nanosleep(20000);  // stores to the other CTA may still be on their way
         __syncwarp();
     }

@@ -452,6 +452,41 @@ struct TeamFft {
         }
     }
 
+    // A thread's own factors of the first KEEP stages, kept in registers from transform to transform.
+    template <int KEEP>
+    struct OwnTwiddles {
+        const cplx<T> *table;
+        cplx<T> w[KEEP > 0 ? KEEP : 1][R];
+        __device__ __forceinline__ OwnTwiddles(const cplx<T> *tw, int t) : table(tw) { load<0>(tw, t); }
+        template <int S>
+        __device__ __forceinline__ void load(const cplx<T> *tw, int t) {
+            constexpr int r = Stage<M, S>::r, st = Stage<M, S>::stride;
+            if constexpr (S < KEEP && (S == 0 || st > 1)) {
+#pragma unroll
+                for (int i = 0; i < R; i++) {
+                    const int k2 = i % r, n1 = S == 0 ? t : (t + NT * (i / r)) % st;
+                    if (S > 0 && k2 == 0) continue;
+                    if constexpr (sizeof(T) == 4) {
+                        const int k = S == 0 ? k2 : k2 - 1;
+                        w[S][i] = tw[2 * (tw4_offset<M>(S) + k / 2 * st + n1) + k % 2];
+                    } else {
+                        w[S][i] = tw[tw_offset<M>(S) + (S == 0 ? k2 : k2 - 1) * st + n1];
+                    }
+                }
+            }
+            if constexpr (S + 1 < KEEP) load<S + 1>(tw, t);
+        }
+    };
+    template <int S, bool INV, int KEEP>
+    __device__ static __forceinline__ void twiddle(cplx<T> *x, const OwnTwiddles<KEEP> &tw, int t) {
+        if constexpr (S >= KEEP) twiddle<S, INV>(x, tw.table, t);
+        else if constexpr (S == 0 || Stage<M, S>::stride > 1) {
+#pragma unroll
+            for (int i = 0; i < R; i++)
+                if (S == 0 || i % Stage<M, S>::r != 0) x[i] = INV ? cmulconj(x[i], tw.w[S][i]) : cmul(x[i], tw.w[S][i]);
+        }
+    }
+
     // x[n] *= exp(-+ i pi n / 16)
     template <bool INV>
     __device__ static __forceinline__ void fold_consts(cplx<T> *x) {
@@ -462,8 +497,8 @@ struct TeamFft {
         }
     }
 
-    template <int S>
-    __device__ static __forceinline__ void forward_from(cplx<T> *x, ExchPair &xp, const cplx<T> *tw, int t, int bar_id) {
+    template <int S, typename TW>
+    __device__ static __forceinline__ void forward_from(cplx<T> *x, ExchPair &xp, const TW &tw, int t, int bar_id) {
         constexpr int r = Stage<M, S>::r;
 #pragma unroll
         for (int c = 0; c < R / r; c++) dft<T, false, r>(x + c * r);
@@ -478,8 +513,8 @@ struct TeamFft {
         }
     }
 
-    template <int S>
-    __device__ static __forceinline__ void inverse_from(cplx<T> *x, ExchPair &xp, const cplx<T> *tw, int t, int bar_id) {
+    template <int S, typename TW>
+    __device__ static __forceinline__ void inverse_from(cplx<T> *x, ExchPair &xp, const TW &tw, int t, int bar_id) {
         constexpr int r = Stage<M, S>::r;
         twiddle<S, true>(x, tw, t);
 #pragma unroll
@@ -565,12 +600,14 @@ struct TeamFft {
 
     // Folded negacyclic transform.  In: x[n2] = a_j - i a_{j+M} for j = t + NT*n2 (no twist applied).
     // Out: the M evaluation points in slot order.
-    __device__ static __forceinline__ void forward(cplx<T> *x, ExchPair &xp, const cplx<T> *tw, int t, int bar_id) {
+    template <typename TW>  // the table, or a thread's OwnTwiddles
+    __device__ static __forceinline__ void forward(cplx<T> *x, ExchPair &xp, const TW &tw, int t, int bar_id) {
         fold_consts<false>(x);
         forward_from<0>(x, xp, tw, t, bar_id);
     }
     // Slot order in -> x[n2] = M * (c_j - i c_{j+M}), j = t + NT*n2 (twist removed).
-    __device__ static __forceinline__ void inverse(cplx<T> *x, ExchPair &xp, const cplx<T> *tw, int t, int bar_id) {
+    template <typename TW>  // the table, or a thread's OwnTwiddles
+    __device__ static __forceinline__ void inverse(cplx<T> *x, ExchPair &xp, const TW &tw, int t, int bar_id) {
         inverse_from<NS - 1>(x, xp, tw, t, bar_id);
         fold_consts<true>(x);
     }

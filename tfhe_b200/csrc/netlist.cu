@@ -251,9 +251,9 @@ struct LevelCost {
 // bootstrap) go on the first level where they are ready.
 // The cap is the end of the waves that the mandatory gates start, waves being counted in the variant's, in half of
 // them, in SMs or in half SMs; or it is where topping up pays most, at a full wave's cost per bootstrap.  No one of
-// them is best throughout, so each is tried and the assignment with the least sum of costs taken.  Measured, split
-// form: ten levels of 75 to 1200 gates 42.6 ms (by half waves; 52.1 by whole ones), six of 18 to 300 11.2 (by SMs;
-// 13.1 by the costs), eight of 6 to 100 10.1 (by half SMs; 11.9).  Creation takes 3.7 instead of 2.4 ms for 5775 gates.
+// them is best throughout, so each is tried and the assignment with the least sum of costs taken.  Split form: ten
+// levels of 75 to 1200 gates 42.6 ms (by half waves; 52.1 by whole ones), six of 18 to 300 11.2 (by SMs; 12.9 by its
+// costs), eight of 6 to 100 10.1 (by half SMs; 11.7 by its costs).  Creation takes 3.7 instead of 2.4 ms for 5775 gates.
 void pack_levels(int num_inputs, int num_gates, const int32_t *gates, const int32_t *in_a, const int32_t *in_b,
                  const int32_t *in_c, int nlev, const LevelCost &cost, std::vector<int> &level) {
     if (num_gates == 0 || cost.wave * cost.shards <= 1) return;
