@@ -556,7 +556,7 @@ static const BrVariant kBrVariants[] = {
     {1024, 3, TFHEB_FP64, 4, 4, true, 11.04, launch_g<double, 1024, 3, false, 4, 4>},
     {1024, 3, TFHEB_FP64, 3, 4, true, 8.58, launch_g<double, 1024, 3, false, 3, 4>},
     {1024, 3, TFHEB_FP64, 2, 4, true, 5.86, launch_g<double, 1024, 3, false, 2, 4>},
-    {1024, 3, TFHEB_FP64, 8, 6, true, 16.08, launch_warp<false, 3, 8, 6>},
+    {1024, 3, TFHEB_FP64, 8, 6, true, 15.75, launch_warp<false, 3, 8, 6>},
     {1024, 3, TFHEB_FP64, 4, 6, false, 8.32, launch_warp_duo<false, 3, 4, 6>},
     {1024, 3, TFHEB_FP64, 3, 6, false, 8.34, launch_warp_duo<false, 3, 3, 6>},
     {1024, 3, TFHEB_FP64, 1, 2, false, 3.67, launch_latency<double, 3, 1, 1024>},
