@@ -559,8 +559,8 @@ static const BrVariant kBrVariants[] = {
     {1024, 3, TFHEB_FP64, 8, 6, true, 15.75, launch_warp<false, 3, 8, 6>},
     {1024, 3, TFHEB_FP64, 4, 6, false, 8.32, launch_warp_duo<false, 3, 4, 6>},
     {1024, 3, TFHEB_FP64, 3, 6, false, 8.34, launch_warp_duo<false, 3, 3, 6>},
-    {1024, 3, TFHEB_FP64, 1, 2, false, 3.67, launch_latency<double, 3, 1, 1024>},
-    {1024, 3, TFHEB_FP64, 1, 1, false, 2.47, launch_latency<double, 3, 2, 1024>, 0, 32, 2},
+    {1024, 3, TFHEB_FP64, 1, 2, false, 3.34, launch_latency<double, 3, 1, 1024>},
+    {1024, 3, TFHEB_FP64, 1, 1, false, 2.35, launch_latency<double, 3, 2, 1024>, 0, 32, 2},
     // the split default at N = 2048: the N = 1024 default's structure with three teams and a 6-deep
     // ring of 16 KB half rows (51.3 ms per 2048 bootstraps; 51.7 ms with output 0's inverse input in
     // registers, 51.9 ms forward interleave only, 53.1 ms no interleave, 54.1 ms rotated words in
@@ -574,8 +574,8 @@ static const BrVariant kBrVariants[] = {
     {2048, 3, TFHEB_SPLIT_FP32, 3, 3, true, 16.81, launch_g<float, 2048, 3, true, 3, 3>},
     {2048, 3, TFHEB_SPLIT_FP32, 2, 3, true, 11.56, launch_g<float, 2048, 3, true, 2, 3>},
     {2048, 3, TFHEB_SPLIT_FP32, 1, 3, false, 7.86, launch_g<float, 2048, 3, true, 1, 3>},
-    // one bootstrap on two SMs, D counting 16 KB rows: 3.42 ms per wave of 74, where the entry above takes 5.9
-    {2048, 3, TFHEB_SPLIT_FP32, 1, 5, false, 4.28, launch_latency<float, 3, 2, 2048>, 0, 32, 2},
+    // one bootstrap on two SMs, D counting 16 KB rows: 3.16 ms per wave of 74, where the entry above takes 5.9
+    {2048, 3, TFHEB_SPLIT_FP32, 1, 5, false, 3.95, launch_latency<float, 3, 2, 2048>, 0, 32, 2},
     {2048, 3, TFHEB_SPLIT_FP32, 2, 4, true, 12.86, launch_paired<2048, 3, 2, 4, 2, false>, 1},
     {2048, 3, TFHEB_SPLIT_FP32, 2, 4, true, 10.56, launch_paired<2048, 3, 2, 4, 2, true>, 1},
     // the warp kernel, D counting 32 KB units: 10.63 ms per wave of 592, against 10.19 ms per 444 for the first entry
@@ -591,14 +591,14 @@ static const BrVariant kBrVariants[] = {
     {1024, 2, TFHEB_SPLIT_FP32, 7, 4, true, 11.49, launch_g<float, 1024, 2, true, 7, 4>},
     {1024, 2, TFHEB_SPLIT_FP32, 8, 8, true, 8.60, launch_warp_split2<8>, 1, 23},
     {1024, 2, TFHEB_SPLIT_FP32, 4, 8, false, 4.82, launch_warp_split2<4>, 1, 23},
-    {1024, 2, TFHEB_SPLIT_FP32, 1, 2, false, 2.37, launch_latency<float, 2, 1, 1024>},
-    {1024, 2, TFHEB_SPLIT_FP32, 1, 2, false, 1.70, launch_latency<float, 2, 2, 1024>, 0, 32, 2},
+    {1024, 2, TFHEB_SPLIT_FP32, 1, 2, false, 2.33, launch_latency<float, 2, 1, 1024>},
+    {1024, 2, TFHEB_SPLIT_FP32, 1, 2, false, 1.67, launch_latency<float, 2, 2, 1024>, 0, 32, 2},
     {1024, 2, TFHEB_FP64, 4, 4, true, 7.90, launch_g<double, 1024, 2, false, 4, 4, false>},
     {1024, 2, TFHEB_FP64, 4, 4, true, 8.38, launch_g<double, 1024, 2, false, 4, 4>},
     {1024, 2, TFHEB_FP64, 8, 8, true, 11.66, launch_warp<false, 2, 8, 8>},
     {1024, 2, TFHEB_FP64, 4, 8, false, 6.35, launch_warp_duo<false, 2, 4, 8>},
     {1024, 2, TFHEB_FP64, 1, 2, false, 2.74, launch_latency<double, 2, 1, 1024>},
-    {1024, 2, TFHEB_FP64, 1, 1, false, 2.10, launch_latency<double, 2, 2, 1024>, 0, 32, 2},
+    {1024, 2, TFHEB_FP64, 1, 1, false, 2.04, launch_latency<double, 2, 2, 1024>, 0, 32, 2},
 };
 
 int br_variants(int N, int l, int precision, int *G, int *D, int cap) {
@@ -705,7 +705,7 @@ static int wave_need(int count, int sms) { return 2 * count <= sms ? 0 : (count 
 
 // The first wave's bootstraps of a rest of `count` (fewer than a wave of `big`): all of them, or as many whole
 // bootstraps per SM as give the least sum of measured times (*us) over the waves.  600 FP64 bootstraps run as
-// 592 + 8 (5.2 + 1.6 ms; 10.1 ms in one wave of eight per SM), 296 split ones as two of 148 (1.67 ms each, against
+// 592 + 8 (5.2 + 1.5 ms; 9.9 ms in one wave of eight per SM), 296 split ones as two of 148 (1.67 ms each, against
 // 3.68 two per SM).
 static int first_wave(const tfheb_params &p, int big, int count, int sms, const BrChoice &choice, float *us) {
     const int need = wave_need(count, sms);

@@ -1,6 +1,6 @@
 // blind_rotate_latency.cu -- the blind rotation of few bootstraps (tfhe_blindRotate_FFT,
 // lwe-bootstrapping-functions-fft.cpp:88-112): one bootstrap per CTA, or per cluster of two CTAs; N = 1024, and the
-// split form at N = 2048 on two CTAs (3.42 ms per wave of 74, against 5.9 ms for one team of blind_rotate_kernel).
+// split form at N = 2048 on two CTAs (3.16 ms per wave of 74, against 5.9 ms for one team of blind_rotate_kernel).
 //
 // A batch far below one wave (a single drop-in gate, a few dozen concurrent callers) waits for one bootstrap's
 // serial chain of n steps, so a step is spread over as many warps as it has independent work:
@@ -11,9 +11,8 @@
 //      spectra are there: their shared-memory reads (two thirds of the phase's) are off the chain;
 //   4. one team per (output polynomial, key limb) runs an inverse transform and adds its rounded words to
 //      the accumulator, the two limbs' teams by shared-memory atomics (integer sums mod 2^32, in any order).
-// A thread's twiddles stay in registers where there is room (N = 1024 split, and FP64 at l = 2 on one CTA).  These two
-// steps took a wave of 148 from 1.84 to 1.67 ms, one of 74 from 1.23 to 1.14 (split, l = 3): the shared-memory pipe is
-// busy three quarters of a step.  Slower: the rotation by each team for itself instead of once (1.24 ms of 1.14),
+// A thread's twiddles stay in registers.  These two steps took a wave of 148 from 1.84 to 1.67 ms, one of 74 from 1.23
+// to 1.14 (split, l = 3): the shared-memory pipe is busy three quarters of a step.  Slower: the rotation by each team for itself instead of once (1.24 ms of 1.14),
 // warps of their own for the multiply-accumulate (1.35).
 // With C = 2 a cluster shares the bootstrap: CTA v keeps polynomial v of the accumulator, transforms its l digits
 // and computes output v, so the only thing the two exchange is the spectra, once a step: each team also
@@ -54,14 +53,18 @@ struct LatencyLayout {
     static constexpr int mac_warps = 8, pairs = 4 * NT / (32 * mac_warps);  // slot pairs of a thread per output
     static constexpr int team_warps = NT / 32;
     static constexpr int warps = team_warps * fwd_teams > mac_warps ? team_warps * fwd_teams : mac_warps;
-    static constexpr int threads = 32 * (warps + 1);
+    // whole warpgroups, for more registers in the consumers': 232 in two of three, 160 in three of four.  With the
+    // twiddles in them: FP64, l = 3 2.32 -> 2.11 (C = 1) and 1.55 -> 1.48 ms (C = 2), N = 2048 3.42 -> 3.16.  Split, l = 3,
+    // C = 1 has room without and ran slower (1.77 against 1.67 ms).
+    static constexpr bool wide = big || (!split && (C == 2 || L == 3));
+    static constexpr int threads = wide ? 32 * (warps + 4) : 32 * (warps + 1), wide_regs = warps == 8 ? 232 : 160;
     static constexpr uint32_t half = (uint32_t)M * 16;    // one output's slots of one key row
     // ring: D stages of stage_digits digits' rows of the CTA's outputs; the first `early` digits' keys of a step go to
     // registers before the spectra have arrived
     static constexpr int stage_digits = big ? 1 : C == 2 ? KPL : L, early = big || C == 1 ? L : KPL;
     static constexpr int D = big ? 5 : !split && C == 2 ? 1 : 2;  // FP64 needs the room; a step outlasts a refill
-    // stages whose twiddles a thread keeps (more spilled, and ran slower: FP64 at l = 3 2.89 against 2.32 ms)
-    static constexpr int own_stages = big ? 0 : split || (C == 1 && L == 2) ? 2 : 0;
+    // stages whose twiddles a thread keeps (a last stage of radix 8 has none)
+    static constexpr int own_stages = big ? 3 : 2;
     static constexpr uint32_t stage = (uint32_t)stage_digits * polys * half;
     static constexpr size_t spec_bytes = sizeof(cplx<T>) * M;  // one digit's spectrum
     static constexpr size_t bars = 0;  // full[D], empty[D], remote[2], abort flag, stop
@@ -92,6 +95,7 @@ struct LatencyLayout {
     static constexpr size_t bytes = xbufs + (size_t)teams * xbufs_of * xbuf_bytes;
     static_assert((2 * D + 2) * 8 + 8 <= ring, "barrier block");
     static_assert(bytes <= 227 * 1024, "shared memory of the variant");
+    static_assert(!wide || warps == 8 || warps == 12, "register split");
     static_assert(team_warps * inv_teams <= warps && KPL % stage_digits == 0, "every inverse transform has a team");
     // place (in float4) of slots 2c, 2c + 1 of thread t in a spectrum.  N = 2048: the multiply-accumulate follows the
     // key's second layout (key_transform.cu), whose lanes hold t's 8 apart; the low three bits are XORed so that
@@ -194,8 +198,9 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
     __syncthreads();
     if constexpr (C == 2) cluster_sync();  // both CTAs' barriers exist before either signals
 
-    if (warp == Lay::warps) {  // ---- the key's stream ----
-        if (lane == 0) {
+    if (Lay::wide ? warp >= Lay::warps : warp == Lay::warps) {  // ---- the key's stream ----
+        if constexpr (Lay::wide) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Lay::wide_regs == 232 ? 40 : 32));
+        if (lane == 0 && (!Lay::wide || warp == Lay::warps)) {
             const uint8_t *bsk = SPLIT ? args.bsk2 : args.bsk;
             const int total = args.nsteps * (KPL / Lay::stage_digits);
             int sent = 0;
@@ -220,6 +225,10 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
         }
         __syncwarp();
     } else {  // ---- consumer warps ----
+        if constexpr (Lay::wide) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Lay::wide_regs));
+        // spares the test whether a warp has a transform; at l = 3, N = 1024 the compiler then reads the keys later
+        // (1.69 against 1.67 ms), elsewhere it is faster (N = 2048 6.6 against 6.8 ms per 148, l = 2 1.17 against 1.19)
+        if constexpr (Lay::big || (SPLIT && L == 2)) __builtin_assume(warp < Lay::warps);
         const int tid = threadIdx.x, team = warp / Lay::team_warps, t = tid & (NT - 1);
         uint32_t *s_acc = reinterpret_cast<uint32_t *>(smem + Lay::acc);
         uint32_t *s_rot = reinterpret_cast<uint32_t *>(smem + Lay::rot);
