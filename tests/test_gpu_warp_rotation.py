@@ -102,18 +102,19 @@ def test_few_bootstraps_equal_a_packed_wave(keys, l, Bgbit, precision, nsteps, c
     ck.set_br_variant(precision, 0)
 
 
-# N = 2048: one bootstrap on two SMs (at most 74 of 148); a step takes six rows through a ring of five
-@pytest.mark.parametrize("count", [1, 2, 73, 74, 75])
+# N = 2048: one bootstrap on two SMs (at most 74 of 148); a step takes six rows through a ring of five, or three
+@pytest.mark.parametrize("count", [1, 2, 73, 74, 75, 148])
 @pytest.mark.parametrize("nsteps", [1, 2, 5, 9])
-def test_large_ring_few_bootstraps_equal_a_packed_wave(large_keys, nsteps, count):
+@pytest.mark.parametrize("precision", [tb.FP64, tb.SPLIT_FP32])
+def test_large_ring_few_bootstraps_equal_a_packed_wave(large_keys, precision, nsteps, count):
     sk, ck = large_keys
     rng = np.random.default_rng(7 * count + nsteps)
     acc = rng.integers(-2**31, 2**31, (592, 2, 2048)).astype(np.int32)
     bara = rng.integers(0, 4096, (592, nsteps)).astype(np.int32)
     bara.flat[:5] = [0, 1, 2047, 2048, 4095]
-    four = int(np.flatnonzero(ck.br_variants(tb.SPLIT_FP32)[0] == 4)[0])
-    want = rotate(ck, tb.SPLIT_FP32, four, bara, acc, nsteps)
-    assert (rotate(ck, tb.SPLIT_FP32, four, bara[:count], acc[:count], nsteps) == want[:count]).all()
+    four = int(np.flatnonzero(ck.br_variants(precision)[0] == 4)[0])
+    want = rotate(ck, precision, four, bara, acc, nsteps)
+    assert (rotate(ck, precision, four, bara[:count], acc[:count], nsteps) == want[:count]).all()
 
 
 # around the waves' ends: all of the last wave's choices, and a last CTA with one of eight warps at work
@@ -152,14 +153,15 @@ def test_stalled_key_stream(keys, precision, count):
     ck.set_br_variant(precision, 0)
 
 
-def test_stalled_key_stream_large_ring(large_keys):
+@pytest.mark.parametrize("precision", [tb.FP64, tb.SPLIT_FP32])
+def test_stalled_key_stream_large_ring(large_keys, precision):
     sk, ck = large_keys
     bara, acc = np.zeros((3, 2), np.int32), np.zeros((3, 2, 2048), np.int32)
     ck.set_wait_timeout(0.05)
     ck.test_stall_key_stream(True)
     with pytest.raises(tb.api.TfhebError) as exc:
-        rotate(ck, tb.SPLIT_FP32, 0, bara, acc, 2)
+        rotate(ck, precision, 0, bara, acc, 2)
     assert exc.value.status == tb.api.TIMEOUT
     ck.test_stall_key_stream(False)
     ck.set_wait_timeout(1.0)
-    rotate(ck, tb.SPLIT_FP32, 0, bara, acc, 2)
+    rotate(ck, precision, 0, bara, acc, 2)

@@ -574,17 +574,19 @@ static const BrVariant kBrVariants[] = {
     {2048, 3, TFHEB_SPLIT_FP32, 3, 3, true, 16.81, launch_g<float, 2048, 3, true, 3, 3>},
     {2048, 3, TFHEB_SPLIT_FP32, 2, 3, true, 11.56, launch_g<float, 2048, 3, true, 2, 3>},
     {2048, 3, TFHEB_SPLIT_FP32, 1, 3, false, 7.86, launch_g<float, 2048, 3, true, 1, 3>},
-    // one bootstrap on two SMs, D counting 16 KB rows: 3.16 ms per wave of 74, where the entry above takes 5.9
-    {2048, 3, TFHEB_SPLIT_FP32, 1, 5, false, 3.95, launch_latency<float, 3, 2, 2048>, 0, 32, 2},
+    // one bootstrap on two SMs, D counting 16 KB rows: 3.04 ms per wave of 74, where the entry above takes 5.9 (and two
+    // of them 6.09 for 148, against its 6.29)
+    {2048, 3, TFHEB_SPLIT_FP32, 1, 5, false, 3.80, launch_latency<float, 3, 2, 2048>, 0, 32, 2},
     {2048, 3, TFHEB_SPLIT_FP32, 2, 4, true, 12.86, launch_paired<2048, 3, 2, 4, 2, false>, 1},
     {2048, 3, TFHEB_SPLIT_FP32, 2, 4, true, 10.56, launch_paired<2048, 3, 2, 4, 2, true>, 1},
     // the warp kernel, D counting 32 KB units: 10.63 ms per wave of 592, against 10.19 ms per 444 for the first entry
     {2048, 3, TFHEB_SPLIT_FP32, 4, 3, true, 13.28, launch_warp_big<true, 3, 4>, 1},
-    // FP64: the last entry is the default (14.86 ms per wave of 592, against 10.35 ms per 296 for the first)
+    // FP64: the entry with G = 4 is the default (14.86 ms per wave of 592, against 10.35 ms per 296 for the first)
     {2048, 3, TFHEB_FP64, 2, 3, true, 12.94, launch_g<double, 2048, 3, false, 2, 3, false>},
     {2048, 3, TFHEB_FP64, 2, 3, true, 14.37, launch_g<double, 2048, 3, false, 2, 3>},
     {2048, 3, TFHEB_FP64, 1, 4, true, 7.66, launch_g<double, 2048, 3, false, 1, 4>},
     {2048, 3, TFHEB_FP64, 4, 3, true, 18.58, launch_warp_big<false, 3, 4>},
+    {2048, 3, TFHEB_FP64, 1, 3, false, 5.90, launch_latency<double, 3, 2, 2048>, 0, 32, 2},  // 4.72 ms; 5.9 with G = 1 above
     {512, 3, TFHEB_SPLIT_FP32, 8, 4, true, 0, launch_g<float, 512, 3, true, 8, 4>},
     {512, 3, TFHEB_FP64, 8, 4, true, 0, launch_g<double, 512, 3, false, 8, 4>},
     // the 80-bit parameter set (n = 500, l = 2, Bgbit = 10; tfhe_gate_bootstrapping.cpp:23-48)
@@ -711,6 +713,13 @@ static int first_wave(const tfheb_params &p, int big, int count, int sms, const 
     const int need = wave_need(count, sms);
     int first = count;
     *us = kBrVariants[wave_variant(p, big, need, choice)].us;
+    if (need == 1 && count <= sms / 2 * 2) {  // or two waves on two SMs per bootstrap (N = 2048 split: 6.09 against 6.29 ms)
+        const float t = 2 * kBrVariants[wave_variant(p, big, 0, choice)].us;
+        if (t > 0 && t < *us) {
+            *us = t;
+            first = sms / 2;
+        }
+    }
     for (int a = 1; a < need && *us > 0; a++) {
         const float ta = kBrVariants[wave_variant(p, big, a, choice)].us;
         float rest = 0;

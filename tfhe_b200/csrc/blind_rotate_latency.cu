@@ -1,6 +1,6 @@
 // blind_rotate_latency.cu -- the blind rotation of few bootstraps (tfhe_blindRotate_FFT,
-// lwe-bootstrapping-functions-fft.cpp:88-112): one bootstrap per CTA, or per cluster of two CTAs; N = 1024, and the
-// split form at N = 2048 on two CTAs (3.16 ms per wave of 74, against 5.9 ms for one team of blind_rotate_kernel).
+// lwe-bootstrapping-functions-fft.cpp:88-112): one bootstrap per CTA, or per cluster of two CTAs; N = 1024, and
+// N = 2048 on two CTAs (split 3.04, FP64 4.72 ms per wave of 74, against 5.9 ms for one team of blind_rotate_kernel).
 //
 // A batch far below one wave (a single drop-in gate, a few dozen concurrent callers) waits for one bootstrap's
 // serial chain of n steps, so a step is spread over as many warps as it has independent work:
@@ -25,8 +25,9 @@
 // runs the same operations, so the bits are the same.
 //
 // The key streams through a ring, issued by a warp of its own: two stages of 48 KB at l = 3 (a step's rows of one
-// output with C = 2, three digits' rows of both with C = 1).  N = 2048 has room for five of one digit's row (16 KB),
-// each given back as soon as its words are in registers (after the products instead: 3.70 ms).
+// output with C = 2, three digits' rows of both with C = 1).  N = 2048 has room for five of one digit's row (16 KB;
+// FP64: three, and that only with the spectra in the exchange buffers and each team rotating for itself, 5.16 against
+// 5.64 ms with two), each given back as soon as its words are in registers (split, after the products instead: 3.70 ms).
 // Waits are bounded as in blind_rotate_kernel.  After one that ran out, all threads of the CTA leave the loop at the end of the same
 // step, the other CTA's next wait runs out too, and the last barrier (all threads of the cluster) keeps
 // each CTA's shared memory alive until the other's stores have landed.
@@ -46,7 +47,9 @@ template <typename T, int L, int C, int N_>
 struct LatencyLayout {
     static constexpr int N = N_, M = N / 2, NT = M / kR, KP1 = 2, KPL = KP1 * L;
     static constexpr bool split = sizeof(T) == 4, big = N == 2048;
-    static_assert(!big || (split && C == 2 && L == 3), "N = 2048: shared memory for the split form on two CTAs only");
+    static_assert(!big || (C == 2 && L == 3), "N = 2048: shared memory for two CTAs only");
+    static constexpr bool spec_in_xbufs = big && !split;  // own spectra in the teams' exchange buffers, for room
+    static constexpr bool direct = spec_in_xbufs;         // and each team rotates for itself
     static constexpr int polys = KP1 / C;                 // polynomials and outputs of a CTA
     static constexpr int fwd_teams = polys * L;           // NT threads each
     static constexpr int inv_teams = polys * (split ? 2 : 1);
@@ -54,7 +57,7 @@ struct LatencyLayout {
     static constexpr int team_warps = NT / 32;
     static constexpr int warps = team_warps * fwd_teams > mac_warps ? team_warps * fwd_teams : mac_warps;
     // whole warpgroups, for more registers in the consumers': 232 in two of three, 160 in three of four.  With the
-    // twiddles in them: FP64, l = 3 2.32 -> 2.11 (C = 1) and 1.55 -> 1.48 ms (C = 2), N = 2048 3.42 -> 3.16.  Split, l = 3,
+    // twiddles in them: FP64, l = 3 2.32 -> 2.11 (C = 1) and 1.55 -> 1.48 ms (C = 2), N = 2048 split 3.42 -> 3.16.  Split, l = 3,
     // C = 1 has room without and ran slower (1.77 against 1.67 ms).
     static constexpr bool wide = big || (!split && (C == 2 || L == 3));
     static constexpr int threads = wide ? 32 * (warps + 4) : 32 * (warps + 1), wide_regs = warps == 8 ? 232 : 160;
@@ -62,9 +65,9 @@ struct LatencyLayout {
     // ring: D stages of stage_digits digits' rows of the CTA's outputs; the first `early` digits' keys of a step go to
     // registers before the spectra have arrived
     static constexpr int stage_digits = big ? 1 : C == 2 ? KPL : L, early = big || C == 1 ? L : KPL;
-    static constexpr int D = big ? 5 : !split && C == 2 ? 1 : 2;  // FP64 needs the room; a step outlasts a refill
+    static constexpr int D = big ? (split ? 5 : 3) : !split && C == 2 ? 1 : 2;  // FP64 needs the room; a step outlasts a refill
     // stages whose twiddles a thread keeps (a last stage of radix 8 has none)
-    static constexpr int own_stages = big ? 3 : 2;
+    static constexpr int own_stages = big ? (split ? 3 : 0) : 2;
     static constexpr uint32_t stage = (uint32_t)stage_digits * polys * half;
     static constexpr size_t spec_bytes = sizeof(cplx<T>) * M;  // one digit's spectrum
     static constexpr size_t bars = 0;  // full[D], empty[D], remote[2], abort flag, stop
@@ -73,8 +76,8 @@ struct LatencyLayout {
     static constexpr size_t acc = (tables + tw_table_bytes<T, M>() + 127) / 128 * 128;
     static constexpr size_t acc_bytes = 4 * (size_t)polys * N;
     static constexpr size_t rot = acc + acc_bytes;                                 // this step's rotated words
-    static constexpr size_t spec = rot + acc_bytes;                                // [team] own digits
-    static constexpr size_t spec_in = spec + fwd_teams * spec_bytes;               // [parity][digit] the other CTA's
+    static constexpr size_t own_spec = rot + (direct ? 0 : acc_bytes);                            // [team] own digits
+    static constexpr size_t spec_in = own_spec + (spec_in_xbufs ? 0 : fwd_teams * spec_bytes);  // [parity][digit] the other CTA's
     static constexpr size_t after_spec = spec_in + (C == 2 ? 2 * L * spec_bytes : 0);
     static constexpr size_t xbuf_bytes = ((size_t)Exch<T, M>::bytes + 15) / 16 * 16;
     static constexpr int xbufs_of = !big && (split || C == 2) ? 2 : 1;  // per team; two save a barrier per exchange
@@ -85,24 +88,30 @@ struct LatencyLayout {
     static constexpr bool sums_in_xbufs = !split && C == 1;
     static constexpr size_t xbufs = after_spec + (sums_in_xbufs || big ? 0 : inv_teams * spec_bytes);
     __host__ __device__ static constexpr size_t sums(int team) {
-        return sums_in_xbufs ? xbufs + (size_t)(inv_teams + team) * xbuf_bytes
+        return spec_in_xbufs ? xbufs + xbuf_bytes  // each slot's digits are read by the thread that writes its sum
+               : sums_in_xbufs ? xbufs + (size_t)(inv_teams + team) * xbuf_bytes
                : !big        ? after_spec + team * spec_bytes
                : team == 0   ? rot
                              : xbufs + (size_t)(teams - 1) * xbufs_of * xbuf_bytes;
     }
     static_assert(!sums_in_xbufs || (teams >= 2 * inv_teams && xbufs_of == 1), "idle exchange buffers");
-    static_assert(!big || (acc_bytes >= spec_bytes && xbuf_bytes >= spec_bytes && teams > inv_teams), "places of the sums");
+    static constexpr size_t spec = spec_in_xbufs ? xbufs : own_spec, spec_stride = spec_in_xbufs ? xbuf_bytes : spec_bytes;
+    static_assert(!spec_in_xbufs || (xbufs_of == 1 && inv_teams == 1 && xbuf_bytes >= spec_bytes), "spectra in exchange buffers");
+    static_assert(!big || !split || (acc_bytes >= spec_bytes && xbuf_bytes >= spec_bytes && teams > inv_teams), "places of the sums");
     static constexpr size_t bytes = xbufs + (size_t)teams * xbufs_of * xbuf_bytes;
     static_assert((2 * D + 2) * 8 + 8 <= ring, "barrier block");
     static_assert(bytes <= 227 * 1024, "shared memory of the variant");
     static_assert(!wide || warps == 8 || warps == 12, "register split");
     static_assert(team_warps * inv_teams <= warps && KPL % stage_digits == 0, "every inverse transform has a team");
-    // place (in float4) of slots 2c, 2c + 1 of thread t in a spectrum.  N = 2048: the multiply-accumulate follows the
-    // key's second layout (key_transform.cu), whose lanes hold t's 8 apart; the low three bits are XORed so that
-    // both sides hit 8 different bank groups
-    __host__ __device__ static constexpr int pair_at(int c, int t) {
-        if (!big) return c * NT + t;
-        return (((c >> 1) * 8 + (t & 7)) * 32 + 16 * (c & 1) + 8 * (t >> 6) + (t >> 3 & 7)) ^ (t & 7);
+    // place (in 16-byte words) of row c of thread t in a spectrum: slots 2c, 2c + 1 (split) or slot c (FP64).  N = 2048: the
+    // multiply-accumulate follows the key's second layout (key_transform.cu), whose lanes hold t's 8 apart; the XOR
+    // lets it read 8 different bank groups, and keeps 8 consecutive t's, which a store to the other CTA sends
+    // as one line, in one line (a place per t in the key's order: 2.1k cycles a step to send FP64's spectra)
+    __host__ __device__ static constexpr int place(int c, int t) { return c * NT + (big ? t ^ (t >> 3 & 7) : t); }
+    // the step's digit at turn dd.  FP64 sums round to the exact integers in any order: there a CTA's own digits go
+    // first, before the wait.  The split form's low limb keeps the digits' order.
+    __host__ __device__ static constexpr int digit(int dd, int rank) {
+        return split || C == 1 || rank == 0 ? dd : (dd + L) % KPL;
     }
 };
 
@@ -201,7 +210,7 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
     if (Lay::wide ? warp >= Lay::warps : warp == Lay::warps) {  // ---- the key's stream ----
         if constexpr (Lay::wide) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Lay::wide_regs == 232 ? 40 : 32));
         if (lane == 0 && (!Lay::wide || warp == Lay::warps)) {
-            const uint8_t *bsk = SPLIT ? args.bsk2 : args.bsk;
+            const uint8_t *bsk = SPLIT || Lay::big ? args.bsk2 : args.bsk;
             const int total = args.nsteps * (KPL / Lay::stage_digits);
             int sent = 0;
             if (!args.stall_producer) {
@@ -212,7 +221,8 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
                     mbar_arrive_expect_tx(full_bar(s), Lay::stage);
                     const uint32_t dst = smem_addr(smem + Lay::ring) + (uint32_t)s * Lay::stage;
                     for (int d = 0; d < Lay::stage_digits; d++) {  // C = 2: output `rank` of each row
-                        const size_t row = (size_t)c * Lay::stage_digits + d;
+                        const size_t row = Lay::stage_digits > 1 ? (size_t)c * Lay::stage_digits + d
+                                                                 : (size_t)(c - c % KPL + Lay::digit(c % KPL, rank));
                         bulk_copy_g2s(dst + (uint32_t)d * Lay::polys * Lay::half, bsk + (row * KP1 + rank) * Lay::half,
                                       Lay::polys * Lay::half, full_bar(s));
                     }
@@ -270,7 +280,7 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
         // |low-limb sum| <= (k+1) l N 2^(Bgbit-1) 2^(S-1), doubled for FP32's error
         const bool low_small = (KPL * N <= 8192) && 13 + Bgbit - 1 + args.split_shift - 1 + 1 <= 44;
         // this team's spectrum here and in the other CTA (per parity)
-        unsigned char *my_spec = smem + Lay::spec + (size_t)(team < Lay::fwd_teams ? team : 0) * Lay::spec_bytes;
+        unsigned char *my_spec = smem + Lay::spec + (size_t)(team < Lay::fwd_teams ? team : 0) * Lay::spec_stride;
         uint32_t far_spec = 0, far_bar = 0;
         if constexpr (C == 2) {
             far_spec = cluster_addr(smem_addr(smem + Lay::spec_in + (size_t)(team < L ? team : 0) * Lay::spec_bytes),
@@ -292,25 +302,31 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
             }
 
             // 1. (X^a - 1) acc + offset: coefficient e = j - a mod 2N is e mod N, negated when e has the N bit
-#pragma unroll
-            for (int i0 = 0; i0 < Lay::polys * N; i0 += consumers) {
-                const int i = i0 + tid;
-                if (Lay::polys * N % consumers != 0 && i >= Lay::polys * N) break;
+            auto rotated = [&](int i) {
                 const int e = (i & (N - 1)) - ai, src = (i & ~(N - 1)) + (e & (N - 1));
                 const uint32_t neg = (uint32_t)((int32_t)((uint32_t)e << (N == 2048 ? 20 : 21)) >> 31), on = offset - neg;
                 const uint32_t x = s_acc[src], y = s_acc[i];
-                s_rot[i] = (x ^ neg) + (on - y);
+                return (x ^ neg) + (on - y);
+            };
+            if constexpr (!Lay::direct) {
+#pragma unroll
+                for (int i0 = 0; i0 < Lay::polys * N; i0 += consumers) {
+                    const int i = i0 + tid;
+                    if (Lay::polys * N % consumers != 0 && i >= Lay::polys * N) break;
+                    s_rot[i] = rotated(i);
+                }
+                team_sync(kAllBar, consumers);
             }
-            team_sync(kAllBar, consumers);
 
             // 2. digit, forward transform, spectrum out
             if (team < Lay::fwd_teams) {
-                const uint32_t *w = s_rot + (team / L) * N + t;
+                const int first = (team / L) * N + t;
+                auto word = [&](int j) { return Lay::direct ? rotated(first + j) : s_rot[first + j]; };
                 cplx<T> z[kR];
 #pragma unroll
                 for (int r = 0; r < kR; r++) {
-                    const T d0 = DigitConv<T>::conv((w[NT * r] >> shift) & maskBg, digit_bias);
-                    const T d1 = DigitConv<T>::conv((w[NT * r + M] >> shift) & maskBg, digit_bias);
+                    const T d0 = DigitConv<T>::conv((word(NT * r) >> shift) & maskBg, digit_bias);
+                    const T d1 = DigitConv<T>::conv((word(NT * r + M) >> shift) & maskBg, digit_bias);
                     z[r] = cplx<T>{d0, -d1};  // a_j - i a_{j+M}; the twist is folded into the FFT
                 }
                 F::forward(z, xp, own_tw, t, 1 + team);
@@ -321,16 +337,16 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
 #pragma unroll
                     for (int m = 0; m < kR / 2; m++) {
                         const float4 v = make_float4(z[2 * m].re, z[2 * m].im, z[2 * m + 1].re, z[2 * m + 1].im);
-                        if constexpr (C == 2) store_remote(far + 16u * (uint32_t)Lay::pair_at(m, t), v, bar);
-                        reinterpret_cast<float4 *>(my_spec)[Lay::pair_at(m, t)] = v;
+                        if constexpr (C == 2) store_remote(far + 16u * (uint32_t)Lay::place(m, t), v, bar);
+                        reinterpret_cast<float4 *>(my_spec)[Lay::place(m, t)] = v;
                     }
                 } else {
-                    // [r][t] {re, im}
+                    // {re, im}
 #pragma unroll
                     for (int r = 0; r < kR; r++) {
                         const double2 v = make_double2(z[r].re, z[r].im);
-                        if constexpr (C == 2) store_remote(far + 16u * (uint32_t)(r * NT + t), v, bar);
-                        reinterpret_cast<double2 *>(my_spec)[r * NT + t] = v;
+                        if constexpr (C == 2) store_remote(far + 16u * (uint32_t)Lay::place(r, t), v, bar);
+                        reinterpret_cast<double2 *>(my_spec)[Lay::place(r, t)] = v;
                     }
                 }
             }
@@ -339,14 +355,16 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
             //    apart, in the order of the key's second layout).  The keys of the first digits come in while the
             //    spectra are on their way to the other CTA; read before the forward transform they delayed it
             //    (2.17 against 1.97 us per step).
-            auto pair = [&](int i) { return Lay::big ? (i * 256 + tid) ^ (warp & 7) : tid; };  // Lay::pair_at of pair i
+            const int big_t = 64 * (lane >> 3 & 1) + 8 * (lane & 7) + ((warp ^ lane) & 7);  // N = 2048: t's part of its place
+            auto pair = [&](int i) { return Lay::big ? (2 * i + (lane >> 4)) * NT + big_t : tid; };  // Lay::place of pair i
             auto key_at = [&](int i, int k) {  // slot 2c + k of pair i in a key row's half
                 if constexpr (Lay::big) return i * 512 + k * 256 + tid;
                 else return (2 * (tid / NT) + k) * NT + (tid & (NT - 1));
             };
-            // the step's digit at turn dd.  FP64 sums round to the exact integers in any order: there the CTA's own
-            // digits go first, before the wait.  The split form's low limb keeps the digits' order.
-            auto digit = [&](int dd) { return SPLIT || C == 1 || rank == 0 ? dd : (dd + L) % KPL; };
+            auto slot_of = [&](int i, int k) {  // Lay::place of slot k of pair i
+                return Lay::big ? (4 * i + 2 * (lane >> 4) + k) * NT + big_t : key_at(i, k);
+            };
+            auto digit = [&](int dd) { return Lay::digit(dd, rank); };
             float4 key[Lay::early][Lay::polys][Lay::pairs][2];  // split {hi.re, lo.re, hi.im, lo.im}; FP64 {re, im}
             auto load_key = [&](int dd) {
                 const int c = (step * KPL + dd) / Lay::stage_digits, s = c % D;
@@ -400,9 +418,9 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
                             if (Lay::big) release(dd + e);
                         }
                     const int d = digit(dd), u = d / L, q = d - u * L;
-                    const unsigned char *sp = smem + Lay::spec + (size_t)d * Lay::spec_bytes;
+                    const unsigned char *sp = smem + Lay::spec + (size_t)d * Lay::spec_stride;
                     if constexpr (C == 2)
-                        sp = u == rank ? smem + Lay::spec + (size_t)q * Lay::spec_bytes
+                        sp = u == rank ? smem + Lay::spec + (size_t)q * Lay::spec_stride
                                        : smem + Lay::spec_in + (size_t)(parity * L + q) * Lay::spec_bytes;
 #pragma unroll
                     for (int i = 0; i < Lay::pairs; i++) {
@@ -424,7 +442,7 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
                         } else {
 #pragma unroll
                             for (int e = 0; e < 2; e++) {
-                                const double2 f = reinterpret_cast<const double2 *>(sp)[key_at(i, e)];
+                                const double2 f = reinterpret_cast<const double2 *>(sp)[slot_of(i, e)];
 #pragma unroll
                                 for (int v = 0; v < Lay::polys; v++) {
                                     const float4 k = key[dd % Lay::early][v][i][e];
@@ -452,7 +470,7 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
                         } else {
                             double2 *o = reinterpret_cast<double2 *>(smem + Lay::sums(v));
 #pragma unroll
-                            for (int e = 0; e < 2; e++) o[key_at(i, e)] = make_double2(accd[v][i][e].re, accd[v][i][e].im);
+                            for (int e = 0; e < 2; e++) o[slot_of(i, e)] = make_double2(accd[v][i][e].re, accd[v][i][e].im);
                         }
                     }
             }
@@ -465,7 +483,7 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
                 if constexpr (SPLIT) {
 #pragma unroll
                     for (int i = 0; i < kR / 2; i++) {
-                        const float4 w = reinterpret_cast<const float4 *>(in)[Lay::pair_at(i, t)];
+                        const float4 w = reinterpret_cast<const float4 *>(in)[Lay::place(i, t)];
                         z[2 * i] = {w.x, w.y};
                         z[2 * i + 1] = {w.z, w.w};
                     }
@@ -491,7 +509,7 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
                 } else {
 #pragma unroll
                     for (int r = 0; r < kR; r++) {
-                        const double2 w = reinterpret_cast<const double2 *>(in)[r * NT + t];
+                        const double2 w = reinterpret_cast<const double2 *>(in)[Lay::place(r, t)];
                         z[r] = {(T)w.x, (T)w.y};
                     }
                     F::inverse(z, xp, own_tw, t, 1 + team);
@@ -518,7 +536,7 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
 template <typename T, int L, int C, int N>
 cudaError_t launch_latency(const BrArgs &a, cudaStream_t s) {
     using Lay = LatencyLayout<T, L, C, N>;
-    if (Lay::split && !a.bsk2) return cudaErrorInvalidValue;
+    if ((Lay::split || Lay::big) && !a.bsk2) return cudaErrorInvalidValue;
     auto kern = blind_rotate_latency_kernel<T, L, C, N>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::bytes);
     if (e != cudaSuccess) return e;
@@ -545,5 +563,6 @@ template cudaError_t launch_latency<float, 2, 2, 1024>(const BrArgs &, cudaStrea
 template cudaError_t launch_latency<double, 2, 1, 1024>(const BrArgs &, cudaStream_t);
 template cudaError_t launch_latency<double, 2, 2, 1024>(const BrArgs &, cudaStream_t);
 template cudaError_t launch_latency<float, 3, 2, 2048>(const BrArgs &, cudaStream_t);
+template cudaError_t launch_latency<double, 3, 2, 2048>(const BrArgs &, cudaStream_t);
 
 }  // namespace tfheb
