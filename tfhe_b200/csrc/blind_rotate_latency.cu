@@ -5,15 +5,15 @@
 // A batch far below one wave (a single drop-in gate, a few dozen concurrent callers) waits for one bootstrap's
 // serial chain of n steps, so a step is spread over as many warps as it has independent work:
 //   1. all warps rotate: (X^a - 1) acc + offset into shared memory;
-//   2. one team of 64 threads per gadget digit runs its forward transform; the spectra go to shared memory;
+//   2. one team of 64 threads (N = 2048: 128) per gadget digit runs its forward transform; the spectra go to shared memory;
 //   3. all warps multiply-accumulate: a thread takes two slots of an output polynomial (both key limbs as a
 //      packed pair in the split form) over the digits in order.  Its keys are in registers before the
 //      spectra are there: their shared-memory reads (two thirds of the phase's) are off the chain;
 //   4. one team per (output polynomial, key limb) runs an inverse transform and adds its rounded words to
 //      the accumulator, the two limbs' teams by shared-memory atomics (integer sums mod 2^32, in any order).
-// A thread's twiddles stay in registers.  These two steps took a wave of 148 from 1.84 to 1.67 ms, one of 74 from 1.23
-// to 1.14 (split, l = 3): the shared-memory pipe is busy three quarters of a step.  Slower: the rotation by each team for itself instead of once (1.24 ms of 1.14),
-// warps of their own for the multiply-accumulate (1.35).
+// A thread's twiddles stay in registers.  These last two took a wave of 148 from 1.84 to 1.67 ms, one of 74 from 1.23
+// to 1.14 (split, l = 3): every phase waits for shared memory.  Slower: the rotation by each team for itself
+// instead of once (1.24 against 1.14 ms), warps of their own for the multiply-accumulate (1.35).
 // With C = 2 a cluster shares the bootstrap: CTA v keeps polynomial v of the accumulator, transforms its l digits
 // and computes output v, so the only thing the two exchange is the spectra, once a step: each team also
 // stores its spectrum into the other CTA's shared memory with st.async, which counts the bytes on the other
@@ -28,8 +28,8 @@
 // output with C = 2, three digits' rows of both with C = 1).  N = 2048 has room for five of one digit's row (16 KB;
 // FP64: three, and that only with the spectra in the exchange buffers and each team rotating for itself, 5.16 against
 // 5.64 ms with two), each given back as soon as its words are in registers (split, after the products instead: 3.70 ms).
-// Waits are bounded as in blind_rotate_kernel.  After one that ran out, all threads of the CTA leave the loop at the end of the same
-// step, the other CTA's next wait runs out too, and the last barrier (all threads of the cluster) keeps
+// Waits are bounded as in blind_rotate_kernel.  After one that ran out, all threads of the CTA leave the loop at the
+// end of the same step, the other CTA's next wait runs out too, and the last barrier (all threads of the cluster) keeps
 // each CTA's shared memory alive until the other's stores have landed.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -57,8 +57,8 @@ struct LatencyLayout {
     static constexpr int team_warps = NT / 32;
     static constexpr int warps = team_warps * fwd_teams > mac_warps ? team_warps * fwd_teams : mac_warps;
     // whole warpgroups, for more registers in the consumers': 232 in two of three, 160 in three of four.  With the
-    // twiddles in them: FP64, l = 3 2.32 -> 2.11 (C = 1) and 1.55 -> 1.48 ms (C = 2), N = 2048 split 3.42 -> 3.16.  Split, l = 3,
-    // C = 1 has room without and ran slower (1.77 against 1.67 ms).
+    // twiddles in them: FP64, l = 3 2.32 -> 2.11 (C = 1) and 1.55 -> 1.48 ms (C = 2), N = 2048 split 3.42 -> 3.16.
+    // Split, l = 3, C = 1 has room without and ran slower (1.77 against 1.67 ms).
     static constexpr bool wide = big || (!split && (C == 2 || L == 3));
     static constexpr int threads = wide ? 32 * (warps + 4) : 32 * (warps + 1), wide_regs = warps == 8 ? 232 : 160;
     static constexpr uint32_t half = (uint32_t)M * 16;    // one output's slots of one key row
@@ -66,7 +66,7 @@ struct LatencyLayout {
     // registers before the spectra have arrived
     static constexpr int stage_digits = big ? 1 : C == 2 ? KPL : L, early = big || C == 1 ? L : KPL;
     static constexpr int D = big ? (split ? 5 : 3) : !split && C == 2 ? 1 : 2;  // FP64 needs the room; a step outlasts a refill
-    // stages whose twiddles a thread keeps (a last stage of radix 8 has none)
+    // stages whose twiddles a thread keeps (a last stage of radix 8 has none; FP64 at N = 2048 has no registers left)
     static constexpr int own_stages = big ? (split ? 3 : 0) : 2;
     static constexpr uint32_t stage = (uint32_t)stage_digits * polys * half;
     static constexpr size_t spec_bytes = sizeof(cplx<T>) * M;  // one digit's spectrum
@@ -76,15 +76,17 @@ struct LatencyLayout {
     static constexpr size_t acc = (tables + tw_table_bytes<T, M>() + 127) / 128 * 128;
     static constexpr size_t acc_bytes = 4 * (size_t)polys * N;
     static constexpr size_t rot = acc + acc_bytes;                                 // this step's rotated words
-    static constexpr size_t own_spec = rot + (direct ? 0 : acc_bytes);                            // [team] own digits
-    static constexpr size_t spec_in = own_spec + (spec_in_xbufs ? 0 : fwd_teams * spec_bytes);  // [parity][digit] the other CTA's
+    static constexpr size_t own_spec = rot + (direct ? 0 : acc_bytes);             // [team] own digits
+    // [parity][digit] the other CTA's
+    static constexpr size_t spec_in = own_spec + (spec_in_xbufs ? 0 : fwd_teams * spec_bytes);
     static constexpr size_t after_spec = spec_in + (C == 2 ? 2 * L * spec_bytes : 0);
     static constexpr size_t xbuf_bytes = ((size_t)Exch<T, M>::bytes + 15) / 16 * 16;
     static constexpr int xbufs_of = !big && (split || C == 2) ? 2 : 1;  // per team; two save a barrier per exchange
     static constexpr int teams = fwd_teams > inv_teams ? fwd_teams : inv_teams;
     // [inverse team] the products' spectra: a region of their own, or where room is short the exchange buffers of
     // the teams that have no inverse transform, idle from the forward transforms on (FP64 in one CTA), or that of
-    // the last team and the rotated words, which the digits were taken from (N = 2048)
+    // the last team and the rotated words, which the digits were taken from (N = 2048 split), or that of the
+    // second team with its digit's spectrum (N = 2048 FP64)
     static constexpr bool sums_in_xbufs = !split && C == 1;
     static constexpr size_t xbufs = after_spec + (sums_in_xbufs || big ? 0 : inv_teams * spec_bytes);
     __host__ __device__ static constexpr size_t sums(int team) {
