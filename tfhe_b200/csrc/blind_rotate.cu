@@ -510,7 +510,7 @@ struct BrVariant {
     float us;  // measured time per step of a wave of SMs x G bootstraps, us (0: not measured)
     cudaError_t (*launch)(const BrArgs &, cudaStream_t);
     int plan = 0;  // 0: one transform per thread; 1: two per thread, spectra in TMEM (blind_rotate_paired.cu)
-    int most_bits = 32;  // the default rule takes the variant for l Bgbit up to this
+    int most_bits = 32;  // the variant serves l Bgbit up to this (a tuned one turns to another kernel by itself beyond)
     int ctas = 1;        // CTAs per bootstrap (a cluster); 2: for waves of at most SMs / 2 bootstraps, `us` of such a one
 };
 static const BrVariant kBrVariants[] = {
@@ -658,6 +658,13 @@ int br_tuned_global(int N, int l, int precision, int tuned) {
     return -1;
 }
 
+// Whether a variant serves a parameter set.
+static bool br_offered(const BrVariant &v, const tfheb_params &p, int precision) {
+    return v.N == p.N && v.l == p.l && v.precision == precision && p.l * p.Bgbit <= v.most_bits;
+}
+
+bool br_variant_offered(int g, const tfheb_params &p, int precision) { return br_offered(kBrVariants[g], p, precision); }
+
 cudaError_t launch_blind_rotate_exact(const tfheb_params &p, int precision, const DeviceBsk &bsk, const int32_t *bara,
                                       int bara_stride, int boots, int nsteps, int32_t mu, const int32_t *acc_in,
                                       int32_t *acc_out, cudaStream_t s, int32_t *d_err, int stall_producer,
@@ -666,13 +673,9 @@ cudaError_t launch_blind_rotate_exact(const tfheb_params &p, int precision, cons
     if (global_index < 0 || global_index >= br_variant_count()) return cudaErrorInvalidValue;
     const BrVariant &v = kBrVariants[global_index];
     if (v.N != p.N || v.l != p.l || v.precision != precision) return cudaErrorInvalidValue;
+    if (!v.tuned && !br_offered(v, p, precision)) return cudaErrorInvalidValue;
     return v.launch(br_args(p, bsk, bara, bara_stride, boots, nsteps, mu, acc_in, acc_out, d_err, stall_producer,
                             timeout_ns), s);
-}
-
-// Whether the default rule may take a variant for a parameter set.
-static bool br_offered(const BrVariant &v, const tfheb_params &p, int precision) {
-    return v.N == p.N && v.l == p.l && v.precision == precision && p.l * p.Bgbit <= v.most_bits;
 }
 
 int br_chosen_global(const tfheb_params &p, int precision, const BrChoice &choice) {

@@ -502,8 +502,9 @@ struct WarpLayout {
     static_assert(bytes(teams) <= 227 * 1024, "shared memory of the variant");
 };
 
-// the digits' top bits of a rotated word are kept in its low 23 bits
-constexpr int kDigitShift = 9;
+// the digits' top bits of a rotated word are kept in its low 23 bits (split form, N = 1024): no parameter set with
+// wider digits may come here
+constexpr int kDigitBits = 23, kDigitShift = 32 - kDigitBits;
 
 __device__ __forceinline__ float2 digit_pair(uint32_t a, uint32_t b) {
     return make_float2(__int_as_float(0x4B000000u | a), __int_as_float(0x4B000000u | b));
@@ -949,6 +950,7 @@ static cudaError_t launch_warp_impl(const BrArgs &args, cudaStream_t s) {
     using Lay = WarpLayout<SPLIT, L, D, MODE>;
     static_assert(G <= Lay::teams, "one warp per bootstrap, or two");
     if ((SPLIT || Lay::big) && !args.bsk2) return cudaErrorInvalidValue;
+    if (SPLIT && !Lay::big && L * args.Bgbit > kDigitBits) return cudaErrorInvalidValue;
     auto kern = blind_rotate_warp_kernel<SPLIT, L, D, MODE>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::bytes(Lay::teams));
     if (e != cudaSuccess) return e;

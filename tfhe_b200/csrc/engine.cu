@@ -962,9 +962,9 @@ tfheb_status tfheb_autotune(tfheb_cloud_key *c, int32_t precision, int32_t boots
     for (int need = 0; need < best_G && need < kSmallNeeds; need++) {
         float fastest = 1e30f;
         for (int g = 0; g < br_variant_count(); g++) {
-            int N = 0, l = 0, prec = 0, G = 0;
-            br_variant_info(g, &N, &l, &prec, &G, nullptr, nullptr);
-            if (N != p.N || l != p.l || prec != precision || G < need || G > best_G) continue;
+            int G = 0;
+            br_variant_info(g, nullptr, nullptr, nullptr, &G, nullptr, nullptr);
+            if (!br_variant_offered(g, p, precision) || G < need || G > best_G) continue;
             if (need > 0 ? br_variant_ctas(g) > 1 : G > 1) continue;
             float ms = 0;
             const int wave = need > 0 ? sms * need : std::max(1, sms / 2);

@@ -171,6 +171,8 @@ cudaError_t launch_blind_rotate_exact(const tfheb_params &p, int precision, cons
 // Size of the whole compiled table and one entry's shape; tuned = an autotuner candidate.
 int br_variant_count();
 void br_variant_info(int global_index, int *N, int *l, int *precision, int *G, int *D, int *tuned);
+// Whether a compiled variant serves a parameter set: ring, gadget length, precision and digit width.
+bool br_variant_offered(int global_index, const tfheb_params &p, int precision);
 // FFT plan of a compiled variant: 0 = one transform per thread (radix-8 team FFT), 1 = two transforms
 // per thread on packed f32x2 with the digit spectra in tensor memory (split-FP32 only)
 int br_variant_plan(int global_index);
