@@ -49,3 +49,17 @@ def test_autotuned_wide_digits(l, Bgbit):
     ck.autotune(precision, boots=1184)
     for count in (20, 100, 200, 300, 444, 592):  # every number of bootstraps per SM up to four
         assert (rotate(ck, precision, acc, bara, count) == want[:count]).all(), count
+
+
+# FP64 sums of products near 2^50 and beyond do not round to exact integers, so their order shows; the other sets' do
+@pytest.mark.parametrize("N,l,Bgbit", [(1024, 2, 11), (1024, 2, 12), (1024, 2, 14), (1024, 2, 16), (1024, 3, 10), (2048, 3, 10)])
+@pytest.mark.parametrize("tuned", [False, True])
+def test_wide_digits_in_fp64(N, l, Bgbit, tuned):
+    precision = tb.FP64
+    acc, bara = operands(N, 1184, 100 + Bgbit)
+    want = whole_waves(N, l, Bgbit, precision, acc, bara)
+    ck = make_key(N, l, Bgbit, precision)
+    if tuned:
+        ck.autotune(precision, boots=1184)
+    for count in (1, 74, 100, 200, 300, 592, 1184):
+        assert (rotate(ck, precision, acc, bara, count) == want[:count]).all(), count

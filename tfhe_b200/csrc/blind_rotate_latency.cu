@@ -21,8 +21,8 @@
 // The received half alternates between two buffers: a CTA writes step s + 2's half only after its own
 // multiply-accumulate of step s + 1, hence after the other's sending of s + 1, hence after the other's
 // multiply-accumulate of step s, which read the same buffer.
-// Every accumulator takes the same products in the same order as in blind_rotate_kernel, and each transform
-// runs the same operations, so the bits are the same.
+// Every accumulator takes the same products in the same order as in blind_rotate_kernel (but for FP64 with C = 2, see
+// LatencyLayout::digit), and each transform runs the same operations, so the bits are the same.
 //
 // The key streams through a ring, issued by a warp of its own: two stages of 48 KB at l = 3 (a step's rows of one
 // output with C = 2, three digits' rows of both with C = 1).  N = 2048 has room for five of one digit's row (16 KB;
@@ -110,8 +110,8 @@ struct LatencyLayout {
     // lets it read 8 different bank groups, and keeps 8 consecutive t's, which a store to the other CTA sends
     // as one line, in one line (a place per t in the key's order: 2.1k cycles a step to send FP64's spectra)
     __host__ __device__ static constexpr int place(int c, int t) { return c * NT + (big ? t ^ (t >> 3 & 7) : t); }
-    // the step's digit at turn dd.  FP64 sums round to the exact integers in any order: there a CTA's own digits go
-    // first, before the wait.  The split form's low limb keeps the digits' order.
+    // the step's digit at turn dd.  FP64 sums round to the exact integers in any order (with the digits that this kernel
+    // is given: kReorderBits in blind_rotate.cu): there a CTA's own digits go first, before the wait.  The split form's low limb keeps the digits' order.
     __host__ __device__ static constexpr int digit(int dd, int rank) {
         return split || C == 1 || rank == 0 ? dd : (dd + L) % KPL;
     }

@@ -520,7 +520,7 @@ __device__ __forceinline__ float2 digit_pair(uint32_t a, uint32_t b) {
 // polynomial u of the accumulator and computes output u.  Split: the digit pairs go to the two in turn, and both
 // read all spectra from TMEM.  FP64: each transforms its polynomial's digits and multiplies them with the key of
 // both outputs; the two partial sums of an output meet at the end (FP64 sums round to the exact integers in
-// any order).
+// any order, as long as digits are narrow enough: kReorderBits in blind_rotate.cu).
 //
 // big: warps w and w + 4 hold the two halves of every transform (WarpFft), and of the slots, key rows and accumulator
 // words; the accumulator keeps even and odd coefficients apart, so that a warp's are consecutive.
