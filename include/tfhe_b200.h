@@ -252,6 +252,11 @@ tfheb_status tfheb_set_wait_timeout(tfheb_cloud_key *ck, uint64_t timeout_ns);
  * the context still usable.  No reference counterpart. */
 tfheb_status tfheb_test_stall_key_stream(tfheb_cloud_key *ck, int32_t stall);
 
+/* Failure-detection test hook: tfheb_cloud_key_to_device's device allocations for the bootstrapping key fail after
+ * `nth` (from 0) more of them, once; negative: never.  A key whose loading failed in a precision is not loaded in
+ * it.  No reference counterpart. */
+tfheb_status tfheb_test_fail_device_alloc(tfheb_cloud_key *ck, int32_t nth);
+
 /* Per-kernel timing: when enabled, every kernel the key launches is bracketed by CUDA events on
  * its stream.  read: ms[4] / launches[4] accumulated for prologue, blind rotation, extraction,
  * keyswitch (reset != 0 clears the totals).  No reference counterpart (the reference has no

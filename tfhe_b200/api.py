@@ -71,6 +71,7 @@ def lib():
         L.tfheb_synchronize.argtypes = [_V]
         L.tfheb_set_wait_timeout.argtypes = [_V, ctypes.c_uint64]
         L.tfheb_test_stall_key_stream.argtypes = [_V, _I32]
+        L.tfheb_test_fail_device_alloc.argtypes = [_V, _I32]
         L.tfheb_fft_slot_order.argtypes = [_I32, _V]
         L.tfheb_br_variants.argtypes = [_I32, _I32, _V, _V, _I32, _V]
         L.tfheb_cloud_key_br_variants.argtypes = [_V, _I32, _V, _V, _I32, _V]
@@ -294,6 +295,9 @@ class CloudKey:
 
     def test_stall_key_stream(self, stall=True):
         _check(lib().tfheb_test_stall_key_stream(self.h, 1 if stall else 0), "tfheb_test_stall_key_stream")
+
+    def test_fail_device_alloc(self, nth):
+        _check(lib().tfheb_test_fail_device_alloc(self.h, nth), "tfheb_test_fail_device_alloc")
 
     def synchronize(self):
         _check(lib().tfheb_synchronize(self.h), "tfheb_synchronize")

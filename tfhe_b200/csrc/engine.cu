@@ -23,6 +23,7 @@ void set_error(const std::string &msg) { g_last_error = msg; }
 
 static tfheb_status cuda_fail(cudaError_t e, const char *where) {
     set_error(std::string(where) + ": " + cudaGetErrorString(e));
+    cudaGetLastError();  // reported: the next launch's check is not to find it again
     return e == cudaErrorMemoryAllocation ? TFHEB_ERR_NOMEM : TFHEB_ERR_CUDA;
 }
 
@@ -381,17 +382,20 @@ tfheb_status tfheb_cloud_key_params(const tfheb_cloud_key *ck, tfheb_params *out
 
 void tfheb_secret_key_free(tfheb_secret_key *sk) { delete sk; }
 
+static void free_device_bsk(DeviceBsk &d) {
+    cudaFree(d.bsk);
+    cudaFree(d.bsk2);
+    cudaFree(d.tables);
+    cudaFree(d.tables2);
+    d = DeviceBsk{};
+}
+
 void tfheb_cloud_key_free(tfheb_cloud_key *c) {
     if (!c) return;
     CloudKey &ck = c->ck;
     if (ck.device >= 0) {
         cudaSetDevice(ck.device);
-        for (auto &d : ck.dbsk) {
-            cudaFree(d.bsk);
-            cudaFree(d.bsk2);
-            cudaFree(d.tables);
-            cudaFree(d.tables2);
-        }
+        for (auto &d : ck.dbsk) free_device_bsk(d);
         free_keyswitch_key(ck.dksk);
         cudaFree(ck.d_bara);
         cudaFree(ck.d_acc);
@@ -479,45 +483,50 @@ tfheb_status tfheb_cloud_key_to_device(tfheb_cloud_key *c, int32_t device, int32
             if (p) cudaFree(p);
         }
     } d_coef, d_tab64;
+    auto alloc = [&](void **ptr, size_t bytes) {
+        const bool fail = ck.fail_alloc >= 0 && ck.fail_alloc-- == 0;
+        return cudaMalloc(ptr, fail ? SIZE_MAX / 2 : bytes);
+    };
     const size_t polys = (size_t)p.n * (p.k + 1) * p.l * (p.k + 1);
     for (int prec = 0; prec < 2; prec++) {
         if (!(precision_mask & (1 << prec))) continue;
-        DeviceBsk &d = ck.dbsk[prec];
-        if (d.bsk && (prec == TFHEB_FP64 || d.split_shift == split_shift)) continue;
-        if (d.bsk) {
-            cudaFree(d.bsk);
-            cudaFree(d.bsk2);
-            cudaFree(d.tables);
-            cudaFree(d.tables2);
-            d.bsk = d.bsk2 = d.tables = d.tables2 = nullptr;
-        }
+        if (ck.dbsk[prec].bsk && (prec == TFHEB_FP64 || ck.dbsk[prec].split_shift == split_shift)) continue;
+        free_device_bsk(ck.dbsk[prec]);
+        // the key counts as loaded once it is complete: until then its buffers belong to this scope
+        struct Loading : DeviceBsk {
+            ~Loading() { free_device_bsk(*this); }
+        } d;
         if (!d_coef.p) {
-            TFHEB_CUDA(cudaMalloc(&d_coef.p, ck.bsk_coef.size() * sizeof(int32_t)));
+            TFHEB_CUDA(alloc(&d_coef.p, ck.bsk_coef.size() * sizeof(int32_t)));
             TFHEB_CUDA(cudaMemcpy(d_coef.p, ck.bsk_coef.data(), ck.bsk_coef.size() * sizeof(int32_t),
                                   cudaMemcpyHostToDevice));
-            TFHEB_CUDA(cudaMalloc(&d_tab64.p, tab.size() * sizeof(double)));
+        }
+        if (!d_tab64.p) {
+            TFHEB_CUDA(alloc(&d_tab64.p, tab.size() * sizeof(double)));
             TFHEB_CUDA(cudaMemcpy(d_tab64.p, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice));
         }
         d.bsk_bytes = polys * (size_t)(p.N / 2) * 16;
-        TFHEB_CUDA(cudaMalloc(&d.bsk, d.bsk_bytes));
-        if (p.N == 2048 || (p.N == 1024 && prec == TFHEB_SPLIT_FP32)) TFHEB_CUDA(cudaMalloc(&d.bsk2, d.bsk_bytes));
+        TFHEB_CUDA(alloc(&d.bsk, d.bsk_bytes));
+        if (p.N == 2048 || (p.N == 1024 && prec == TFHEB_SPLIT_FP32)) TFHEB_CUDA(alloc(&d.bsk2, d.bsk_bytes));
         d.split_shift = prec == TFHEB_SPLIT_FP32 ? split_shift : 0;
         TFHEB_CUDA(launch_bsk_to_fft(p, prec, static_cast<const int32_t *>(d_coef.p),
                                      static_cast<const double *>(d_tab64.p), d.bsk, d.bsk2, split_shift, ck.stream));
         if (prec == TFHEB_FP64) {
-            TFHEB_CUDA(cudaMalloc(&d.tables, tab.size() * sizeof(double)));
+            TFHEB_CUDA(alloc(&d.tables, tab.size() * sizeof(double)));
             TFHEB_CUDA(cudaMemcpy(d.tables, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice));
         } else {
             std::vector<float> tf;
             build_tables_f32(p.N, tf);
-            TFHEB_CUDA(cudaMalloc(&d.tables, tf.size() * sizeof(float)));
+            TFHEB_CUDA(alloc(&d.tables, tf.size() * sizeof(float)));
             TFHEB_CUDA(cudaMemcpy(d.tables, tf.data(), tf.size() * sizeof(float), cudaMemcpyHostToDevice));
             build_tables_f32_paired(p.N, tf);
-            TFHEB_CUDA(cudaMalloc(&d.tables2, tf.size() * sizeof(float)));
+            TFHEB_CUDA(alloc(&d.tables2, tf.size() * sizeof(float)));
             TFHEB_CUDA(cudaMemcpy(d.tables2, tf.data(), tf.size() * sizeof(float), cudaMemcpyHostToDevice));
         }
+        TFHEB_CUDA(cudaStreamSynchronize(ck.stream));
+        ck.dbsk[prec] = d;
+        static_cast<DeviceBsk &>(d) = DeviceBsk{};
     }
-    TFHEB_CUDA(cudaStreamSynchronize(ck.stream));
     return TFHEB_OK;
 }
 
@@ -984,6 +993,13 @@ tfheb_status tfheb_test_stall_key_stream(tfheb_cloud_key *c, int32_t stall) {
     if (!c) return TFHEB_ERR_INVALID;
     std::lock_guard<std::mutex> lock(c->mu);
     c->ck.stall_producer = stall != 0;
+    return TFHEB_OK;
+}
+
+tfheb_status tfheb_test_fail_device_alloc(tfheb_cloud_key *c, int32_t nth) {
+    if (!c) return TFHEB_ERR_INVALID;
+    std::lock_guard<std::mutex> lock(c->mu);
+    c->ck.fail_alloc = nth;
     return TFHEB_OK;
 }
 

@@ -110,6 +110,7 @@ struct CloudKey {
     int32_t *d_err = nullptr;       // device error word (bounded waits that ran out)
     uint64_t wait_timeout_ns = 1000000000ull;  // limit of every device-side wait
     int stall_producer = 0;         // test hook: the key-streaming warp issues nothing
+    int fail_alloc = -1;            // test hook: allocations of the bootstrapping key's buffers before one fails
     BrChoice br[2];                 // blind-rotation launch variants per precision
     int launches = 0;               // kernels launched (for the bench's launch count)
     // optional per-kernel timing with CUDA events on the launching stream
