@@ -29,8 +29,10 @@
 // FP64: three, and that only with the spectra in the exchange buffers and each team rotating for itself, 5.16 against
 // 5.64 ms with two), each given back as soon as its words are in registers (split, after the products instead: 3.70 ms).
 // Waits are bounded as in blind_rotate_kernel.  After one that ran out, all threads of the CTA leave the loop at the
-// end of the same step, the other CTA's next wait runs out too, and the last barrier (all threads of the cluster) keeps
-// each CTA's shared memory alive until the other's stores have landed.
+// end of the same step or of the next, and the other CTA's next wait for its spectra runs out too.  Each CTA tells the
+// other how many steps it ran; after the last barrier (all threads of the cluster), which neither passes while it may
+// still send, a CTA whose waits ran out waits for every spectrum that it was sent: a barrier does not order st.async,
+// and a late one would land in the shared memory of the SM's next CTA (tests/test_cluster_exchange.py models this).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -70,7 +72,7 @@ struct LatencyLayout {
     static constexpr int own_stages = big ? (split ? 3 : 0) : 2;
     static constexpr uint32_t stage = (uint32_t)stage_digits * polys * half;
     static constexpr size_t spec_bytes = sizeof(cplx<T>) * M;  // one digit's spectrum
-    static constexpr size_t bars = 0;  // full[D], empty[D], remote[2], abort flag, stop
+    static constexpr size_t bars = 0;  // full[D], empty[D], remote[2], abort flag, stop, steps of this CTA and of the other
     static constexpr size_t ring = 128;
     static constexpr size_t tables = ring + D * (size_t)stage;
     static constexpr size_t acc = (tables + tw_table_bytes<T, M>() + 127) / 128 * 128;
@@ -101,7 +103,7 @@ struct LatencyLayout {
     static_assert(!spec_in_xbufs || (xbufs_of == 1 && inv_teams == 1 && xbuf_bytes >= spec_bytes), "spectra in exchange buffers");
     static_assert(!big || !split || (acc_bytes >= spec_bytes && xbuf_bytes >= spec_bytes && teams > inv_teams), "places of the sums");
     static constexpr size_t bytes = xbufs + (size_t)teams * xbufs_of * xbuf_bytes;
-    static_assert((2 * D + 2) * 8 + 8 <= ring, "barrier block");
+    static_assert((2 * D + 2) * 8 + 16 <= ring, "barrier block");
     static_assert(bytes <= 227 * 1024, "shared memory of the variant");
     static_assert(!wide || warps == 8 || warps == 12, "register split");
     static_assert(team_warps * inv_teams <= warps && KPL % stage_digits == 0, "every inverse transform has a team");
@@ -154,17 +156,17 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t par
     return ok != 0;
 }
 // wait_bounded for the other CTA's stores
-__device__ __forceinline__ void wait_bounded_cluster(uint32_t bar, uint32_t parity, volatile int32_t *abort_flag,
+__device__ __forceinline__ bool wait_bounded_cluster(uint32_t bar, uint32_t parity, volatile int32_t *abort_flag,
                                                      uint64_t timeout_ns, int32_t *err) {
-    if (mbar_try_wait_cluster(bar, parity, 0)) return;
+    if (mbar_try_wait_cluster(bar, parity, 0)) return true;
     const uint64_t t0 = global_timer_ns();
     for (;;) {
-        if (*abort_flag) return;
-        if (mbar_try_wait_cluster(bar, parity, kWaitSleepNs)) return;
+        if (*abort_flag) return false;
+        if (mbar_try_wait_cluster(bar, parity, kWaitSleepNs)) return true;
         if (global_timer_ns() - t0 > timeout_ns) {
             *abort_flag = 1;
             atomicOr(err, 1);
-            return;
+            return false;
         }
     }
 }
@@ -190,6 +192,7 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
     auto remote_bar = [&](int s) { return bar0 + 8u * (2 * D + s); };
     volatile int32_t *abort_flag = reinterpret_cast<volatile int32_t *>(smem + Lay::bars + 8 * (2 * D + 2));
     volatile int32_t *stop = abort_flag + 1;  // one thread's reading of the flag, the same for all warps in a step
+    volatile int32_t *ran = abort_flag + 2;  // steps that this CTA and the other ran, known after the last barrier
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < D; s++) {
@@ -294,7 +297,8 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
 
         int a_next = args.nsteps > 0 ? my_bara[0] : 0;
         bool aborted = false;
-        for (int step = 0; step < args.nsteps && !aborted; step++) {
+        int step = 0;
+        for (; step < args.nsteps && !aborted; step++) {
             const int ai = a_next & (2 * N - 1);
             if (step + 1 < args.nsteps) a_next = my_bara[step + 1];
             const int parity = step & 1;
@@ -529,10 +533,26 @@ __global__ void __launch_bounds__(LatencyLayout<T, L, C, N>::threads, 1) blind_r
 
         uint32_t *dst = reinterpret_cast<uint32_t *>(args.acc_out) + ((size_t)boot * KP1 + rank) * N;
         for (int i = tid; i < Lay::polys * N; i += consumers) dst[i] = s_acc[i];
-        if (C == 2 && aborted) __nanosleep(20000);  // stores to the other CTA may still be on their way
+        if (C == 2 && tid == 0) {
+            ran[0] = step;
+            const uint32_t far_ran = cluster_addr(bar0 + 8u * (2 * D + 2) + 12u, (uint32_t)(rank ^ 1));  // its ran[1]
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(far_ran), "r"(step) : "memory");
+        }
         __syncwarp();
     }
-    if constexpr (C == 2) cluster_sync();
+    if constexpr (C == 2) {
+        cluster_sync();  // neither CTA sends any more
+        // Without an abort here every step's wait saw its spectra land.  After one at most the last two steps' are
+        // unseen, and the other CTA ran at most two steps more, for which nothing expects the bytes yet.
+        if (threadIdx.x == 0 && *abort_flag) {
+            const int step = ran[0], sent = ran[1];
+            volatile int32_t no_abort = 0;
+            for (int s = max(0, min(step, sent) - 2); s < sent; s++) {
+                if (s >= step) mbar_arrive_expect_tx(remote_bar(s & 1), (uint32_t)(L * Lay::spec_bytes));
+                if (!wait_bounded_cluster(remote_bar(s & 1), (uint32_t)(s >> 1) & 1u, &no_abort, args.timeout_ns, args.err)) break;
+            }
+        }
+    }
 }
 
 template <typename T, int L, int C, int N>
