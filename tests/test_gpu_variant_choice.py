@@ -63,3 +63,30 @@ def test_wide_digits_in_fp64(N, l, Bgbit, tuned):
         ck.autotune(precision, boots=1184)
     for count in (1, 74, 100, 200, 300, 592, 1184):
         assert (rotate(ck, precision, acc, bara, count) == want[:count]).all(), count
+
+
+# a launch costs as much as a step or two: a rotation of one step is cut into no more launches than pay for themselves
+@pytest.mark.parametrize("N,l,Bgbit,precision,count,launches", [
+    (1024, 3, 7, tb.SPLIT_FP32, 700, 1), (1024, 3, 7, tb.SPLIT_FP32, 1500, 1), (1024, 3, 7, tb.SPLIT_FP32, 296, 1),
+    (1024, 3, 7, tb.FP64, 600, 1), (1024, 2, 10, tb.SPLIT_FP32, 700, 1), (2048, 3, 8, tb.SPLIT_FP32, 148, 1),
+    # a second packed wave takes 18.6 us, the rest in a launch of its own 7.7 + 7
+    (2048, 3, 8, tb.FP64, 700, 2)])
+def test_one_step_in_few_launches(N, l, Bgbit, precision, count, launches):
+    ck = make_key(N, l, Bgbit, precision)
+    acc, bara = operands(N, count, count)
+    got = torch.from_numpy(acc).cuda()
+    one = torch.from_numpy(np.ascontiguousarray(bara[:, :1])).cuda()
+    before = tb.kernel_launches()
+    ck.blind_rotate_device(one, got, count, 1, precision=precision)
+    ck.synchronize()
+    assert tb.kernel_launches() - before == launches
+    # the same step of the packed kernel: a whole wave of it
+    G = ck.br_variants(precision)[0]
+    wave = torch.cuda.get_device_properties(0).multi_processor_count * int(G[0])
+    pad = -count % wave
+    want = torch.from_numpy(np.concatenate([acc, np.repeat(acc[:1], pad, 0)])).cuda()
+    bara1 = np.concatenate([bara[:, :1], np.repeat(bara[:1, :1], pad, 0)])
+    ck.set_br_variant(precision, 0)
+    ck.blind_rotate_device(torch.from_numpy(bara1).cuda(), want, count + pad, 1, precision=precision)
+    ck.synchronize()
+    assert (got.cpu().numpy() == want[:count].cpu().numpy()).all()

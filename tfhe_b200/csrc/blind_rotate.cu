@@ -711,42 +711,65 @@ static int wave_variant(const tfheb_params &p, int big, int need, const BrChoice
     return pick;
 }
 
-// Bootstraps per SM that a wave of `count` needs (0: two SMs for each).
-static int wave_need(int count, int sms) { return 2 * count <= sms ? 0 : (count + sms - 1) / sms; }
+// What a launch takes beside its waves, us: the launch itself, the CTAs' setup and their last copies (5.0 to 10.4 by
+// variant, 6.6 in the middle).  Rotations of one or a few steps are cut into fewer waves for it: 700 split bootstraps of one
+// step run as one packed wave (20.7 us), not as 592 + 108 (12.8 + 8.3).
+constexpr float kLaunchUs = 7.0f;
 
-// The first wave's bootstraps of a rest of `count` (fewer than a wave of `big`): all of them, or as many whole
-// bootstraps per SM as give the least sum of measured times (*us) over the waves.  600 FP64 bootstraps run as
-// 592 + 8 (5.2 + 1.5 ms; 9.9 ms in one wave of eight per SM), 296 split ones as two of 148 (1.67 ms each, against
-// 3.68 two per SM).
-static int first_wave(const tfheb_params &p, int big, int count, int sms, const BrChoice &choice, float *us) {
-    const int need = wave_need(count, sms);
-    int first = count;
-    *us = kBrVariants[wave_variant(p, big, need, choice)].us;
-    if (need == 1 && count <= sms / 2 * 2) {  // or two waves on two SMs per bootstrap (N = 2048 split: 6.09 against 6.29 ms)
-        const float t = 2 * kBrVariants[wave_variant(p, big, 0, choice)].us;
-        if (t > 0 && t < *us) {
-            *us = t;
-            first = sms / 2;
+// The waves of a rest of `count` bootstraps, fewer than a wave of `big`, for nsteps steps: whole bootstraps per SM, by the
+// least sum of measured times.  600 FP64 bootstraps run as 592 + 8 (5.2 + 1.5 ms; 9.9 ms in one wave of eight per SM),
+// 296 split ones as two of 148 (1.67 ms each, against 3.68 two per SM).
+// Level k = 1 .. need stands for the last k bootstraps per SM of the rest; its last one (k = 1) has `low` bootstraps,
+// which two SMs each may serve, in one wave or in two (N = 2048 split, 148: 6.09 against 6.29 ms).
+struct RestWaves {
+    static constexpr int kMost = 16;  // bootstraps per SM of the largest variant, and one more wave
+    int waves = 0;
+    struct {
+        int variant, count;
+    } wave[kMost];
+    float us = 0;  // 0: not known
+};
+
+static RestWaves rest_waves(const tfheb_params &p, int big, int count, int sms, int nsteps, const BrChoice &choice) {
+    RestWaves out;
+    const int need = (count + sms - 1) / sms, low = count - (need - 1) * sms, pairs = sms / 2;
+    auto cost = [&](int g) { return kBrVariants[g].us > 0 ? kBrVariants[g].us * (float)nsteps + kLaunchUs : 0.f; };
+    int variant[RestWaves::kMost], first[RestWaves::kMost];  // first[k]: bootstraps per SM of the next wave, -1: two of `pairs`
+    float own[RestWaves::kMost], best[RestWaves::kMost];
+    for (int k = 1; k <= need; k++) {
+        variant[k] = wave_variant(p, big, k, choice);
+        own[k] = cost(variant[k]);
+        if (k == 1) {  // by itself the last bootstrap per SM may have two SMs
+            const int two = wave_variant(p, big, 0, choice);
+            const int g = low <= pairs ? two : variant[1];
+            best[1] = cost(g);
+            first[1] = 1;
+            if (low > pairs && low <= 2 * pairs && cost(two) > 0 && 2 * cost(two) < best[1]) best[1] = 2 * cost(two), first[1] = -1;
+            continue;
         }
+        best[k] = own[k];
+        first[k] = k;
+        for (int a = 1; a < k && own[k] > 0; a++)
+            if (own[a] > 0 && best[k - a] > 0 && own[a] + best[k - a] < best[k]) best[k] = own[a] + best[k - a], first[k] = a;
     }
-    for (int a = 1; a < need && *us > 0; a++) {
-        const float ta = kBrVariants[wave_variant(p, big, a, choice)].us;
-        float rest = 0;
-        if (ta == 0 || ta >= *us) continue;
-        first_wave(p, big, count - a * sms, sms, choice, &rest);
-        if (rest > 0 && ta + rest < *us) {
-            *us = ta + rest;
-            first = a * sms;
+    out.us = best[need];
+    for (int k = need, left = count; k > 0;) {
+        int n = first[k] < k ? first[k] * sms : left, g = variant[first[k] > 0 ? first[k] : 1];
+        if (k == 1 && (first[1] < 0 || low <= pairs)) {
+            g = wave_variant(p, big, 0, choice);
+            if (first[1] < 0) n = pairs;
         }
+        out.wave[out.waves++] = {g, n};
+        left -= n;
+        if (first[k] < 0 && left > 0) out.wave[out.waves++] = {g, left};
+        k = first[k] < 0 ? 0 : k - first[k];
     }
-    return first;
+    return out;
 }
 
 float br_rest_us(const tfheb_params &p, int precision, const BrChoice &choice, int sms, int count) {
     const int big = br_chosen_global(p, precision, choice);
-    float us = 0;
-    if (big >= 0 && count > 0) first_wave(p, big, count, sms, choice, &us);
-    return us;
+    return big >= 0 && count > 0 ? rest_waves(p, big, count, sms, p.n, choice).us / (float)p.n : 0.f;
 }
 
 // Full waves of the chosen variant (SMs x G bootstraps each), then the rest in waves of whatever runs that many
@@ -764,31 +787,22 @@ cudaError_t launch_blind_rotate(const tfheb_params &p, int precision, const Devi
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         sms = 0;
-    for (int first = 0; first < boots;) {
-        int g = big, count = boots - first;
-        const int wave = sms * kBrVariants[big].G, rest = sms > 0 ? count % wave : 0;
-        if (rest > 0) {
-            float us = 0;
-            const int part = first_wave(p, big, rest, sms, choice, &us);
-            g = wave_variant(p, big, wave_need(part, sms), choice);
-            if (g != big || part < rest) {  // the full waves by themselves, then the rest wave by wave
-                if (count > wave) {
-                    g = big;
-                    count -= rest;
-                } else {
-                    count = part;
-                }
-            }
-        }
+    auto launch = [&](int g, int first, int count) {
         const size_t at = (size_t)first * (p.k + 1) * p.N;
-        const cudaError_t e = launch_blind_rotate_exact(
-            p, precision, bsk, bara + (size_t)first * bara_stride, bara_stride, count, nsteps, mu,
-            acc_in ? acc_in + at : nullptr, acc_out + at, s, d_err, stall_producer, timeout_ns, g);
-        if (e != cudaSuccess) return e;
         if (launches) ++*launches;
-        first += count;
-    }
-    return cudaSuccess;
+        return launch_blind_rotate_exact(p, precision, bsk, bara + (size_t)first * bara_stride, bara_stride, count, nsteps,
+                                         mu, acc_in ? acc_in + at : nullptr, acc_out + at, s, d_err, stall_producer,
+                                         timeout_ns, g);
+    };
+    const int wave = sms * kBrVariants[big].G, rest = wave > 0 ? boots % wave : 0, full = boots - rest;
+    if (rest == 0) return launch(big, 0, boots);
+    const RestWaves tail = rest_waves(p, big, rest, sms, nsteps, choice);
+    // after full waves the rest may be one more of them in the same launch
+    if (full > 0 && !(tail.us < kBrVariants[big].us * (float)nsteps)) return launch(big, 0, boots);
+    cudaError_t e = full > 0 ? launch(big, 0, full) : cudaSuccess;
+    for (int w = 0, at = full; w < tail.waves && e == cudaSuccess; at += tail.wave[w++].count)
+        e = launch(tail.wave[w].variant, at, tail.wave[w].count);
+    return e;
 }
 
 struct ExtVariant {
