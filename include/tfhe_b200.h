@@ -282,8 +282,8 @@ tfheb_status tfheb_measure_dft8(int32_t device, int32_t method, double *ns_per_d
  * depth; *count receives how many exist (arrays filled up to cap).  Two entries may share both
  * numbers: one streams the key with a dedicated warp, the other from its first thread.  tfheb_cloud_key_br_variants
  * lists them for a key's own parameter set (the 80-bit set has l = 2).  tfheb_set_br_variant picks
- * one for a key; tfheb_autotune times them all on `boots` synthetic bootstraps, keeps the fastest
- * for the key, and writes each variant's time to ms[] (up to cap).  It then times, for each g below
+ * one for a key, or with -1 returns it to a new key's default (which entry 0 is not);
+ * tfheb_autotune times them all on `boots` synthetic bootstraps, keeps the fastest for the key, and writes each variant's time to ms[] (up to cap).  It then times, for each g below
  * the winner's bootstraps per CTA, every compiled variant that fits a full wave of SMs x g bootstraps
  * and keeps the fastest for such waves.  A key that was neither set nor tuned uses the variant with
  * the least time per bootstrap in the library's own measurements.  Either way a batch runs as full

@@ -283,6 +283,8 @@ class CloudKey:
                 for g, d, pl, m in zip(G, D, P, ms)]
 
     def set_br_variant(self, precision, variant):
+        """A candidate of br_variants for full waves, or -1: a new key's default rule, after autotune or another
+        variant."""
         _check(lib().tfheb_set_br_variant(self.h, precision, variant), "tfheb_set_br_variant")
 
     def set_keyswitch_kernel(self, which):

@@ -875,10 +875,11 @@ tfheb_status tfheb_cloud_key_br_plans(const tfheb_cloud_key *c, int32_t precisio
 
 tfheb_status tfheb_set_br_variant(tfheb_cloud_key *c, int32_t precision, int32_t variant) {
     if (!c || (precision != TFHEB_FP64 && precision != TFHEB_SPLIT_FP32)) return TFHEB_ERR_INVALID;
-    if (variant < 0 || variant >= br_variants(c->ck.p.N, c->ck.p.l, precision, nullptr, nullptr, 0))
+    if (variant < -1 || variant >= br_variants(c->ck.p.N, c->ck.p.l, precision, nullptr, nullptr, 0))
         return TFHEB_ERR_INVALID;
     std::lock_guard<std::mutex> lock(c->mu);
-    c->ck.br[precision].tuned = variant;
+    if (variant < 0) c->ck.br[precision] = BrChoice{};  // as a new key
+    else c->ck.br[precision].tuned = variant;
     return TFHEB_OK;
 }
 
