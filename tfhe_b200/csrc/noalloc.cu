@@ -144,6 +144,7 @@ extern "C" tfheb_status tfheb_gate_batch_device_noalloc(tfheb_cloud_key *c, int3
     int32_t *ksin = reinterpret_cast<int32_t *>(b + off_ksin);
 
     int32_t cst = 0, sa = 0, sb = 0;
+    int rotations = 0;
     if (gate != TFHEB_MUX) gate_form(gate, &cst, &sa, &sb);
     fill_descs_kernel<<<(count + 255) / 256, 256, 0, s>>>(bd, gd, count, gate == TFHEB_MUX, cst, sa, sb,
                                                         modswitch_to_torus32(-1, 8), modswitch_to_torus32(1, 8));
@@ -152,13 +153,13 @@ extern "C" tfheb_status tfheb_gate_batch_device_noalloc(tfheb_cloud_key *c, int3
     if (e == cudaSuccess)
         e = launch_blind_rotate(p, precision, ck.dbsk[precision], bara, (int)bs, (int)boots, p.n,
                                 modswitch_to_torus32(1, 8), nullptr, acc, s, ck.d_err, ck.stall_producer,
-                                ck.wait_timeout_ns, ck.br[precision]);
+                                ck.wait_timeout_ns, ck.br[precision], &rotations);
     if (e == cudaSuccess) e = launch_extract(p, gd, count, acc, ksin, (int)kN1, s);
     if (e == cudaSuccess) e = launch_keyswitch(ck, count, ksin, (int)kN1, d_out, s);
     if (e != cudaSuccess) {
         set_error(std::string("tfheb_gate_batch_device_noalloc: ") + cudaGetErrorString(e));
         return TFHEB_ERR_CUDA;
     }
-    g_kernel_launches += 5;
+    g_kernel_launches += 4 + rotations;
     return TFHEB_OK;
 }
