@@ -550,6 +550,10 @@ def main():
         sms = torch.cuda.get_device_properties(local_rank).multi_processor_count
         lanes = 128 if args.form == "split" else 64
         nominal = sms * lanes * 2 * (clk.get("sm_max_mhz") or 1965.0) * 1e6 / 1e12
+        # the kernel of the candidate that the autotuner kept for full waves
+        best = min(tuning[args.form], key=lambda v: v["ms"])
+        kernel = ("blind_rotate_warp_kernel" if best["teams_per_cta"] == 8 else
+                  "blind_rotate_paired_kernel" if best["plan"] else "blind_rotate_kernel")
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": main_r["total_ms"] / args.steps, "higher_is_better": True,
@@ -565,7 +569,7 @@ def main():
                 "kernel_ms": other_r["kernel_ms"]},
             "kernel_ms": {"prologue": main_r["kernel_ms"][0], "blind_rotate": main_r["kernel_ms"][1],
                           "extract": main_r["kernel_ms"][2], "keyswitch": main_r["kernel_ms"][3]},
-            "roofline": {"bound": "fp32" if args.form == "split" else "fp64", "kernel": "blind_rotate_kernel",
+            "roofline": {"bound": "fp32" if args.form == "split" else "fp64", "kernel": kernel,
                          "achieved": achieved, "peak": pk, "unit": "TFLOP/s", "frac": achieved / pk,
                          "peak_source": "measured FMA-chain probe on this GPU (tfheb_measure_fma_peak)",
                          "peak_nominal": nominal, "frac_nominal": achieved / nominal,
@@ -577,8 +581,9 @@ def main():
             "peaks_measured": peak,
             "autotune": tuning,
             "plans": {"0": "radix-8 team FFT, one transform per thread",
-                      "1": "radix-8 team FFT, two transforms per thread on packed f32x2, digit spectra in TMEM "
-                           "(candidates differ in ring depth and in how many transform pairs run interleaved)"},
+                      "1": "radix-8 FFT, two transforms per thread on packed f32x2, digit spectra in TMEM "
+                           "(candidates differ in ring depth and in how many transform pairs run interleaved)",
+                      "teams_per_cta 8": "either, a warp per transform with its exchanges in TMEM"},
             "clocks": clk,
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": 2 * B * (p.n + 1) * 4,
                     "d2h_bytes_per_step": B * (p.n + 1) * 4, "errors": e2e_errors,

@@ -297,7 +297,8 @@ tfheb_status tfheb_cloud_key_br_variants(const tfheb_cloud_key *ck, int32_t prec
 /* FFT plan of each variant of tfheb_cloud_key_br_variants, same order: 0 = the radix-8 team FFT with
  * one transform per thread; 1 = the same transform, two per thread on packed f32x2, with the digit
  * spectra parked in tensor memory and the multiply-accumulate one output polynomial at a time
- * (split-FP32; the same bits as plan 0).  The autotuner times both plans. */
+ * (split-FP32; the same bits as plan 0).  Entries with 8 bootstraps per CTA at N = 1024, or 4 at
+ * N = 2048, run either plan's arithmetic with one or two warps per transform and its exchanges in tensor memory.  The autotuner times both plans. */
 tfheb_status tfheb_cloud_key_br_plans(const tfheb_cloud_key *ck, int32_t precision, int32_t *plan, int32_t cap,
                                       int32_t *count);
 tfheb_status tfheb_set_br_variant(tfheb_cloud_key *ck, int32_t precision, int32_t variant);

@@ -544,7 +544,7 @@ static const BrVariant kBrVariants[] = {
     {1024, 3, TFHEB_SPLIT_FP32, 6, 6, true, 10.50, launch_paired<1024, 3, 6, 6, 2, true>, 1},
     // one warp per bootstrap, exchanges in TMEM (blind_rotate_warp.cu; D counts 16 KB units): the split default
     {1024, 3, TFHEB_SPLIT_FP32, 8, 6, true, 10.94, launch_warp_split3, 1, 23},
-    // the paired kernel with 3-6 teams, for waves of that many (3 and 4: for digits the warp kernel does not take)
+    // the paired kernel with 3-6 teams, for waves of that many (3 to 5: for digits the warp kernel does not take)
     {1024, 3, TFHEB_SPLIT_FP32, 6, 12, false, 10.33, launch_paired_il3<1024, 3, 6, 12, 1>, 1},
     {1024, 3, TFHEB_SPLIT_FP32, 5, 12, false, 9.57, launch_paired_il3<1024, 3, 5, 12, 1>, 1},
     {1024, 3, TFHEB_SPLIT_FP32, 4, 12, false, 7.86, launch_paired_il3<1024, 3, 4, 12, 1>, 1},

@@ -1,5 +1,5 @@
-// br_common.cuh -- pieces shared by the blind-rotation kernels (blind_rotate.cu,
-// blind_rotate_paired.cu): launch arguments, the exact integer/float conversions and the
+// br_common.cuh -- pieces shared by the blind-rotation kernels (blind_rotate.cu, blind_rotate_paired.cu,
+// blind_rotate_warp.cu, blind_rotate_latency.cu): launch arguments, the exact integer/float conversions and the
 // (X^a - 1) rotation.  Every kernel computes these the same way, so all give the same bits.
 #pragma once
 

@@ -602,8 +602,8 @@ cudaError_t launch_keyswitch(const CloudKey &ck, int count, const int32_t *in, i
     if (count <= 0) return cudaSuccess;
     const tfheb_params &p = ck.p;
     // default: the tensor-core kernel wherever it is built (t = 8, basebit = 2), at every batch size
-    // (measured per 4096 / 1036 / 256 / 1 samples: 0.305 / 0.114 / 0.044 / 0.035 ms, against 1.82 /
-    // 0.578 / 0.225 / 0.077 ms for the register-key and 2.89 / 0.738 / 0.196 / 0.049 ms for the
+    // (measured per 4096 / 1036 / 256 / 1 samples: 0.219 / 0.081 / 0.028 / 0.021 ms, against 1.82 /
+    // 0.576 / 0.223 / 0.075 ms for the register-key and 2.88 / 0.736 / 0.195 / 0.047 ms for the
     // tiled kernel); otherwise the one-CTA-per-sample kernel
     if ((ck.ks_kernel == 4 || ck.ks_kernel == 0) && ck.dksk.mma_groups != 0)
         return launch_keyswitch_mma(ck, count, in, in_stride, out, s);

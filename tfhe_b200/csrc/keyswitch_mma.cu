@@ -22,8 +22,8 @@
 // modulo 2^32 (a unit that one CTA does alone is stored).
 //
 // What bounds it: the products.  One of M 128, N 256, K 32 takes 267 cycles of an SM here (256 at 4096 multiply-adds per
-// cycle); 4096 samples of the default set are 277 quads per SM, 6 products each: 0.217 ms, and 0.227 ms measured
-// (0.300 ms with the h = 0 bytes and five waves of quarter units; one sample 0.025 ms, was 0.035).  Twice the row
+// cycle); 4096 samples of the default set are 277 quads per SM, 6 products each: 0.217 ms, and 0.219 ms measured
+// (0.305 ms with the h = 0 bytes and five waves of quarter units; one sample 0.021 ms, was 0.035).  Twice the row
 // threads or 32-byte swizzled operands changed nothing.
 //
 // Roles (320 threads):

@@ -1,5 +1,5 @@
-// tmem.cuh -- tensor memory (TMEM) and tcgen05 helpers shared by the paired blind-rotation kernel and
-// the tensor-core keyswitch (sm_100a inline PTX).
+// tmem.cuh -- tensor memory (TMEM) and tcgen05 helpers shared by the paired and the warp blind-rotation
+// kernel and the tensor-core keyswitch (sm_100a inline PTX).
 //
 // TMEM is 512 columns x 128 lanes of 32-bit cells per SM.  A warp reads and writes the 32 lanes of
 // its quadrant (warp % 4); a TMEM address is lane << 16 | column.
